@@ -43,6 +43,7 @@ int64_t instinct_step(torch::Tensor p, torch::Tensor grad, torch::Tensor m, c10:
 std::vector<torch::Tensor> anchor_select(torch::Tensor s, torch::Tensor tau, int64_t A);
 std::vector<torch::Tensor> moe_slots(torch::Tensor e_flat, int64_t E, int64_t C);
 std::vector<torch::Tensor> lock_find(torch::Tensor x, int64_t vocab, int64_t n_keys, bool longest_only);
+std::vector<torch::Tensor> lock_find_bucket(torch::Tensor x, int64_t vocab, int64_t n_keys, c10::optional<torch::Tensor> bucket);
 std::vector<torch::Tensor> moe_route_fwd(torch::Tensor logits, torch::Tensor real, torch::Tensor k_tok, int64_t k_max);
 std::vector<torch::Tensor> mem_read_fwd(torch::Tensor q, torch::Tensor faces, torch::Tensor valid, torch::Tensor dim_pen,
                                         int64_t Fn, double scale);
@@ -110,6 +111,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("anchor_select", &mb::anchor_select);
   m.def("moe_slots", &mb::moe_slots);
   m.def("lock_find", &mb::lock_find);
+  m.def("lock_find_bucket", &mb::lock_find_bucket);
   m.def("attn_fwd_tc", &mb::attn_fwd_tc, "causal / sliding-window attention forward on tcgen05 (head dim 64)");
   m.def("attn_status_read", &mb::attn_status_read);
   m.def("attn_bwd_tc", &mb::attn_bwd_tc, "causal / sliding-window attention backward on tcgen05 (head dim 64)");

@@ -1,5 +1,5 @@
-// Discrete selection kernels: anchor selection (threshold + causal per-text cap + stable compaction), MoE capacity
-// slotting in arrival order, and the keys-and-locks pointer search.  All produce exactly the decisions of the sort /
+// Discrete selection kernels: anchor selection (threshold + causal per-text cap + stable compaction) and MoE capacity
+// slotting in arrival order.  Both produce exactly the decisions of the sort /
 // cumsum formulations they replace (ties resolved towards the smaller index).
 #include <torch/extension.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -307,72 +307,6 @@ torch::Tensor moe_route_bwd(torch::Tensor probs, torch::Tensor top_e, torch::Ten
       dl.data_ptr<float>(), N, E, k_max);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return dl;
-}
-
-// Keys and locks: for each position t and n-gram length n = 1..n_keys, the latest j < t whose n-gram ending at j
-// equals the one ending at t; the candidate is the token after j.  The text is staged in shared memory; grid (texts,
-// slices): a block takes runs of blockDim positions spread evenly over the text (late positions scan further back, so
-// contiguous halves would be unbalanced), which keeps a batch of few long texts (4 x 16 384) on all SMs.
-__global__ void lock_find_kernel(const long long* __restrict__ x, long long* __restrict__ cand, bool* __restrict__ on,
-                                 long long* __restrict__ src, int T, int n_keys, int longest_only) {
-  extern __shared__ int tok[];
-  const int b = blockIdx.x;
-  const long long* xr = x + (long long)b * T;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) tok[t] = (int)xr[t];
-  __syncthreads();
-  for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < T; t += gridDim.y * blockDim.x) {
-    int last[3] = {-1, -1, -1};
-    const int a0 = tok[t], a1 = t >= 1 ? tok[t - 1] : -1, a2 = t >= 2 ? tok[t - 2] : -1;
-    int need = n_keys;                                   // how many key lengths are still unresolved
-    for (int j = t - 1; j >= 0 && need > 0; --j) {
-      if (tok[j] != a0) continue;
-      if (last[0] < 0) { last[0] = j; --need; }
-      if (n_keys >= 2 && t >= 1 && j >= 1 && tok[j - 1] == a1) {
-        if (last[1] < 0) { last[1] = j; --need; }
-        if (n_keys >= 3 && t >= 2 && j >= 2 && tok[j - 2] == a2 && last[2] < 0) { last[2] = j; --need; }
-      }
-      // a longer key can only match where the shorter one matches, so once the 1-gram is found we keep scanning
-      // only for the longer ones; stop early when position constraints make them impossible
-      if (n_keys >= 2 && t < 1 && last[0] >= 0) break;
-    }
-    bool ok[3];
-    for (int n = 0; n < n_keys; ++n) ok[n] = last[n] >= 0;
-    if (longest_only) {
-      for (int n = 0; n < n_keys - 1; ++n)
-        for (int q = n + 1; q < n_keys; ++q) if (ok[q]) ok[n] = false;
-    }
-    for (int n = 0; n < n_keys; ++n) {
-      const bool found = last[n] >= 0;
-      const int sp = found ? min(last[n] + 1, T - 1) : 0;
-      const long long o = ((long long)b * T + t) * n_keys + n;
-      cand[o] = found ? tok[sp] : 0;
-      src[o] = sp;
-      on[o] = ok[n];
-    }
-  }
-}
-
-std::vector<torch::Tensor> lock_find(torch::Tensor x, int64_t vocab, int64_t n_keys, bool longest_only) {
-  const c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.scalar_type() == torch::kInt64, "lock_find: (B,T) int64");
-  TORCH_CHECK(n_keys >= 1 && n_keys <= 3, "lock_find: 1..3 key lengths");
-  const int B = x.size(0), T = x.size(1);
-  TORCH_CHECK((size_t)T * 4 <= 200 * 1024, "lock_find: text too long for shared memory staging");
-  auto cand = torch::empty({B, T, n_keys}, x.options());
-  auto src = torch::empty({B, T, n_keys}, x.options());
-  auto on = torch::empty({B, T, n_keys}, x.options().dtype(torch::kBool));
-  if (B) {
-    size_t smem = (size_t)T * 4;
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(lock_find_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int threads = 256;
-    const int slices = std::max(1, std::min((T + threads - 1) / threads, (4 * 148 + B - 1) / B));
-    lock_find_kernel<<<dim3(B, slices), threads, smem, cur_stream()>>>(reinterpret_cast<const long long*>(x.data_ptr<int64_t>()),
-        reinterpret_cast<long long*>(cand.data_ptr<int64_t>()), on.data_ptr<bool>(),
-        reinterpret_cast<long long*>(src.data_ptr<int64_t>()), T, (int)n_keys, longest_only ? 1 : 0);
-  }
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {cand, on, src};
 }
 
 }  // namespace mb

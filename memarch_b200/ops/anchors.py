@@ -5,7 +5,7 @@ anchor states and `scatter_add` of the heavy layers' delta (1681, 1702), keys-an
 stable sorts (1499-1535), phrase-table `searchsorted` (1441-1450).
 
 GPU bodies: `anchor_select` (one CTA per text: threshold, prefix count, compaction into idx/valid in one pass),
-`lock_find` (hash of 1/2/3-gram keys, last earlier occurrence) and `gather_rows`/`scatter_add_rows`.
+`lock_find` (hash tables of 1/2/3-gram keys, last earlier occurrence) and `gather_rows`/`scatter_add_rows`.
 """
 from __future__ import annotations
 
@@ -25,9 +25,14 @@ def select_anchors(s, tau, A):
 
 def find_locks(x, vocab, n_keys=3, lock_bucket=None):
     if _ext.use_cuda(x):
-        cand, on, src = _ext.C().lock_find(x.contiguous(), int(vocab), int(n_keys), lock_bucket is not None)
+        fused = lock_bucket is None or (lock_bucket.dtype == torch.int64 and lock_bucket.device == x.device
+                                        and lock_bucket.is_contiguous() and lock_bucket.dim() == 1)
         _ext.count()
-        bk = lock_bucket[x.clamp(max=lock_bucket.numel() - 1)] if lock_bucket is not None else torch.zeros_like(x)
+        if fused:
+            cand, on, src, bk = _ext.C().lock_find_bucket(x.contiguous(), int(vocab), int(n_keys), lock_bucket)
+            return cand, on, bk, src
+        cand, on, src = _ext.C().lock_find(x.contiguous(), int(vocab), int(n_keys), True)
+        bk = lock_bucket[x.clamp(max=lock_bucket.numel() - 1)]
         return cand, on, bk, src
     return ref.find_locks(x, vocab, n_keys, lock_bucket)
 
