@@ -1,6 +1,5 @@
-// Row-wise and elementwise kernels (HBM-bound): RMSNorm fwd/bwd, relu^2, SwiGLU, RoPE on packed qkv, the
-// cross-entropy row kernel (plain and pointer-mixture), slot gathers / weighted gather-sums for MoE dispatch and
-// combine.  All use 16-byte vector accesses and fp32 math.
+// Row-wise and elementwise kernels (HBM-bound): relu^2, SwiGLU, RoPE on packed qkv, slot gathers / weighted gather-sums
+// for MoE dispatch and combine.  All use 16-byte vector accesses and fp32 math.
 #include <torch/extension.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -22,178 +21,6 @@ template <typename T> __device__ __forceinline__ void st4(T* p, float4 v);
 template <> __device__ __forceinline__ void st4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 template <> __device__ __forceinline__ void st4<bf16>(bf16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
-}
-
-// ------------------------------------------------------------------------------------------------ RMSNorm
-template <typename TX, typename TY>
-__global__ void rmsnorm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, TY* __restrict__ y,
-                                   float* __restrict__ rstd, int d, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const TX* xr = x + row * d;
-  float ss = 0.f;
-  for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
-    float4 v = ld4(xr + c);
-    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-  }
-  ss = block_sum(ss, red);
-  const float r = rsqrtf(ss / d + eps);
-  if (threadIdx.x == 0) rstd[row] = r;
-  TY* yr = y + row * d;
-  for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
-    float4 v = ld4(xr + c), g = ld4(w + c);
-    st4(yr + c, make_float4(v.x * r * g.x, v.y * r * g.y, v.z * r * g.z, v.w * r * g.w));
-  }
-}
-
-// dx = r*(g*w) - x * r^3/d * sum(g*w*x); dw += g * x * r (block-local accumulation over its rows, then atomics)
-// Optional `add` (fp32, same shape): a gradient that reached x by another path (the residual stream) is summed in
-// the same pass; optional `dx_lo`: the result is also written in bf16 (the branch that produced part of x wants it).
-template <typename TX, typename TG, int NV>
-__global__ void rmsnorm_bwd_kernel(const TG* __restrict__ dy, const TX* __restrict__ x, const float* __restrict__ w,
-                                   const float* __restrict__ rstd, TX* __restrict__ dx, float* __restrict__ dw,
-                                   int n_rows, int d, const float* __restrict__ add, bf16* __restrict__ dx_lo) {
-  __shared__ float red[32];
-  // d <= NV * 4 * blockDim.x; a row's x, dy and w stay in registers between the dot product and the update
-  float4 acc[NV], ww[NV];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int c = (i * blockDim.x + threadIdx.x) * 4;
-    ww[i] = c < d ? ld4(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  for (long long row = blockIdx.x; row < n_rows; row += gridDim.x) {
-    const TX* xr = x + row * d;
-    const TG* gr = dy + row * d;
-    const float r = rstd[row];
-    float4 xv[NV], gv[NV];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = (i * blockDim.x + threadIdx.x) * 4;
-      if (c < d) {
-        xv[i] = ld4(xr + c);
-        gv[i] = ld4(gr + c);
-        dot += gv[i].x * ww[i].x * xv[i].x + gv[i].y * ww[i].y * xv[i].y + gv[i].z * ww[i].z * xv[i].z +
-               gv[i].w * ww[i].w * xv[i].w;
-      }
-    }
-    dot = block_sum(dot, red);
-    const float k = dot * r * r * r / d;
-    TX* dxr = dx + row * d;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = (i * blockDim.x + threadIdx.x) * 4;
-      if (c < d) {
-        const float4 v = xv[i], g = gv[i];
-        float4 o = make_float4(r * g.x * ww[i].x - v.x * k, r * g.y * ww[i].y - v.y * k, r * g.z * ww[i].z - v.z * k,
-                               r * g.w * ww[i].w - v.w * k);
-        if (add) { const float4 q = ld4(add + row * d + c); o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w; }
-        st4(dxr + c, o);
-        if (dx_lo) st4(dx_lo + row * d + c, o);
-        acc[i].x += g.x * v.x * r; acc[i].y += g.y * v.y * r; acc[i].z += g.z * v.z * r; acc[i].w += g.w * v.w * r;
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (i * blockDim.x + threadIdx.x) * 4;
-    if (c < d) {
-      atomicAdd(dw + c, acc[i].x); atomicAdd(dw + c + 1, acc[i].y);
-      atomicAdd(dw + c + 2, acc[i].z); atomicAdd(dw + c + 3, acc[i].w);
-    }
-  }
-}
-
-// h = x (fp32) + y (bf16); n = rmsnorm(h) * w in bf16: the residual add and the next normalisation in one pass.
-__global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x, const bf16* __restrict__ y, const float* __restrict__ w,
-                                       float* __restrict__ h, bf16* __restrict__ n, float* __restrict__ rstd, int d, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const float* xr = x + row * d;
-  const bf16* yr = y + row * d;
-  float* hr = h + row * d;
-  float ss = 0.f;
-  for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
-    float4 a = ld4(xr + c), b = ld4(yr + c);
-    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-    st4(hr + c, a);
-    ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-  }
-  ss = block_sum(ss, red);
-  const float r = rsqrtf(ss / d + eps);
-  if (threadIdx.x == 0) rstd[row] = r;
-  bf16* nr = n + row * d;
-  for (int c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
-    float4 v = ld4(hr + c), g = ld4(w + c);          // each thread re-reads exactly what it wrote
-    st4(nr + c, make_float4(v.x * r * g.x, v.y * r * g.y, v.z * r * g.z, v.w * r * g.w));
-  }
-}
-std::vector<torch::Tensor> add_rmsnorm_fwd(torch::Tensor x, torch::Tensor y, torch::Tensor w, double eps) {
-  const c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && y.is_contiguous() && x.scalar_type() == torch::kFloat32 &&
-              y.scalar_type() == torch::kBFloat16 && x.numel() == y.numel() && x.size(1) % 4 == 0, "add_rmsnorm: fp32 + bf16");
-  const int n = x.size(0), d = x.size(1);
-  torch::Tensor wf = w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32);
-  auto h = torch::empty_like(x);
-  auto nn = torch::empty({n, d}, x.options().dtype(torch::kBFloat16));
-  auto rstd = torch::empty({n}, x.options().dtype(torch::kFloat32));
-  if (n) add_rmsnorm_fwd_kernel<<<n, d >= 1024 ? 256 : 128, 0, cur_stream()>>>(x.data_ptr<float>(),
-      reinterpret_cast<const bf16*>(y.data_ptr()), wf.data_ptr<float>(), h.data_ptr<float>(), reinterpret_cast<bf16*>(nn.data_ptr()),
-      rstd.data_ptr<float>(), d, (float)eps);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {h, nn, rstd};
-}
-
-std::vector<torch::Tensor> rmsnorm_fwd(torch::Tensor x, torch::Tensor w, double eps, bool out_bf16) {
-  const c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(1) % 4 == 0, "rmsnorm: (N,d) contiguous, d % 4 == 0");
-  const int n = x.size(0), d = x.size(1);
-  torch::Tensor wf = w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32);
-  auto y = torch::empty({n, d}, x.options().dtype(out_bf16 ? torch::kBFloat16 : torch::kFloat32));
-  auto rstd = torch::empty({n}, x.options().dtype(torch::kFloat32));
-  if (n == 0) return {y, rstd};
-  const int threads = d >= 1024 ? 256 : 128;
-  const bool xb = x.scalar_type() == torch::kBFloat16;
-#define LAUNCH(TX, TY) rmsnorm_fwd_kernel<TX, TY><<<n, threads, 0, cur_stream()>>>( \
-      reinterpret_cast<const TX*>(x.data_ptr()), wf.data_ptr<float>(), reinterpret_cast<TY*>(y.data_ptr()), \
-      rstd.data_ptr<float>(), d, (float)eps)
-  if (xb && out_bf16) LAUNCH(bf16, bf16); else if (xb) LAUNCH(bf16, float);
-  else if (out_bf16) LAUNCH(float, bf16); else LAUNCH(float, float);
-#undef LAUNCH
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {y, rstd};
-}
-
-std::vector<torch::Tensor> rmsnorm_bwd(torch::Tensor dy, torch::Tensor x, torch::Tensor w, torch::Tensor rstd,
-                                       c10::optional<torch::Tensor> add_, bool want_lo) {
-  const c10::cuda::CUDAGuard guard(x.device());
-  const float* add = nullptr;
-  if (add_.has_value() && add_->defined()) {
-    TORCH_CHECK(add_->scalar_type() == torch::kFloat32 && add_->is_contiguous() && add_->numel() == x.numel(), "rmsnorm_bwd: add");
-    add = add_->data_ptr<float>();
-  }
-  const int n = x.size(0), d = x.size(1);
-  TORCH_CHECK(d <= 8 * 4 * 256 && d % 4 == 0, "rmsnorm_bwd: d <= 8192");
-  torch::Tensor wf = w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32);
-  auto dx = torch::empty_like(x);
-  auto dw = torch::zeros({d}, x.options().dtype(torch::kFloat32));
-  torch::Tensor lo = want_lo ? torch::empty({n, d}, x.options().dtype(torch::kBFloat16)) : torch::Tensor();
-  bf16* lop = want_lo ? reinterpret_cast<bf16*>(lo.data_ptr()) : nullptr;
-  if (n == 0) return {dx, dw, lo};
-  const int grid = std::min(n, 148 * 8);
-  const bool xb = x.scalar_type() == torch::kBFloat16, gb = dy.scalar_type() == torch::kBFloat16;
-#define LAUNCH_NV(TX, TG, NV) rmsnorm_bwd_kernel<TX, TG, NV><<<grid, 256, 0, cur_stream()>>>( \
-      reinterpret_cast<const TG*>(dy.data_ptr()), reinterpret_cast<const TX*>(x.data_ptr()), wf.data_ptr<float>(), \
-      rstd.data_ptr<float>(), reinterpret_cast<TX*>(dx.data_ptr()), dw.data_ptr<float>(), n, d, add, lop)
-#define LAUNCH(TX, TG) do { if (d <= 2048) LAUNCH_NV(TX, TG, 2); else if (d <= 4096) LAUNCH_NV(TX, TG, 4); \
-                            else LAUNCH_NV(TX, TG, 8); } while (0)
-  if (xb && gb) LAUNCH(bf16, bf16); else if (xb) LAUNCH(bf16, float);
-  else if (gb) LAUNCH(float, bf16); else LAUNCH(float, float);
-#undef LAUNCH
-#undef LAUNCH_NV
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {dx, dw, lo};
 }
 
 // ------------------------------------------------------------------------------------------------ activations
@@ -471,91 +298,6 @@ torch::Tensor resid_add(torch::Tensor x, torch::Tensor y) {
       reinterpret_cast<const bf16*>(y.data_ptr()), out.data_ptr<float>(), n4);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return out;
-}
-
-// ------------------------------------------------------------------------------------------------ CE row kernel
-// One block per row of bf16 logits: online max/sum -> lse; loss; logits overwritten with d(loss)/d(logits).
-// With gate/hit: pointer mixture P = (1-g)*p_y + g*hit, loss = -log max(P,1e-30), grad = w*(softmax - onehot),
-// w = (1-g)*p_y/P, dg = (p_y - hit)/P.
-__global__ void ce_rows_kernel(bf16* __restrict__ logits, const long long* __restrict__ y, float* __restrict__ loss,
-                               const float* __restrict__ gate, const float* __restrict__ hit, float* __restrict__ dg,
-                               long long stride, int V) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  bf16* p = logits + row * stride;
-  const int V8 = V / 8;
-  float m = -INFINITY, s = 0.f;
-  for (int i = threadIdx.x; i < V8; i += blockDim.x) {
-    uint4 u = reinterpret_cast<const uint4*>(p)[i];
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(&u);
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { float2 f = unpack_bf16(q[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
-    float mx = v[0];
-#pragma unroll
-    for (int j = 1; j < 8; ++j) mx = fmaxf(mx, v[j]);
-    const float mn = fmaxf(m, mx);
-    float add = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) add += __expf(v[j] - mn);
-    s = s * __expf(m - mn) + add;
-    m = mn;
-  }
-  for (int c = V8 * 8 + threadIdx.x; c < V; c += blockDim.x) {
-    float v = __bfloat162float(p[c]);
-    const float mn = fmaxf(m, v);
-    s = s * __expf(m - mn) + __expf(v - mn);
-    m = mn;
-  }
-  const float M = block_max(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - M);
-  s = block_sum(s, red);
-  const float lse = M + logf(s);
-  const long long yy = y[row];
-  const float xy = __bfloat162float(p[yy]);
-  float wgt = 1.f;
-  __syncthreads();                                           // every thread has read p[yy] before anyone overwrites it
-  if (gate != nullptr) {
-    const float g = gate[row], h = hit[row];
-    const float py = __expf(xy - lse);
-    float P = fmaxf((1.f - g) * py + g * h, 1e-30f);
-    wgt = (1.f - g) * py / P;
-    if (threadIdx.x == 0) { loss[row] = -logf(P); dg[row] = (py - h) / P; }
-  } else if (threadIdx.x == 0) {
-    loss[row] = lse - xy;
-  }
-  for (int i = threadIdx.x; i < V8; i += blockDim.x) {
-    uint4 u = reinterpret_cast<const uint4*>(p)[i];
-    uint32_t* q = reinterpret_cast<uint32_t*>(&u);
-    const int c0 = i * 8;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 f = unpack_bf16(q[j]);
-      float a = __expf(f.x - lse) - ((c0 + 2 * j) == yy ? 1.f : 0.f);
-      float b = __expf(f.y - lse) - ((c0 + 2 * j + 1) == yy ? 1.f : 0.f);
-      q[j] = pack_bf16(wgt * a, wgt * b);
-    }
-    reinterpret_cast<uint4*>(p)[i] = u;
-  }
-  for (int c = V8 * 8 + threadIdx.x; c < V; c += blockDim.x) {
-    float v = __bfloat162float(p[c]);
-    p[c] = __float2bfloat16(wgt * (__expf(v - lse) - (c == yy ? 1.f : 0.f)));
-  }
-}
-void ce_rows(torch::Tensor logits, torch::Tensor y, torch::Tensor loss, c10::optional<torch::Tensor> gate,
-             c10::optional<torch::Tensor> hit, c10::optional<torch::Tensor> dg) {
-  const c10::cuda::CUDAGuard guard(logits.device());
-  TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.scalar_type() == torch::kBFloat16, "ce_rows: bf16 (n,V)");
-  TORCH_CHECK(y.scalar_type() == torch::kInt64 && y.is_contiguous() && loss.is_contiguous(), "ce_rows: y int64");
-  TORCH_CHECK(logits.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(logits.data_ptr()) & 15) == 0, "ce_rows: row alignment");
-  const int n = logits.size(0), V = logits.size(1);
-  if (!n) return;
-  const bool mix = gate.has_value() && gate->defined();
-  ce_rows_kernel<<<n, 512, 0, cur_stream()>>>(
-      reinterpret_cast<bf16*>(logits.data_ptr()), y.data_ptr<int64_t>() ? reinterpret_cast<const long long*>(y.data_ptr<int64_t>()) : nullptr,
-      loss.data_ptr<float>(), mix ? gate->data_ptr<float>() : nullptr, mix ? hit->data_ptr<float>() : nullptr,
-      mix ? dg->data_ptr<float>() : nullptr, logits.stride(0), V);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
 // ------------------------------------------------------------------------------------------------ gathers

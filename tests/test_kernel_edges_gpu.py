@@ -52,3 +52,46 @@ def test_lock_find_tables_and_scan(text, B, T, n_keys):
     if n_keys == 1:
         got, want = anchors.find_locks(x.cuda(), V, 1, None), ref.find_locks(x, V, 2, None)
         assert torch.equal(got[0][..., 0].cpu(), want[0][..., 0]) and torch.equal(got[3][..., 0].cpu(), want[3][..., 0])
+
+
+# ------------------------------------------------------------------------------------------------ RMSNorm, cross-entropy rows
+@pytest.mark.parametrize("n,d", [(1, 8), (3, 256), (5, 264), (17, 512), (9, 520), (33, 1024), (2, 1032), (700, 2048), (3, 2056), (4, 4096), (5, 4104), (2, 8192), (3, 8200), (5000, 64)])
+def test_rmsnorm_widths(n, d):
+    from memarch_b200.ops import _ext
+    C = _ext.C()
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x, w = torch.randn(n, d, device="cuda", generator=g), torch.rand(d, device="cuda", generator=g) + 0.5
+    y, dy, add = (torch.randn(n, d, device="cuda", generator=g) for _ in range(3))
+    yb, dyb = y.bfloat16(), dy.bfloat16()
+    xs = (x.double() + yb.double()).requires_grad_()
+    wd = w.double().requires_grad_()
+    ref = xs * torch.rsqrt(xs.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+    h, out, rstd = C.add_rmsnorm_fwd(x, yb, w, 1e-6)
+    assert _rel(h, xs.detach()) < 1e-6 and _rel(out, ref.detach()) < 4e-3           # bf16 rounding: 2^-9 per element
+    out32, _ = C.rmsnorm_fwd(h, w, 1e-6, False)
+    assert _rel(out32, ref.detach()) < 1e-6
+    outb, _ = C.rmsnorm_fwd(h.bfloat16(), w, 1e-6, True)
+    assert _rel(outb, ref.detach()) < 8e-3
+    if d > 8192:
+        return
+    ref.backward(dyb.double())
+    for a in (None, add):
+        dx, dw, lo = C.rmsnorm_bwd(dyb, h, w, rstd, a, True)
+        want = xs.grad if a is None else xs.grad + a.double()
+        assert _rel(dx, want) < 1e-5 and _rel(lo, want) < 4e-3 and _rel(dw, wd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("n,V", [(1, 8), (3, 9), (5, 4096), (4, 16384 + 8), (2, 16389), (3, 50304)])
+def test_ce_rows_sizes(n, V):
+    from memarch_b200.ops import _ext
+    g = torch.Generator(device="cuda").manual_seed(V)
+    lg = torch.empty(n, (V + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :V]
+    lg.copy_(torch.randn(n, V, device="cuda", generator=g) * 4)
+    y = torch.randint(0, V, (n,), device="cuda", generator=g)
+    y[0], y[-1] = V - 1, 0
+    x = lg.double().requires_grad_()
+    loss = torch.nn.functional.cross_entropy(x, y, reduction="none")
+    loss.sum().backward()
+    out = torch.empty(n, device="cuda")
+    _ext.C().ce_rows(lg, y, out, None, None, None)
+    assert _rel(out, loss.detach()) < 1e-5 and _rel(lg, x.grad) < 4e-3
