@@ -10,11 +10,16 @@
 // Epilogues: plain store (bf16 or fp32, optional += into fp32), relu^2 (also stores the pre-activation),
 // relu^2 backward (acc * 2*relu(aux)), SwiGLU over column halves, per-row scale.
 // Every mbarrier wait is bounded; on a timeout the kernel records a code in `status`, drains and returns.
-#include <torch/extension.h>
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
+#include <cuda.h>
+
+#include <algorithm>
+#include <cstdlib>
+#include <stdexcept>
+#include <string>
+#include <type_traits>
 
 #include "common.cuh"
+#include "gemm_api.h"
 
 namespace mb {
 
@@ -24,36 +29,11 @@ constexpr int GEMM_THREADS = 192;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int GROUP_M = 8;
 
-enum { EPI_NONE = 0, EPI_RELU2 = 1, EPI_DRELU2 = 2, EPI_SWIGLU = 3, EPI_ROWSCALE = 4, EPI_DSWIGLU = 5 };
-
-struct GemmParams {
-  int M, N, K, G;                 // logical per-group problem; for EPI_SWIGLU N = 2H (B rows), out has H columns
-  void* out;
-  void* out2;
-  const void* aux;
-  long long out_gs, out2_gs, aux_gs;   // group strides in elements
-  int ldo, ldo2, ldaux;                // row pitches in elements
-  int epi, out_f32, accumulate;
-  int m_tiles, n_tiles;
-  int ntail;                 // 1: the last N tile issues MMAs only as wide as its valid columns (rounded up to 16)
-  int* status;
-  // M may be cut into `n_seg` segments of `seg_M` rows, each read through its own A tensor map (a peer GPU's
-  // buffer) and, when `out_seg_on`, written to its own output base (the owner GPU's buffer).  Tiles never straddle
-  // segments.  Plain GEMM: n_seg = 1, seg_M = M.
-  int n_seg, seg_M, tiles_per_seg, a_g_off, out_g_off, out_seg_on;
-  void* out_seg[8];
-  // Pair kernel v3 only.  store_tma: the epilogue leaves through TMA stores (local output, one segment); otherwise
-  // through coalesced row stores from the staged tile (peer buffers, segmented output).
-  // counts: valid extent per group (device ints) - count_mode 1: rows of A/out (tiles wholly past it are not
-  // computed and are written as zeros), 2: length of the contraction (k-blocks past it are not read).
-  int store_tma, count_mode, dbg, group_m;
-  int aux_tma;             // the aux operand of an epilogue (pre-activations) is prefetched by TMA into the staging tiles
-  const int* counts;
-};
-
 struct TmapSet { CUtensorMap m[8]; };
 
+// work item t -> group, row tile, column tile (the items of one output tile's splits are neighbours)
 __device__ __forceinline__ void tile_coords(int t, const GemmParams& p, int& g, int& mt, int& nt) {
+  if (p.splits > 1) t /= p.splits;
   int per_g = p.m_tiles * p.n_tiles;
   g = t / per_g;
   int r = t - g * per_g;
@@ -789,6 +769,14 @@ __device__ __forceinline__ int group_kblocks(const GemmParams& p, int g) {
   return (k + BK - 1) / BK;
 }
 
+// first k-block of work item t; `num_kb` (the group's k-blocks) shrinks to the item's share
+__device__ __forceinline__ int split_start(const GemmParams& p, int t, int& num_kb) {
+  if (p.splits <= 1) return 0;
+  const int kb0 = (t % p.splits) * p.kb_split;
+  num_kb = min(p.kb_split, num_kb - kb0);
+  return kb0;
+}
+
 // MH = 256-row MMA blocks per tile.  MH 1: 256 x 256 tile, 5 operand stages of 32 KB, accumulators double-buffered in
 // TMEM (2 x 256 columns), so the epilogue of a tile runs under the MMAs of the next.  MH 2: 512 x 256 tile - every
 // B k-block feeds two MMAs, so the pair pulls 96 KB per 512x256x64 of work instead of 128 KB (a quarter less L2 and
@@ -827,7 +815,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int total = p.G * p.m_tiles * p.n_tiles;
+  const int total = p.G * p.m_tiles * p.n_tiles * max(1, p.splits);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES3; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -868,7 +856,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         const int m0 = mseg0 + (int)rank * BM;
         const CUtensorMap* tA = &tmAs.m[seg];
         const int ga = g + p.a_g_off;
-        const int num_kb = group_kblocks(p, g);
+        int num_kb = group_kblocks(p, g);
+        const int kb0 = split_start(p, t, num_kb);
         const int nb = (p.epi == EPI_SWIGLU) ? (rank == 0 ? nt * 128 : (p.N >> 1) + nt * 128)
                                              : nt * BN + (int)rank * (tile_n_eff(p, nt) >> 1);
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -879,7 +868,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
           uint8_t* sB = sA + MH * A_BYTES;
           const uint32_t lfull = mapa_shared(smem_u32(&full[stage]), 0);      // the leader's barrier
           if (leader) mbar_expect_tx(&full[stage], 2 * STAGE_B);               // bytes of both CTAs
-          const int k0 = kb * BK;
+          const int k0 = (kb0 + kb) * BK;
 #pragma unroll
           for (int h = 0; h < MH; ++h) {                                       // this CTA's 128 rows of each 256-row block
             const int mh = m0 + h * 256;
@@ -929,6 +918,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         const int seg = mt_ / p.tiles_per_seg;
         if (seg * p.seg_M + (mt_ - seg * p.tiles_per_seg) * TILE_M >= group_rows(p, g_)) return;
         nkb = group_kblocks(p, g_);
+        split_start(p, t, nkb);
         idesc = idesc_bf16(256, tile_n_eff(p, nt_), A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       };
       int num_kb, nxt_kb = 0;
@@ -1056,13 +1046,17 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+static void check(bool ok, const char* what) {            // becomes a Python RuntimeError in the bindings
+  if (!ok) throw std::runtime_error(what);
+}
+
 static EncodeTiledFn encode_fn() {
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
-    TORCH_CHECK(e == cudaSuccess && p != nullptr, "cuTensorMapEncodeTiled entry point not found");
+    check(e == cudaSuccess && p != nullptr, "cuTensorMapEncodeTiled entry point not found");
     fn = reinterpret_cast<EncodeTiledFn>(p);
   }
   return fn;
@@ -1080,8 +1074,8 @@ CUtensorMap make_tmap(const void* base, int esz, uint64_t inner, uint64_t rows, 
   cuuint64_t strides[2] = {row_pitch_el * esz, (groups > 1 ? group_pitch_el : row_pitch_el * rows) * esz};
   cuuint32_t box[3] = {box_inner, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  TORCH_CHECK((reinterpret_cast<uintptr_t>(base) & 15) == 0, "TMA operand must be 16-byte aligned");
-  TORCH_CHECK(strides[0] % 16 == 0 && strides[1] % 16 == 0, "TMA operand pitches must be multiples of 16 bytes");
+  check((reinterpret_cast<uintptr_t>(base) & 15) == 0, "TMA operand must be 16-byte aligned");
+  check(strides[0] % 16 == 0 && strides[1] % 16 == 0, "TMA operand pitches must be multiples of 16 bytes");
   const CUtensorMapDataType dt = esz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                 : esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   CUresult r = encode_fn()(&m, dt, 3,
@@ -1089,7 +1083,7 @@ CUtensorMap make_tmap(const void* base, int esz, uint64_t inner, uint64_t rows, 
                            CU_TENSOR_MAP_SWIZZLE_128B,
                            promote ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_NONE,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TORCH_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", static_cast<int>(r));
+  if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(r)));
   return m;
 }
 CUtensorMap make_tmap_bf16(const void* base, uint64_t inner, uint64_t rows, uint64_t groups, uint64_t row_pitch_el,
@@ -1097,30 +1091,28 @@ CUtensorMap make_tmap_bf16(const void* base, uint64_t inner, uint64_t rows, uint
   return make_tmap(base, 2, inner, rows, groups, row_pitch_el, group_pitch_el, box_inner, box_rows, true);
 }
 
-static int* status_word(int device) {
+int* gemm_status_word(int device) {
   static int* words[16] = {nullptr};
-  TORCH_CHECK(device >= 0 && device < 16, "device index out of range");
+  check(device >= 0 && device < 16, "device index out of range");
   if (!words[device]) {
-    TORCH_CHECK(cudaMalloc(&words[device], sizeof(int)) == cudaSuccess, "status word alloc failed");
+    check(cudaMalloc(&words[device], sizeof(int)) == cudaSuccess, "status word alloc failed");
     cudaMemset(words[device], 0, sizeof(int));
   }
   return words[device];
 }
 
-int* gemm_status_word(int device) { return status_word(device); }
-
 int gemm_status(int device) {
   int v = 0;
-  cudaMemcpy(&v, status_word(device), sizeof(int), cudaMemcpyDeviceToHost);
+  cudaMemcpy(&v, gemm_status_word(device), sizeof(int), cudaMemcpyDeviceToHost);
   int z = 0;
-  if (v) cudaMemcpy(status_word(device), &z, sizeof(int), cudaMemcpyHostToDevice);
+  if (v) cudaMemcpy(gemm_status_word(device), &z, sizeof(int), cudaMemcpyHostToDevice);
   return v;
 }
 
 // The CTA-pair (cta_group::2) kernel is the default for tiles of >= 256 rows; MEMARCH_GEMM_PAIR=0 or
 // gemm_set_pair(false) selects the single-CTA kernel everywhere.
 static int g_pair = -1;
-static bool use_pair_kernel() {
+bool gemm_pair_on() {
   if (g_pair < 0) {
     const char* e = std::getenv("MEMARCH_GEMM_PAIR");
     g_pair = (e && e[0] == '0') ? 0 : 1;
@@ -1132,19 +1124,24 @@ void gemm_set_pair(bool on) { g_pair = on ? 1 : 0; }
 static int g_dbg = 0, g_group_m = 0;
 void gemm_set_debug(int64_t dbg, int64_t group_m) { g_dbg = (int)dbg; g_group_m = (int)group_m; }
 
+static bool tma_stores_on() {
+  static const bool off = []() { const char* e = std::getenv("MEMARCH_GEMM_TMA_STORE"); return e && e[0] == '0'; }();
+  return !off && !(g_dbg & DBG_DIRECT_STORE);
+}
+
 // Raw launcher shared by the torch binding and the fused multi-GPU paths (which pass peer pointers for A).
 // A_list: one base pointer per M-segment (n_seg of them, each (a_groups, seg_M, K) or MN-major (a_groups, K, seg_M)).
 void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_groups, long long a_rows_pitch, long long a_gs,
                      bool a_mn, const void* B, long long b_rows_pitch, long long b_gs, bool b_mn, GemmParams p,
                      cudaStream_t stream, int max_ctas) {
   const int N = p.N, K = p.K, G = p.G;
-  TORCH_CHECK(n_seg >= 1 && n_seg <= 8, "gemm: 1..8 segments");
+  check(n_seg >= 1 && n_seg <= 8, "gemm: 1..8 segments");
   TmapSet tmAs;
   for (int i = 0; i < n_seg; ++i)
     tmAs.m[i] = a_mn ? make_tmap_bf16(A_list[i], seg_M, K, a_groups, a_rows_pitch, a_gs, 64, 64)
                      : make_tmap_bf16(A_list[i], K, seg_M, a_groups, a_rows_pitch, a_gs, 64, BM);
   for (int i = n_seg; i < 8; ++i) tmAs.m[i] = tmAs.m[0];
-  const bool pair = use_pair_kernel() && seg_M >= 256;
+  const bool pair = gemm_pair_on() && seg_M >= 256;
   const bool sw = p.epi == EPI_SWIGLU;
   const int n_tiles = sw ? ((N / 2) + 127) / 128 : (N + BN - 1) / BN;
   // 512-row tiles (see PairCfg) when the contraction is long enough to pay for the half-exposed epilogue and the
@@ -1157,7 +1154,7 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
       return (double)tiles / (double)(((tiles + pairs - 1) / pairs) * pairs);
     };
     static const bool tall_env = []() { const char* e = std::getenv("MEMARCH_GEMM_TALL"); return !(e && e[0] == '0'); }();
-    tall = tall_env && K >= 8192 && wave_eff(512) >= wave_eff(256) - 0.02;
+    tall = tall_env && p.splits <= 1 && K >= 8192 && wave_eff(512) >= wave_eff(256) - 0.02;
     if (g_dbg & DBG_TALL_OFF) tall = false;
     if (g_dbg & DBG_TALL_ON) tall = true;
   }
@@ -1169,11 +1166,13 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
   p.n_tiles = n_tiles;
   static const bool ntail_on = []() { const char* e = std::getenv("MEMARCH_GEMM_NTAIL"); return !(e && e[0] == '0'); }();
   p.ntail = ntail_on ? 1 : 0;
-  const int total = G * p.m_tiles * p.n_tiles;
+  check(p.splits <= 1 || (pair && !tall && n_seg == 1 && p.count_mode == 0 && p.epi == EPI_NONE && p.out_f32 && p.accumulate),
+        "gemm: split contraction needs the pair kernel, a plain epilogue and an accumulating fp32 output");
+  const int total = G * p.m_tiles * p.n_tiles * std::max(1, p.splits);
   int grid = pair ? 2 * std::min(total, max_ctas / 2) : std::min(total, max_ctas);
   if (grid <= 0) return;
   const bool v3 = pair;
-  TORCH_CHECK(v3 || p.count_mode == 0, "gemm: per-group extents need the pair kernel (>= 256 rows)");
+  check(v3 || p.count_mode == 0, "gemm: per-group extents need the pair kernel (>= 256 rows)");
   const bool deep = v3 && !tall && p.epi == EPI_DSWIGLU && !a_mn;
   const int smem_bytes = v3 ? (tall ? PairCfg<2>::SMEM : deep ? PairCfg<1, true>::SMEM : PairCfg<1>::SMEM) : SMEM_BYTES;
   CUtensorMap tmO = tmB, tmO2 = tmB;
@@ -1185,8 +1184,8 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
     // through coalesced row stores (peer buffers are only ever written with plain stores)
     p.store_tma = (n_seg == 1 && !p.out_seg_on && (p.ldo * esz) % 16 == 0 && (G == 1 || (p.out_gs * esz) % 16 == 0) &&
                    (!p.out2 || ((p.ldo2 * 2) % 16 == 0 && (G == 1 || (p.out2_gs * 2) % 16 == 0)))) ? 1 : 0;
-    static const bool tma_off = []() { const char* e = std::getenv("MEMARCH_GEMM_TMA_STORE"); return e && e[0] == '0'; }();
-    if (tma_off || (g_dbg & DBG_DIRECT_STORE)) p.store_tma = 0;
+    if (!tma_stores_on()) p.store_tma = 0;
+    check(p.splits <= 1 || p.store_tma, "gemm: split contraction adds its parts with TMA stores");
     if (p.store_tma) {
       const int No = sw ? N / 2 : N;
       tmO = make_tmap(p.out, esz, No, p.M, G, p.ldo, p.out_gs, p.out_f32 ? 32 : 64, 32, false);
@@ -1214,7 +1213,7 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 15][id]) {
-      TORCH_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) == cudaSuccess,
+      check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) == cudaSuccess,
                   "cannot raise dynamic shared memory for the GEMM kernel");
       attr_set[dev & 15][id] = true;
     }
@@ -1243,7 +1242,8 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
     else if (a_mn && !b_mn) launch(gemm_tc_kernel<true, false>, id);
     else launch(gemm_tc_kernel<true, true>, id);
   }
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  const cudaError_t le = cudaGetLastError();
+  check(le == cudaSuccess, cudaGetErrorString(le));
 }
 
 void launch_gemm(const void* A, long long a_rows_pitch, long long a_gs, bool a_mn, const void* B, long long b_rows_pitch,
@@ -1252,7 +1252,36 @@ void launch_gemm(const void* A, long long a_rows_pitch, long long a_gs, bool a_m
   launch_gemm_seg(list, 1, p.M, p.G, a_rows_pitch, a_gs, a_mn, B, b_rows_pitch, b_gs, b_mn, p, stream, max_ctas);
 }
 
-static int sm_count() {
+// fp32 -> bf16 copy of a (rows, n) matrix, n % 4 == 0
+__global__ void __launch_bounds__(256) round_rows_kernel(const float4* __restrict__ src, bf16* __restrict__ dst, long long n4, int row4, int ldo) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / row4;
+    const float4 v = src[i];
+    *reinterpret_cast<uint2*>(dst + r * ldo + (i - r * row4) * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  }
+}
+void round_rows_launch(const float* src, void* dst, long long rows, int n, int ldo, cudaStream_t stream) {
+  const long long n4 = rows * (n / 4);
+  const int grid = (int)std::min<long long>((n4 + 255) / 256, 148 * 8);
+  round_rows_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<bf16*>(dst), n4, n / 4, ldo);
+}
+
+// How many runs to cut the contraction of one plain product into (1: none).  A product with fewer output tiles than
+// half of the 74 CTA pairs leaves the rest of the chip idle; every run costs a clear, an fp32 reduce-add and (for bf16) a
+// rounding pass over the output, so a run keeps at least 8 k-blocks (512 of the contraction).  (1000, 256, K = 50304):
+// 333 us whole, 38 + 5 in 18 runs; (256, 1024, K = 2048): 20 us whole, 11.5 + 4 in 4.
+int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
+  kb_split = 0;
+  if (G != 1 || M < 256 || !gemm_pair_on() || !tma_stores_on()) return 1;
+  const int tiles = ((M + 255) / 256) * ((N + BN - 1) / BN), pairs = max_ctas / 2, kb = (K + BK - 1) / BK;
+  if (2 * tiles > pairs || kb < 32) return 1;
+  const int want = std::min(pairs / tiles, kb / 8);
+  if (want < 2) return 1;
+  kb_split = (kb + want - 1) / want;
+  return (kb + kb_split - 1) / kb_split;
+}
+
+int gemm_sm_count() {
   static int n = 0;
   if (!n) {
     int dev = 0;
@@ -1260,126 +1289,6 @@ static int sm_count() {
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   }
   return n;
-}
-
-// torch binding.  a: (G?, M, K) or MN-major (G?, K, M); b: (G?, N, K) or MN-major (G?, K, N).
-torch::Tensor gemm(torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor> out_,
-                   c10::optional<torch::Tensor> out2_, c10::optional<torch::Tensor> aux_, bool a_mn, bool b_mn,
-                   bool accumulate, int64_t epi, bool out_f32, int64_t groups, c10::optional<torch::Tensor> counts_,
-                   int64_t count_mode) {
-  TORCH_CHECK(a.is_cuda() && b.is_cuda(), "gemm: CUDA tensors expected");
-  TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm: bf16 operands");
-  const c10::cuda::CUDAGuard guard(a.device());
-  const int G = (int)groups;
-  auto as3 = [&](torch::Tensor t) { return t.dim() == 2 ? t.unsqueeze(0) : t; };
-  torch::Tensor A = as3(a), B = as3(b);
-  TORCH_CHECK(A.dim() == 3 && B.dim() == 3 && A.size(0) == G && B.size(0) == G, "gemm: group dimension mismatch");
-  TORCH_CHECK(A.stride(2) == 1 && B.stride(2) == 1, "gemm: innermost dimension must be contiguous");
-  const int M = a_mn ? A.size(2) : A.size(1), K = a_mn ? A.size(1) : A.size(2);
-  const int N = b_mn ? B.size(2) : B.size(1), Kb = b_mn ? B.size(1) : B.size(2);
-  TORCH_CHECK(K == Kb, "gemm: K mismatch ", K, " vs ", Kb);
-  const int Nout = epi == EPI_SWIGLU ? N / 2 : (epi == EPI_DSWIGLU ? 2 * N : N);
-  torch::Tensor out;
-  if (out_.has_value() && out_->defined()) {
-    out = *out_;
-  } else {
-    auto opt = a.options().dtype(out_f32 ? torch::kFloat32 : torch::kBFloat16);
-    out = (a.dim() == 2 && G == 1) ? torch::empty({M, Nout}, opt) : torch::empty({G, M, Nout}, opt);
-  }
-  TORCH_CHECK(out.scalar_type() == (out_f32 ? torch::kFloat32 : torch::kBFloat16), "gemm: out dtype");
-  torch::Tensor O = as3(out);
-  TORCH_CHECK(O.size(0) == G && O.size(1) == M && O.size(2) == Nout && O.stride(2) == 1, "gemm: out shape");
-  GemmParams p{};
-  p.M = M; p.N = N; p.K = K; p.G = G;
-  p.out = O.data_ptr(); p.ldo = (int)O.stride(1); p.out_gs = G > 1 ? O.stride(0) : 0;
-  p.epi = (int)epi; p.out_f32 = out_f32; p.accumulate = accumulate;
-  TORCH_CHECK(!accumulate || out_f32, "gemm: accumulate needs an fp32 output");
-  const int vec = out_f32 ? 4 : 8;
-  TORCH_CHECK(p.ldo % vec == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (p.out_gs % vec) == 0,
-              "gemm: output must allow 16-byte row stores");
-  if (out2_.has_value() && out2_->defined()) {
-    torch::Tensor O2 = as3(*out2_);
-    TORCH_CHECK(O2.scalar_type() == torch::kBFloat16 && O2.stride(2) == 1 && O2.size(1) == M, "gemm: out2");
-    p.out2 = O2.data_ptr(); p.ldo2 = (int)O2.stride(1); p.out2_gs = G > 1 ? O2.stride(0) : 0;
-    TORCH_CHECK(p.ldo2 % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out2) & 15) == 0, "gemm: out2 alignment");
-  }
-  TORCH_CHECK(epi != EPI_RELU2 || p.out2 != nullptr, "gemm: relu2 epilogue needs out2 for the pre-activation");
-  if (aux_.has_value() && aux_->defined()) {
-    if (epi == EPI_ROWSCALE) {
-      TORCH_CHECK(aux_->scalar_type() == torch::kFloat32 && aux_->is_contiguous(), "gemm: row scale must be fp32");
-      p.aux = aux_->data_ptr(); p.aux_gs = G > 1 ? M : 0;
-    } else {
-      torch::Tensor X = as3(*aux_);
-      TORCH_CHECK(X.scalar_type() == torch::kBFloat16 && X.stride(2) == 1 && X.size(1) == M &&
-                  X.size(2) == (epi == EPI_DSWIGLU ? 2 * N : N), "gemm: aux");
-      p.aux = X.data_ptr(); p.ldaux = (int)X.stride(1); p.aux_gs = G > 1 ? X.stride(0) : 0;
-      TORCH_CHECK(p.ldaux % 8 == 0 && (reinterpret_cast<uintptr_t>(p.aux) & 15) == 0, "gemm: aux alignment");
-    }
-  }
-  TORCH_CHECK((epi != EPI_DRELU2 && epi != EPI_ROWSCALE && epi != EPI_DSWIGLU) || p.aux != nullptr, "gemm: epilogue needs aux");
-  TORCH_CHECK(epi != EPI_DSWIGLU || (!out_f32 && N % 8 == 0 && M >= 256 && use_pair_kernel()),
-              "gemm: the SwiGLU-backward epilogue writes bf16, needs a hidden width that is a multiple of 8 and the pair kernel (>= 256 rows)");
-  if (counts_.has_value() && counts_->defined() && count_mode != 0) {
-    TORCH_CHECK(counts_->is_cuda() && counts_->scalar_type() == torch::kInt32 && counts_->is_contiguous() &&
-                counts_->numel() >= G, "gemm: counts must be a contiguous int32 CUDA tensor with one entry per group");
-    TORCH_CHECK(count_mode == 1 || count_mode == 2, "gemm: count_mode 1 (rows) or 2 (contraction length)");
-    p.counts = counts_->data_ptr<int>(); p.count_mode = (int)count_mode;
-  }
-  TORCH_CHECK(epi != EPI_SWIGLU || (!out_f32 && N % 16 == 0),
-              "gemm: the SwiGLU epilogue writes bf16 and needs column halves of a multiple of 8 (16-byte TMA coordinates)");
-  p.status = status_word(a.get_device());
-  launch_gemm(A.data_ptr(), A.stride(1), G > 1 ? A.stride(0) : 0, a_mn, B.data_ptr(), B.stride(1), G > 1 ? B.stride(0) : 0,
-              b_mn, p, at::cuda::getCurrentCUDAStream(), sm_count());
-  return out;
-}
-
-// Segmented GEMM over peer buffers (expert parallelism without a separate all-to-all):
-//   A rows of segment s come from `a_ptrs[s]`, a (a_groups, seg_M, K) bf16 buffer (a peer GPU's dispatch buffer);
-//   group g of this launch reads A group `a_g_off + g`;
-//   the result goes to `out_local` (G, n_seg*seg_M, N) or, when `out_ptrs` is given, rows of segment s go to
-//   `out_ptrs[s]`, a (.., seg_M, N) buffer with row pitch `out_ld` and group pitch `out_gs` at group `out_g_off + g`.
-torch::Tensor gemm_peer(std::vector<int64_t> a_ptrs, int64_t seg_M, int64_t K, int64_t a_groups, int64_t a_pitch,
-                        int64_t a_gs, int64_t a_g_off, torch::Tensor b, bool b_mn, c10::optional<torch::Tensor> out_local,
-                        std::vector<int64_t> out_ptrs, int64_t out_ld, int64_t out_gs, int64_t out_g_off,
-                        c10::optional<torch::Tensor> out2_, c10::optional<torch::Tensor> aux_, int64_t epi, int64_t groups) {
-  TORCH_CHECK(b.is_cuda() && b.scalar_type() == torch::kBFloat16, "gemm_peer: bf16 B");
-  const c10::cuda::CUDAGuard guard(b.device());
-  const int G = (int)groups, n_seg = (int)a_ptrs.size();
-  torch::Tensor B = b.dim() == 2 ? b.unsqueeze(0) : b;
-  TORCH_CHECK(B.size(0) == G && B.stride(2) == 1, "gemm_peer: B groups");
-  const int N = b_mn ? B.size(2) : B.size(1), Kb = b_mn ? B.size(1) : B.size(2);
-  TORCH_CHECK(Kb == K, "gemm_peer: K mismatch");
-  const int M = n_seg * (int)seg_M;
-  GemmParams p{};
-  p.M = M; p.N = N; p.K = (int)K; p.G = G;
-  p.epi = (int)epi; p.a_g_off = (int)a_g_off;
-  torch::Tensor out;
-  if (!out_ptrs.empty()) {
-    TORCH_CHECK((int)out_ptrs.size() == n_seg, "gemm_peer: one output base per segment");
-    for (int i = 0; i < n_seg; ++i) p.out_seg[i] = reinterpret_cast<void*>(out_ptrs[i]);
-    p.out_seg_on = 1; p.out_g_off = (int)out_g_off; p.ldo = (int)out_ld; p.out_gs = out_gs;
-    p.out = p.out_seg[0];
-    TORCH_CHECK(out_ld % 8 == 0 && out_gs % 8 == 0, "gemm_peer: output pitches");
-  } else {
-    out = (out_local.has_value() && out_local->defined()) ? *out_local : torch::empty({G, M, N}, b.options());
-    TORCH_CHECK(out.dim() == 3 && out.size(0) == G && out.size(1) == M && out.size(2) == N && out.stride(2) == 1, "gemm_peer: out");
-    p.out = out.data_ptr(); p.ldo = (int)out.stride(1); p.out_gs = out.stride(0);
-  }
-  if (out2_.has_value() && out2_->defined()) {
-    TORCH_CHECK(out2_->dim() == 3 && out2_->size(1) == M && out2_->stride(2) == 1, "gemm_peer: out2");
-    p.out2 = out2_->data_ptr(); p.ldo2 = (int)out2_->stride(1); p.out2_gs = out2_->stride(0);
-  }
-  if (aux_.has_value() && aux_->defined()) {
-    TORCH_CHECK(aux_->dim() == 3 && aux_->size(1) == M && aux_->stride(2) == 1, "gemm_peer: aux");
-    p.aux = aux_->data_ptr(); p.ldaux = (int)aux_->stride(1); p.aux_gs = aux_->stride(0);
-  }
-  TORCH_CHECK(epi != EPI_RELU2 || p.out2 != nullptr, "gemm_peer: relu2 epilogue needs out2");
-  p.status = status_word(b.get_device());
-  std::vector<const void*> list(n_seg);
-  for (int i = 0; i < n_seg; ++i) list[i] = reinterpret_cast<const void*>(a_ptrs[i]);
-  launch_gemm_seg(list.data(), n_seg, (int)seg_M, (int)a_groups, a_pitch, a_gs, false, B.data_ptr(), B.stride(1),
-                  G > 1 ? B.stride(0) : 0, b_mn, p, at::cuda::getCurrentCUDAStream(), sm_count());
-  return out;
 }
 
 }  // namespace mb

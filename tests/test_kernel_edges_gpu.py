@@ -95,3 +95,24 @@ def test_ce_rows_sizes(n, V):
     out = torch.empty(n, device="cuda")
     _ext.C().ce_rows(lg, y, out, None, None, None)
     assert _rel(out, loss.detach()) < 1e-5 and _rel(lg, x.grad) < 4e-3
+
+
+# ------------------------------------------------------------------------------------------------ split contraction
+@pytest.mark.parametrize("M,N,K", [(256, 8, 2048), (264, 256, 2056), (1000, 256, 50304), (512, 1536, 4096), (300, 264, 8200), (2048, 2048, 2048)])
+def test_gemm_split_contraction(M, N, K):
+    """Few output tiles and a long contraction: all operand layouts, bf16 / fp32 / accumulating outputs."""
+    from memarch_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A, B = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    want = A.double() @ B.double().t()
+    for a_mn in (False, True):
+        for b_mn in (False, True):
+            a = A.t().contiguous() if a_mn else A
+            b = B.t().contiguous() if b_mn else B
+            if (a_mn and M % 8) or (b_mn and N % 8):
+                continue
+            assert _rel(gemm(a, b, a_mn=a_mn, b_mn=b_mn), want) < 4e-3
+            assert _rel(gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32), want) < 1e-5
+            acc = torch.ones(M, N, device="cuda")
+            gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=acc, out_dtype=torch.float32, accumulate=True)
+            assert _rel(acc, want + 1) < 1e-5
