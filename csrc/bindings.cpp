@@ -62,6 +62,11 @@ std::vector<torch::Tensor> reread_bwd(torch::Tensor dgot, torch::Tensor dcostw, 
 std::vector<torch::Tensor> rope_route_topk(torch::Tensor S, torch::Tensor lval, torch::Tensor lp, torch::Tensor avalid,
                                            torch::Tensor open_from, int64_t H, int64_t K, int64_t q0, double scale);
 std::vector<torch::Tensor> attn_fwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, int64_t window, double scale);
+std::vector<torch::Tensor> route_fwd(torch::Tensor x, torch::Tensor w, torch::Tensor real, torch::Tensor k_tok, int64_t k, int64_t C);
+std::vector<torch::Tensor> route_bwd(torch::Tensor x, torch::Tensor w, torch::Tensor real, torch::Tensor k_tok, torch::Tensor probs,
+                                     torch::Tensor top_e, torch::Tensor flat_idx, torch::Tensor aux_grad, int64_t C,
+                                     c10::optional<torch::Tensor> d_wt, c10::optional<torch::Tensor> d_wtab,
+                                     c10::optional<torch::Tensor> d_aux, c10::optional<torch::Tensor> d_probs);
 int64_t attn_status_read();
 std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor dout, torch::Tensor lse,
                                        torch::Tensor delta, int64_t window, double scale);
@@ -114,6 +119,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("lock_find_bucket", &mb::lock_find_bucket);
   m.def("attn_fwd_tc", &mb::attn_fwd_tc, "causal / sliding-window attention forward on tcgen05 (head dim 64)");
   m.def("attn_status_read", &mb::attn_status_read);
+  m.def("route_fwd", &mb::route_fwd, "router, slotting and auxiliary loss of an expert layer");
+  m.def("route_bwd", &mb::route_bwd);
   m.def("attn_bwd_tc", &mb::attn_bwd_tc, "causal / sliding-window attention backward on tcgen05 (head dim 64)");
   m.def("attn_bwd_status_read", &mb::attn_bwd_status_read);
   m.def("mem_read_fwd", &mb::mem_read_fwd);

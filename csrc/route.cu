@@ -1,0 +1,346 @@
+// The router of an expert layer in two launches forward and two (and a clear) backward.
+//
+// Forward 1 (route_fwd_kernel): logits = x W^T in fp32 from the bf16 rows, softmax, top-k by probability (ties: smaller
+// expert first), budget k_tok, renormalised weights, and per block of 32 tokens the number of choices and the sum of
+// probabilities of every expert.
+// Forward 2 (route_place_kernel): choices in (token, choice) order take the next free place of their expert, places beyond C
+// drop; a block's first free places are the sums of the earlier blocks' numbers.  Fills the slot table, its inverse,
+// the combine weights of the places, and (first block) filled places, dropped share and the Switch auxiliary loss
+//   aux = E * sum_e (choices of e / all choices) * (mean probability of e over the real tokens).
+// Backward 1 (route_dx_kernel): gradient of the logits from the gradients of the weights, of the place weights and of aux, and
+// dx = dlogits W.  Backward 2 (route_dw_kernel): dW = dlogits^T x.
+// All of it is memory-bound on x (33 MB for 8192 x 2048).  A warp takes 8 tokens at a time, so that W (E x d fp32) is read
+// once per 8 tokens and mostly from L1.  ROUTE_TIME
+#include "common.cuh"
+#include "route_api.h"
+
+namespace mb {
+
+constexpr int RT_WARPS = 4, RT_TOK = ROUTE_TOK / RT_WARPS;      // 8 tokens per warp
+
+__device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t q[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { const float2 f = unpack_bf16(q[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
+}
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+__global__ void __launch_bounds__(RT_WARPS * 32) route_fwd_kernel(RouteArgs a) {
+  __shared__ float ps_sh[ROUTE_E];
+  __shared__ int cnt_sh[ROUTE_E], real_sh;
+  extern __shared__ float lg_sh[];                       // (ROUTE_TOK, E) logits
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = a.E;
+  for (int i = threadIdx.x; i < E; i += blockDim.x) { ps_sh[i] = 0.f; cnt_sh[i] = 0; }
+  if (threadIdx.x == 0) real_sh = 0;
+  __syncthreads();
+  const int n0 = blockIdx.x * ROUTE_TOK + warp * RT_TOK;
+  const int nt = min(RT_TOK, a.N - n0);                  // may be <= 0
+  const bf16* X = reinterpret_cast<const bf16*>(a.x);
+  float* lg = lg_sh + warp * RT_TOK * E;
+  // 8 tokens x 4 experts at a time: every lane sums its columns, then the 32 sums are reduced over the lanes, the lane that
+  // ends up with sum v = token * 4 + expert writes it
+  for (int e0 = 0; e0 < E; e0 += 4) {
+    float acc[32];
+#pragma unroll
+    for (int v = 0; v < 32; ++v) acc[v] = 0.f;
+    if (nt > 0) {
+      for (int c = lane * 8; c < a.d; c += 256) {
+        float w[4][8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (e0 + j < E) load8(a.w + (long long)(e0 + j) * a.d + c, w[j]);
+          else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) w[j][u] = 0.f;
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < RT_TOK; ++t) {
+          float x[8];
+          load8(X + (long long)(n0 + min(t, nt - 1)) * a.d + c, x);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc[t * 4 + j] = fmaf(x[u], w[j][u], acc[t * 4 + j]);
+        }
+      }
+    }
+    // reduce-scatter: after the step with offset o a lane holds o sums, of those whose index agrees with its own bits
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int v = 0; v < o; ++v) {
+        const float send = up ? acc[v] : acc[v + o], keep = up ? acc[v + o] : acc[v];
+        acc[v] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    const int t = lane >> 2, e = e0 + (lane & 3);
+    if (e < E) lg[t * E + e] = acc[0];
+  }
+  __syncwarp();
+  for (int t = 0; t < nt; ++t) {
+    const long long n = n0 + t;
+    float v[ROUTE_E / 32];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < ROUTE_E / 32; ++i) {
+      const int e = lane + 32 * i;
+      v[i] = e < E ? lg[t * E + e] : -INFINITY;
+      mx = fmaxf(mx, v[i]);
+    }
+    mx = warp_max(mx);
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROUTE_E / 32; ++i) { v[i] = lane + 32 * i < E ? expf(v[i] - mx) : 0.f; sum += v[i]; }
+    const float inv = 1.f / warp_sum(sum);
+    const bool is_real = a.real[n];
+    const int kt = (int)a.k_tok[n];
+#pragma unroll
+    for (int i = 0; i < ROUTE_E / 32; ++i) {
+      const int e = lane + 32 * i;
+      v[i] *= inv;
+      if (e < E) {
+        a.probs[n * E + e] = v[i];
+        if (is_real) atomicAdd(&ps_sh[e], v[i]);
+      } else {
+        v[i] = -1.f;
+      }
+    }
+    float mine_p = 0.f, kept = 0.f;                      // lane j < k ends up with choice j
+    int mine_e = E;
+    for (int j = 0; j < a.k; ++j) {
+      float bp = -1.f;
+      int be = ROUTE_E;
+#pragma unroll
+      for (int i = 0; i < ROUTE_E / 32; ++i)
+        if (v[i] > bp) { bp = v[i]; be = lane + 32 * i; }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float op = __shfl_xor_sync(0xffffffffu, bp, o);
+        const int oe = __shfl_xor_sync(0xffffffffu, be, o);
+        if (op > bp || (op == bp && oe < be)) { bp = op; be = oe; }
+      }
+#pragma unroll
+      for (int i = 0; i < ROUTE_E / 32; ++i) if (be == lane + 32 * i) v[i] = -1.f;
+      if (j < kt) kept += bp;
+      if (lane == j) { mine_p = bp; mine_e = be; }
+    }
+    if (lane < a.k) {
+      const bool keep = lane < kt && mine_e < E;         // mine_e is out of range only where the logits are NaN
+      mine_e = min(mine_e, E);
+      a.top_e[n * a.k + lane] = mine_e;
+      a.wt[n * a.k + lane] = keep ? mine_p / fmaxf(kept, 1e-9f) : 0.f;
+      a.flat_idx[n * a.k + lane] = keep ? mine_e : E;    // the expert for now; route_place_kernel turns it into a place
+      if (keep) atomicAdd(&cnt_sh[mine_e], 1);
+    }
+    if (lane == 0 && is_real) atomicAdd(&real_sh, 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < E; i += blockDim.x) {
+    a.hist[(long long)blockIdx.x * E + i] = cnt_sh[i];
+    a.psum[(long long)blockIdx.x * E + i] = ps_sh[i];
+  }
+  if (threadIdx.x == 0) a.n_real[blockIdx.x] = real_sh;
+}
+
+__global__ void __launch_bounds__(256) route_place_kernel(RouteArgs a) {
+  __shared__ int base[ROUTE_E], total[ROUTE_E];
+  __shared__ float ps[ROUTE_E];
+  __shared__ unsigned char ch[ROUTE_TOK * ROUTE_K];
+  __shared__ int real_sh;
+  const int E = a.E, nb = gridDim.x, tid = threadIdx.x;
+  const bool first = blockIdx.x == 0;
+  for (int e = tid; e < E; e += blockDim.x) { base[e] = 0; total[e] = 0; ps[e] = 0.f; }
+  if (tid == 0) real_sh = 0;
+  __syncthreads();
+  // sums over the blocks: a thread takes one expert and every (256 / E)-th block
+  const int lanes = blockDim.x / E;
+  if (tid < lanes * E) {
+    const int e = tid % E;
+    int before = 0, all = 0;
+    float p = 0.f;
+    for (int b = tid / E; b < nb; b += lanes) {
+      const int h = a.hist[(long long)b * E + e];
+      all += h;
+      if (b < (int)blockIdx.x) before += h;
+      if (first) p += a.psum[(long long)b * E + e];
+    }
+    atomicAdd(&base[e], before);
+    atomicAdd(&total[e], all);
+    if (first) atomicAdd(&ps[e], p);
+  }
+  if (first) {
+    int r = 0;
+    for (int b = tid; b < nb; b += blockDim.x) r += a.n_real[b];
+    if (r) atomicAdd(&real_sh, r);
+  }
+  const int n0 = blockIdx.x * ROUTE_TOK, nch = min(ROUTE_TOK, a.N - n0) * a.k;
+  for (int i = tid; i < nch; i += blockDim.x) ch[i] = (unsigned char)a.flat_idx[(long long)n0 * a.k + i];
+  __syncthreads();
+  const long long EC = (long long)E * a.C;
+  for (int i = tid; i < nch; i += blockDim.x) {
+    const int e = ch[i];
+    long long place = EC;
+    if (e < E) {
+      int rank = base[e];
+      for (int j = 0; j < i; ++j) rank += ch[j] == e;
+      if (rank < a.C) {
+        place = (long long)e * a.C + rank;
+        a.table[place] = n0 + i / a.k;
+        a.wtab[place] = a.wt[(long long)n0 * a.k + i];
+      }
+    }
+    a.flat_idx[(long long)n0 * a.k + i] = place;
+  }
+  // the places nobody takes
+  for (long long q = blockIdx.x * (long long)blockDim.x + tid; q < EC; q += (long long)nb * blockDim.x)
+    if ((int)(q % a.C) >= total[q / a.C]) { a.table[q] = a.N; a.wtab[q] = 0.f; }
+  if (first) {
+    for (int e = tid; e < E; e += blockDim.x) a.counts[e] = min(total[e], a.C);
+    if (tid == 0) {
+      int kept = 0, placed = 0;
+      for (int e = 0; e < E; ++e) { kept += total[e]; placed += min(total[e], a.C); }
+      *a.dropped = 1.f - (float)placed / (float)max(kept, 1);
+      const float scale = (float)E / ((float)max(kept, 1) * (float)max(real_sh, 1));
+      float s = 0.f;
+      for (int e = 0; e < E; ++e) {
+        const float g = scale * (float)total[e];
+        a.aux_grad[e] = g;
+        s += g * ps[e];
+      }
+      *a.aux = s;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(RT_WARPS * 32) route_dx_kernel(RouteArgs a) {
+  extern __shared__ float dl_sh[];                       // (ROUTE_TOK, E)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = a.E;
+  const int n0 = blockIdx.x * ROUTE_TOK + warp * RT_TOK;
+  const int nt = min(RT_TOK, a.N - n0);
+  float* dl = dl_sh + warp * RT_TOK * E;
+  const float d_aux = a.d_aux ? *a.d_aux : 0.f;
+  for (int t = 0; t < RT_TOK; ++t) {
+    if (t >= nt) {                                       // absent tokens of the last block
+      for (int e = lane; e < E; e += 32) dl[t * E + e] = 0.f;
+      continue;
+    }
+    const long long n = n0 + t;
+    const int kt = (int)a.k_tok[n];
+    const bool is_real = a.real[n];
+    // lane j < k: choice j
+    int te = ROUTE_E;
+    float tp = 0.f, g = 0.f;
+    if (lane < a.k) {
+      te = (int)a.top_e[n * a.k + lane];
+      if (lane < kt && te < E) {
+        tp = a.probs[n * E + te];
+        if (a.d_wt) g = a.d_wt[n * a.k + lane];
+        if (a.d_wtab) {
+          const long long place = a.flat_idx[n * a.k + lane];
+          if (place < (long long)E * a.C) g += a.d_wtab[place];
+        }
+      }
+    }
+    const float s0 = warp_sum(tp), s = fmaxf(s0, 1e-9f);
+    const float dot = warp_sum(g * tp) / s;
+    const float dtp = lane < kt && lane < a.k ? (g - (s0 < 1e-9f ? 0.f : dot)) / s : 0.f;
+    float pr[ROUTE_E / 32], dp[ROUTE_E / 32], pd = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROUTE_E / 32; ++i) {
+      const int e = lane + 32 * i;
+      pr[i] = e < E ? a.probs[n * E + e] : 0.f;
+      dp[i] = e < E ? (a.d_probs ? a.d_probs[n * E + e] : 0.f) + (is_real ? d_aux * a.aux_grad[e] : 0.f) : 0.f;
+      for (int j = 0; j < a.k; ++j) {
+        const int ej = __shfl_sync(0xffffffffu, te, j);
+        const float dj = __shfl_sync(0xffffffffu, dtp, j);
+        if (ej == e) dp[i] += dj;
+      }
+      pd += pr[i] * dp[i];
+    }
+    pd = warp_sum(pd);
+#pragma unroll
+    for (int i = 0; i < ROUTE_E / 32; ++i) {
+      const int e = lane + 32 * i;
+      if (e < E) {
+        const float v = pr[i] * (dp[i] - pd);
+        dl[t * E + e] = v;
+        a.dl[n * E + e] = v;
+      }
+    }
+  }
+  __syncwarp();
+  if (nt <= 0) return;
+  bf16* DX = reinterpret_cast<bf16*>(a.dx);
+  for (int c = lane * 8; c < a.d; c += 256) {
+    float acc[RT_TOK][8];
+#pragma unroll
+    for (int t = 0; t < RT_TOK; ++t)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[t][u] = 0.f;
+    for (int e = 0; e < E; ++e) {
+      float w[8];
+      load8(a.w + (long long)e * a.d + c, w);
+#pragma unroll
+      for (int t = 0; t < RT_TOK; ++t) {
+        const float v = dl[t * E + e];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc[t][u] = fmaf(v, w[u], acc[t][u]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < RT_TOK; ++t)
+      if (t < nt)
+        *reinterpret_cast<uint4*>(DX + (long long)(n0 + t) * a.d + c) =
+            make_uint4(pack_bf16(acc[t][0], acc[t][1]), pack_bf16(acc[t][2], acc[t][3]), pack_bf16(acc[t][4], acc[t][5]), pack_bf16(acc[t][6], acc[t][7]));
+  }
+}
+
+// grid (column tiles of 512, token runs, groups of 8 experts): a thread owns two columns of 8 experts
+constexpr int DW_RUN = 64;
+__global__ void __launch_bounds__(256) route_dw_kernel(RouteArgs a) {
+  __shared__ __align__(16) float g[DW_RUN][8];
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 2, e0 = blockIdx.z * 8;
+  const int n0 = blockIdx.y * DW_RUN, n1 = min(a.N, n0 + DW_RUN);
+  for (int i = threadIdx.x; i < (n1 - n0) * 8; i += 256) {
+    const int e = e0 + (i & 7);
+    g[i >> 3][i & 7] = e < a.E ? a.dl[(long long)(n0 + (i >> 3)) * a.E + e] : 0.f;
+  }
+  __syncthreads();
+  if (c >= a.d) return;
+  float acc[8][2] = {};
+  const uint32_t* X = reinterpret_cast<const uint32_t*>(a.x);
+  const long long pitch = a.d / 2;
+#pragma unroll 8
+  for (int n = n0; n < n1; ++n) {
+    const float2 x = unpack_bf16(X[n * pitch + c / 2]);
+    const float4 g0 = *reinterpret_cast<const float4*>(g[n - n0]), g1 = *reinterpret_cast<const float4*>(g[n - n0] + 4);
+    const float ge[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { acc[j][0] = fmaf(ge[j], x.x, acc[j][0]); acc[j][1] = fmaf(ge[j], x.y, acc[j][1]); }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (e0 + j < a.E) {
+      float* dst = a.dw + (long long)(e0 + j) * a.d + c;
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(acc[j][0]), "f"(acc[j][1]) : "memory");
+    }
+}
+
+void route_fwd_launch(const RouteArgs& a) {
+  const int nb = route_blocks(a.N);
+  route_fwd_kernel<<<nb, RT_WARPS * 32, (size_t)ROUTE_TOK * a.E * 4, a.stream>>>(a);
+  route_place_kernel<<<nb, 256, 0, a.stream>>>(a);
+}
+void route_bwd_launch(const RouteArgs& a) {
+  cudaMemsetAsync(a.dw, 0, sizeof(float) * (size_t)a.E * a.d, a.stream);
+  route_dx_kernel<<<route_blocks(a.N), RT_WARPS * 32, (size_t)ROUTE_TOK * a.E * 4, a.stream>>>(a);
+  route_dw_kernel<<<dim3((a.d + 511) / 512, (a.N + DW_RUN - 1) / DW_RUN, (a.E + 7) / 8), 256, 0, a.stream>>>(a);
+}
+
+}  // namespace mb

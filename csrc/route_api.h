@@ -1,0 +1,40 @@
+// Host interface of the fused MoE router (route.cu): plain pointers, no torch types.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace mb {
+
+constexpr int ROUTE_E = 128, ROUTE_K = 8, ROUTE_TOK = 32;     // experts, choices per token, tokens per block
+
+struct RouteArgs {
+  const void* x;               // (N, d) bf16
+  const float* w;              // (E, d)
+  const bool* real;            // (N)
+  const long long* k_tok;      // (N)
+  int N, d, E, k, C;           // k choices per token, C places per expert
+  // forward results
+  float* probs;                // (N, E)
+  long long* top_e;            // (N, k)
+  float* wt;                   // (N, k)
+  float* wtab;                 // (E * C)
+  long long* table;            // (E * C): token of every place, N = empty
+  long long* flat_idx;         // (N, k): place of every choice, E * C = none
+  float* dropped;              // scalar
+  float* aux;                  // scalar
+  float* aux_grad;             // (E): d aux / d (sum of probs of expert e over the real tokens)
+  int* counts;                 // (E): filled places
+  int* hist;                   // workspace (blocks, E)
+  float* psum;                 // workspace (blocks, E)
+  int* n_real;                 // workspace (blocks)
+  // backward (null: no gradient arrives there)
+  const float *d_wt, *d_wtab, *d_aux, *d_probs;
+  float* dl;                   // workspace (N, E): gradient of the logits
+  void* dx;                    // (N, d) bf16
+  float* dw;                   // (E, d)
+  cudaStream_t stream;
+};
+inline int route_blocks(int N) { return (N + ROUTE_TOK - 1) / ROUTE_TOK; }
+void route_fwd_launch(const RouteArgs& a);
+void route_bwd_launch(const RouteArgs& a);
+
+}  // namespace mb

@@ -192,9 +192,47 @@ def moe_route(xf, router_w, real, k_tok, k_max, E):
     return ref.moe_route(xf, router_w, real, k_tok, k_max, E)
 
 
+class _RouteSlot(torch.autograd.Function):
+    """Router product, softmax, top-k, budget, slotting, place weights and the auxiliary loss in two kernels; backward to
+    the rows and the router weight in two (`csrc/route.cu`)."""
+
+    @staticmethod
+    def forward(ctx, xf, router_w, real, k_tok, k_max, C):
+        w, wtab, aux, probs, table, flat_idx, dropped, counts, top_e, aux_grad = _ext.C().route_fwd(
+            xf, router_w, real, k_tok, int(k_max), int(C))
+        _ext.count(2)
+        ctx.save_for_backward(xf, router_w, real, k_tok, probs, top_e, flat_idx, aux_grad)
+        ctx.C = int(C)
+        ctx.mark_non_differentiable(table, flat_idx, dropped, counts)
+        ctx.set_materialize_grads(False)
+        return w, wtab, aux, probs, table, flat_idx, dropped, counts
+
+    @staticmethod
+    def backward(ctx, dw, dwtab, daux, dprobs, *_):
+        if dw is None and dwtab is None and daux is None and dprobs is None:
+            return None, None, None, None, None, None
+        c = lambda t: None if t is None else t.contiguous()
+        dx, dW = _ext.C().route_bwd(*ctx.saved_tensors, ctx.C, c(dw), c(dwtab), c(daux), c(dprobs))
+        _ext.count(2)
+        return dx, dW, None, None, None, None
+
+
+def _fused_route(xf, router_w, real, k_tok, k_max, E, C):
+    """Whether the fused kernels take these arguments: bf16 rows, an fp32 router, 16-byte rows."""
+    return (_ext.use_cuda(xf) and xf.dim() == 2 and xf.dtype == torch.bfloat16 and xf.shape[1] % 8 == 0 and xf.shape[0] > 0
+            and router_w.dtype == torch.float32 and router_w.shape == (E, xf.shape[1]) and router_w.is_contiguous()
+            and 1 <= k_max <= min(8, E) and E <= 128 and C >= 1 and xf.is_contiguous()
+            and real.dtype == torch.bool and k_tok.dtype == torch.int64 and real.is_contiguous() and k_tok.is_contiguous()
+            and xf.data_ptr() % 16 == 0 and router_w.data_ptr() % 16 == 0)
+
+
 def route_and_slot(xf, router_w, real, k_tok, k_max, E, C, want_counts=False):
     """Router + capacity slotting.  Returns (w (N,k), table, wtab, flat_idx, aux, dropped, probs) and, with
     `want_counts`, the filled places per expert (int32 on the GPU, None on CPU) as an eighth value."""
+    if _fused_route(xf, router_w, real, k_tok, k_max, E, C):
+        w, wtab, aux, probs, table, flat_idx, dropped, counts = _RouteSlot.apply(xf, router_w, real, k_tok, k_max, C)
+        out = (w, table, wtab, flat_idx, aux, dropped, probs)
+        return out + (counts,) if want_counts else out
     probs, top_e, keep, w, e_flat, aux = moe_route(xf, router_w, real, k_tok, k_max, E)
     counts = None
     with torch.no_grad():

@@ -116,3 +116,32 @@ def test_gemm_split_contraction(M, N, K):
             acc = torch.ones(M, N, device="cuda")
             gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=acc, out_dtype=torch.float32, accumulate=True)
             assert _rel(acc, want + 1) < 1e-5
+
+
+# ------------------------------------------------------------------------------------------------ routing
+@pytest.mark.parametrize("N,d,E,k,C", [(1, 8, 1, 1, 1), (31, 64, 3, 2, 7), (33, 256, 8, 2, 64), (100, 264, 48, 4, 3), (700, 2048, 8, 2, 176), (257, 512, 128, 8, 9), (4000, 768, 16, 2, 626)])
+def test_route_and_slot_fused(N, d, E, k, C):
+    """Every output and both gradients of the fused router against the PyTorch statement (fp32 router product)."""
+    from memarch_b200 import ops
+    from memarch_b200.ops import ref
+    g = torch.Generator().manual_seed(N + E)
+    x = torch.randn(N, d, generator=g).bfloat16()
+    w = torch.randn(E, d, generator=g) * d ** -0.5
+    real = torch.rand(N, generator=g) > 0.2
+    k_tok = torch.randint(1, k + 1, (N,), generator=g) * real
+    gw, gt, gp = torch.randn(N, k, generator=g), torch.randn(E * C, generator=g), torch.randn(N, E, generator=g)
+    xc, wc = x.float().requires_grad_(), w.clone().requires_grad_()
+    probs, top_e, keep, wt, e_flat, aux = ref.moe_route(xc, wc, real, k_tok, k, E)
+    table, _, flat, dropped = ref.moe_slots(e_flat, wt.detach(), E, C)
+    ok = flat < E * C
+    wtab = torch.zeros(E * C + 1).scatter(0, flat.reshape(-1), (wt * ok).reshape(-1))[:-1]
+    ((wt * gw).sum() + (wtab * gt).sum() + (probs * gp).sum() + 3 * aux).backward()
+    xg, wg = x.cuda().requires_grad_(), w.cuda().requires_grad_()
+    o = ops.route_and_slot(xg, wg, real.cuda(), k_tok.cuda(), k, E, C, want_counts=True)
+    assert torch.equal(o[1].cpu(), table) and torch.equal(o[3].cpu(), flat)
+    assert torch.equal(o[7].cpu().long(), torch.bincount(flat[ok] // C, minlength=E))
+    for a, b in ((o[0], wt), (o[2], wtab), (o[6], probs)):
+        assert (a.cpu() - b).abs().max() < 1e-5
+    assert abs(float(o[4]) - float(aux)) < 1e-5 * max(1.0, float(aux)) and abs(float(o[5]) - float(dropped)) < 1e-6
+    ((o[0] * gw.cuda()).sum() + (o[2] * gt.cuda()).sum() + (o[6] * gp.cuda()).sum() + 3 * o[4]).backward()
+    assert _rel(xg.grad.cpu(), xc.grad) < 4e-3 and _rel(wg.grad.cpu(), wc.grad) < 1e-4
