@@ -17,27 +17,9 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "instinct_args.h"
 
 namespace mb {
-
-struct InstinctArgs {
-  void* p;                 // weight (bf16 or fp32)
-  const void* g;           // gradient
-  void* m;                 // momentum
-  float* w;                // exact fp32 copy of a bf16 weight, or nullptr
-  int p_bf16, g_bf16, m_bf16;
-  const float* gain;       // device scalar: gain of this weight on the current situation card
-  const float* stake;      // device scalar
-  const float* lr;         // device scalar: lr * scale
-  float beta, wd;
-  int sr;                  // stochastic rounding of bf16 stores
-  const long long* seed;   // device step counter for the rounding hash
-  unsigned salt;
-  const bool* frozen;      // optional mask over the leading dimension: frozen slices keep their weights
-  long long frozen_stride;
-  long long E, R, C;
-  void* shadow;            // optional bf16 copy of an fp32 weight, refreshed by `apply` (what the GEMMs read)
-};
 
 __device__ __forceinline__ float ldv(const void* base, long long i, int is_bf16) {
   return is_bf16 ? __bfloat162float(reinterpret_cast<const bf16*>(base)[i]) : reinterpret_cast<const float*>(base)[i];
@@ -71,6 +53,15 @@ __device__ __forceinline__ float4 mom4(const InstinctArgs& a, long long i, float
 __device__ __forceinline__ float mom1(const InstinctArgs& a, long long i, float& g) {
   g = ldv(a.g, i, a.g_bf16);
   return a.beta * ldv(a.m, i, a.m_bf16) + (1.f - a.beta) * g;
+}
+
+__device__ __forceinline__ void cp_async16(void* s, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(s)), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_async8(void* s, const void* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(s)), "l"(g) : "memory");
 }
 
 // Column scales of expert e into shared memory: dst[c] = scale(sum1[e,c]) * scale(sum2[e,c]) (either may be null).
@@ -165,6 +156,163 @@ __global__ void instinct_stat_cols(InstinctArgs a, const float* __restrict__ col
   }
 #pragma unroll
   for (int j = 0; j < VEC; ++j) atomicAdd(colsq_out + e * a.C + c + j, acc[j]);
+}
+
+// The same for rows of whole 16-byte pieces (C % 256 == 0): 32 lanes x 8 columns by 8 row lanes, four rows of both arrays in
+// flight per thread, the eight partial sums of a column meet in shared memory, so a block adds to a column once.  With
+// one row lane per column (above) filling the chip on a single matrix takes up to 100 blocks per column, whose additions to the
+// same address then cost more than the reading: 15 us per pass of a (4096, 1024) weight against 8.  A stack of experts has
+// enough strips for the form above, which keeps more rows in flight there (82 against 142 us for 8 x 2048 x 6144).
+__device__ __forceinline__ void ld8(const void* base, long long i, int is_bf16, float* o) {
+  if (is_bf16) {
+    const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(base) + i);
+    const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y; o[4] = c.x; o[5] = c.y; o[6] = d.x; o[7] = d.y;
+  } else {
+    const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i);
+    const float4 b = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + i + 4);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+  }
+}
+static __global__ void __launch_bounds__(256) instinct_stat_cols_s8(InstinctArgs a, const float* __restrict__ colsum, float col_count,
+                                                                    const float* __restrict__ rowsum, float row_count,
+                                                                    float* __restrict__ colsq_out, int rows_per_block) {
+  extern __shared__ float rsm[];
+  __shared__ float part[8][256];
+  const long long e = blockIdx.z;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long c = (long long)blockIdx.x * 256 + tx * 8;
+  const long long r0 = (long long)blockIdx.y * rows_per_block, r1 = min(a.R, r0 + rows_per_block);
+  if (rowsum) {
+    for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) rsm[r - r0] = scale_of(rowsum[e * a.R + r], row_count);
+    __syncthreads();
+  }
+  const float b = a.beta, b1 = 1.f - a.beta;
+  float cs[8], acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { cs[j] = colsum ? scale_of(colsum[e * a.C + c + j], col_count) : 1.f; acc[j] = 0.f; }
+#pragma unroll 4
+  for (long long r = r0 + ty; r < r1; r += 8) {
+    const long long i = (e * a.R + r) * a.C + c;
+    float g[8], m[8];
+    ld8(a.g, i, a.g_bf16, g);
+    ld8(a.m, i, a.m_bf16, m);
+    const float rs = rowsum ? rsm[r - r0] : 1.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float v = (b * m[j] + b1 * g[j]) * cs[j] * rs;
+      acc[j] += v * v;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) part[ty][tx * 8 + j] = acc[j];
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x];
+  atomicAdd(colsq_out + e * a.C + (long long)blockIdx.x * 256 + threadIdx.x, t);
+}
+
+// Rows, then columns, in one pass over bf16 g and m, streamed: rowsq[e,r] = sum_c (mf * cin[e,c])^2 and
+// colsq[e,c] += sum_r (mf * cin[e,c] * scale(rowsq[e,r]))^2.  A block walks a contiguous run of rows; a thread owns the same
+// 4 NV columns of every row, so the column sums stay in its registers until the expert ends, and each thread reads from
+// the ring only what it copied itself: one barrier (the row sums') per group of U rows.  1 block of 512 per SM, U rows
+// are about 48 KB of g and m, RC_GROUPS groups in the ring.  (8, 2048, 6144): 95 us against
+// 78 + 76 for the two passes; (8, 6144, 2048): 147 against 78 + 76; with 1024 columns or less half the threads idle and the
+// two passes win.
+constexpr int RC_GROUPS = 4;
+template <int NV, int U>
+__global__ void __launch_bounds__(512) instinct_rowcol_s8(InstinctArgs a, const float* __restrict__ colsum_in, float col_count,
+                                                          float* __restrict__ rowsq, float* __restrict__ colsq) {
+  extern __shared__ __align__(16) uint8_t rc_ring[];
+  __shared__ __align__(16) float red[2][U][16];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long long C = a.C;
+  const float b = a.beta, b1 = 1.f - a.beta, Cf = (float)C;
+  const bf16 *G = reinterpret_cast<const bf16*>(a.g), *M = reinterpret_cast<const bf16*>(a.m);
+  uint2* ring = reinterpret_cast<uint2*>(rc_ring) + tid;               // slot (group, row, array, i): 512 x 8 bytes
+  const long long ER = a.E * a.R;
+  const long long lo = ER * blockIdx.x / gridDim.x, hi = ER * (blockIdx.x + 1) / gridDim.x;
+  int turn = 0;
+  for (long long seg = lo; seg < hi;) {
+    const long long e = seg / a.R, seg_hi = min(hi, (e + 1) * a.R);
+    auto issue = [&](int group, long long row) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const long long c = (i * 512 + tid) * 4ll;
+          if (c < C && row + u < seg_hi) {
+            cp_async8(ring + (((group * U + u) * 2) * NV + i) * 512, G + (row + u) * C + c);
+            cp_async8(ring + (((group * U + u) * 2 + 1) * NV + i) * 512, M + (row + u) * C + c);
+          }
+        }
+      cp_async_commit();
+    };
+    for (int g = 0; g < RC_GROUPS; ++g) issue(g, seg + g * U);
+    float cs[NV][4], acc[NV][4];
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long long c = (i * 512 + tid) * 4ll + j;
+        cs[i][j] = c < C ? (colsum_in ? scale_of(colsum_in[e * C + c], col_count) : 1.f) : 0.f;
+        acc[i][j] = 0.f;
+      }
+    int group = 0;
+    for (long long row = seg; row < seg_hi; row += U) {
+      cp_async_wait<RC_GROUPS - 1>();
+      float v[U][NV][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const uint2 g = ring[(((group * U + u) * 2) * NV + i) * 512], m = ring[(((group * U + u) * 2 + 1) * NV + i) * 512];
+          const float2 g0 = unpack_bf16(g.x), g1 = unpack_bf16(g.y), m0 = unpack_bf16(m.x), m1 = unpack_bf16(m.y);
+          const bool in = (i * 512 + tid) * 4ll < C && row + u < seg_hi;      // slots never filled hold anything
+          v[u][i][0] = in ? (b * m0.x + b1 * g0.x) * cs[i][0] : 0.f;
+          v[u][i][1] = in ? (b * m0.y + b1 * g0.y) * cs[i][1] : 0.f;
+          v[u][i][2] = in ? (b * m1.x + b1 * g1.x) * cs[i][2] : 0.f;
+          v[u][i][3] = in ? (b * m1.y + b1 * g1.y) * cs[i][3] : 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) t += v[u][i][j] * v[u][i][j];
+        }
+        t = warp_sum(t);
+        if (lane == 0) red[turn][u][warp] = t;
+      }
+      issue(group, row + RC_GROUPS * U);
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; k += 4) {
+          const float4 q = *reinterpret_cast<const float4*>(&red[turn][u][k]);
+          t += (q.x + q.y) + (q.z + q.w);
+        }
+        if (row + u < seg_hi) {
+          if (tid == 0) rowsq[row + u] = t;
+          const float rs = scale_of(t, Cf);
+#pragma unroll
+          for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { const float w = v[u][i][j] * rs; acc[i][j] += w * w; }
+        }
+      }
+      turn ^= 1;
+      if (++group == RC_GROUPS) group = 0;
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long long c = (i * 512 + tid) * 4ll + j;
+        if (c < C) atomicAdd(colsq + e * C + c, acc[i][j]);
+      }
+    seg = seg_hi;
+  }
 }
 
 // Rows, then columns, in one pass: rowsq_out[e,r] = sum_c (mf*cin[e,c])^2 and
@@ -386,22 +534,13 @@ __global__ void instinct_apply(InstinctArgs a, const float* __restrict__ rowsum,
 // a warp that loads a few chunks of its row into registers, then computes, does little better (2.6 / 4.4 TB/s): HBM
 // wants well over 100 KB in flight per SM all the time.  So here every thread keeps a ring of S chunks (8 elements of
 // each input array) in shared memory, filled by cp.async copies issued S chunks ahead of the one it consumes;
-// a warp owns a contiguous run of rows, so its stream is one linear span of memory, and the ring runs across row
+// a warp owns a contiguous run of chunks, so its stream is one linear span of memory, and the ring runs across row
 // boundaries.  One block per SM; C % 256 == 0 (a chunk of 32 lanes x 8 never straddles rows).
-__device__ __forceinline__ void cp_async16(void* s, const void* g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(s)), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // A lane's 8 elements of a 256-element chunk are two groups of four, 128 elements apart: columns lane*4 .. +3 and
 // 128 + lane*4 .. +3.  Every warp-wide load or store then covers one contiguous span of full 32-byte sectors whatever
 // the element size (with 8 consecutive elements per lane an fp32 array needs two 16-byte accesses at a 32-byte lane
 // stride, each touching all sectors of the chunk and using half of each: the word tables with their fp32 gradients
 // ran at 1.8 TB/s).
-__device__ __forceinline__ void cp_async8(void* s, const void* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(s)), "l"(g) : "memory");
-}
 struct Ring8 {             // this thread's ring: slot (stage, q) is 16 bytes; slots of one (stage, q) are contiguous over threads
   uint4* base;
   int T, nslot;
@@ -453,21 +592,20 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
   ring.base = reinterpret_cast<uint4*>(sm + (colsum ? a.C : 0)) + threadIdx.x;
   ring.T = blockDim.x;
   ring.nslot = gs + ms;
-  const long long cpr = a.C >> 8;                       // chunks per row
-  const long long ER = a.E * a.R;
-  const long long lo = ER * blockIdx.x / gridDim.x, hi = ER * (blockIdx.x + 1) / gridDim.x;
+  const long long cpr = a.C >> 8, cpe = a.R * cpr;       // chunks per row, per expert
+  const long long NC = a.E * cpe;
+  const long long lo = NC * blockIdx.x / gridDim.x, hi = NC * (blockIdx.x + 1) / gridDim.x;
   for (long long seg = lo; seg < hi;) {
-    const long long e = seg / a.R, seg_hi = min(hi, (e + 1) * a.R);
+    const long long e = seg / cpe, seg_hi = min(hi, (e + 1) * cpe);
     if (cs) {
       __syncthreads();
       load_colscale(cs, colsum, nullptr, e, a.C, col_count);
     }
-    const long long rpw = (seg_hi - seg + nw - 1) / nw;
-    const long long r0 = min(seg_hi, seg + warp * rpw), r1 = min(seg_hi, r0 + rpw);
-    const long long total = (r1 - r0) * cpr;
+    const long long cpw = (seg_hi - seg + nw - 1) / nw;
+    const long long f0 = min(seg_hi, seg + warp * cpw), total = min(seg_hi, f0 + cpw) - f0;
     // both arrays bf16: 8 consecutive elements per lane are one full 16-byte copy each (faster than two 8-byte ones)
     const bool packed = a.g_bf16 && a.m_bf16;
-    const long long el0 = r0 * a.C + lane * (packed ? 8 : 4);
+    const long long el0 = (f0 << 8) + lane * (packed ? 8 : 4);
     auto issue = [&](int stage, long long k) {
       if (packed) {
         cp_async16(ring.slot(stage, 0), reinterpret_cast<const bf16*>(a.g) + el0 + (k << 8));
@@ -483,7 +621,8 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
       cp_async_commit();
     }
     int stage = 0;
-    long long row = r0, cin = 0;
+    long long row = f0 / cpr, cin = f0 - row * cpr;
+    bool whole = cin == 0;                               // the row began in this warp
     float ss = 0.f, sa = 0.f;
     for (long long k = 0; k < total; ++k) {
       cp_async_wait<S - 1>();
@@ -504,14 +643,21 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
         ss += v * v;
         sa += fabsf(g[j]);
       }
-      if (++cin == cpr) {
+      if (++cin == cpr || k + 1 == total) {
+        // a row cut between warps is added up in the zeroed array
         ss = warp_sum(ss);
         if (rowabs) sa = warp_sum(sa);
         if (lane == 0) {
-          rowsq[row] = ss;
-          if (rowabs) rowabs[row] = sa;
+          if (whole && cin == cpr) {
+            rowsq[row] = ss;
+            if (rowabs) rowabs[row] = sa;
+          } else {
+            atomicAdd(rowsq + row, ss);
+            if (rowabs) atomicAdd(rowabs + row, sa);
+          }
         }
         ++row; cin = 0; ss = 0.f; sa = 0.f;
+        whole = true;
       }
       if (++stage == S) stage = 0;
     }
@@ -520,7 +666,8 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
   }
 }
 
-// The update without the staged last row norm (instinct_apply with fuse_row_norm = 0), streamed.  Stochastic
+// The update without the staged last row norm (instinct_apply with fuse_row_norm = 0), streamed.  Nothing is summed
+// here, so the work is dealt out in chunks, not rows: a weight of 1024 rows keeps all warps busy too.  Stochastic
 // rounding keeps the per-element hash of the block-per-row kernel, so both produce the same bits.
 // Dynamic shared memory: C floats with column sums, then the rings (g, m and the weight's exact copy).
 template <int S>
@@ -547,19 +694,18 @@ __global__ void __launch_bounds__(384) instinct_apply_s8(InstinctArgs a, const f
   ring.base = reinterpret_cast<uint4*>(sm + (has_col ? C : 0)) + threadIdx.x;
   ring.T = blockDim.x;
   ring.nslot = gs + ms + ws;
-  const long long cpr = C >> 8;
-  const long long ER = a.E * a.R;
-  const long long lo = ER * blockIdx.x / gridDim.x, hi = ER * (blockIdx.x + 1) / gridDim.x;
+  const long long cpr = C >> 8, cpe = a.R * cpr;          // chunks per row, per expert
+  const long long NC = a.E * cpe;
+  const long long lo = NC * blockIdx.x / gridDim.x, hi = NC * (blockIdx.x + 1) / gridDim.x;
   for (long long seg = lo; seg < hi;) {
-    const long long e = seg / a.R, seg_hi = min(hi, (e + 1) * a.R);
+    const long long e = seg / cpe, seg_hi = min(hi, (e + 1) * cpe);
     if (has_col) {
       __syncthreads();
       load_colscale(colk, colsum1, colsum2, e, C, col_count);
     }
-    const long long rpw = (seg_hi - seg + nw - 1) / nw;
-    const long long r0 = min(seg_hi, seg + warp * rpw), r1 = min(seg_hi, r0 + rpw);
-    const long long total = (r1 - r0) * cpr;
-    const long long el0 = r0 * C + lane * 4;
+    const long long cpw = (seg_hi - seg + nw - 1) / nw;
+    const long long f0 = min(seg_hi, seg + warp * cpw), total = min(seg_hi, f0 + cpw) - f0;
+    const long long el0 = (f0 << 8) + lane * 4;
     auto issue = [&](int stage, long long k) {
       ring.issue8(stage, 0, a.g, el0 + (k << 8), a.g_bf16);
       ring.issue8(stage, gs, a.m, el0 + (k << 8), a.m_bf16);
@@ -571,11 +717,11 @@ __global__ void __launch_bounds__(384) instinct_apply_s8(InstinctArgs a, const f
       cp_async_commit();
     }
     int stage = 0;
-    long long row = r0, cin = 0;
+    long long row = f0 / cpr, cin = f0 - row * cpr;
     float rs = 1.f;
     bool moves = true;
     for (long long k = 0; k < total; ++k) {
-      if (cin == 0) {
+      if (k == 0 || cin == 0) {
         rs = rowsum ? scale_of(rowsum[row], row_count) : 1.f;
         if (rowsum2) rs *= scale_of(rowsum2[row] * rs * rs, row_count);
         const bool frozen = a.frozen && a.frozen[(row * C) / a.frozen_stride];
@@ -725,15 +871,6 @@ static __global__ void instinct_lag_rows_select(float* __restrict__ cs, float* _
   }
 }
 
-// Scratch layout (fp32, ZEROED by the caller, 16-byte aligned base): [rowA][rowB][rowabs] of pad4(E*R) each,
-// [colA][colB] of pad4(E*C) each, [rel 4]; every sub-array starts on a 16-byte boundary.
-inline long long instinct_pad4(long long n) { return (n + 3) & ~3ll; }
-inline long long instinct_scratch_floats(long long E, long long R, long long C) {
-  return 3 * instinct_pad4(E * R) + 2 * instinct_pad4(E * C) + 4;
-}
-
-constexpr size_t INSTINCT_SMEM_MAX = 200 * 1024;     // dynamic shared memory the row-staging kernels may ask for
-
 // Launch sequence; returns the number of kernels launched, or -1 when this weight cannot take the requested form
 // (nothing is launched then).  `cs` / `cs_ok`: lagged homeostasis state (previous step's second-axis mean squares and
 // the "all positive" flag), or null for the exact form.
@@ -775,8 +912,10 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INSTINCT_SMEM_MAX);
   };
   // streaming forms: 16-byte accesses on every array, whole chunks of 256 columns, enough rows to fill the GPU
-  const bool s8 = vec && a.C % 256 == 0 && (a.shadow == nullptr || (reinterpret_cast<uintptr_t>(a.shadow) & 15) == 0) &&
-                  ER >= 148 * 16;
+  const bool aligned8 = vec && a.C % 256 == 0 && (a.shadow == nullptr || (reinterpret_cast<uintptr_t>(a.shadow) & 15) == 0);
+  // dealt out in chunks of 256 elements: two or more for each of 148 x 16 warps (sums), four for each of 148 x 12 (update),
+  // else filling and draining the rings costs more than the block-per-row form
+  const bool s8_rows = aligned8 && ER * (a.C >> 8) >= 2 * 148 * 16, s8_chunks = aligned8 && ER * (a.C >> 8) >= 4 * 148 * 12;
   constexpr size_t S8_SMEM = 216 * 1024;
   // launch `kern<S>` with the deepest ring that fits beside `head` bytes: T threads, `slots` 16-byte slots per stage
   auto s8_launch = [&](auto k12, auto k8, auto k6, auto k4, int T, int slots, size_t head, auto&&... args) {
@@ -792,7 +931,7 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   };
   auto stat_rows = [&](const float* colsum, float* out, float* absout) {
     const size_t smem = colsum ? Cb : 0;
-    if (s8 && smem + 4 * 512 * 4 * 16 <= S8_SMEM) {
+    if (s8_rows && smem + 4 * 512 * 4 * 16 <= S8_SMEM) {
       s8_launch(instinct_stat_rows_s8<12>, instinct_stat_rows_s8<8>, instinct_stat_rows_s8<6>, instinct_stat_rows_s8<4>, 512,
                 (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2), smem, a, colsum, Rf, out, absout);
       return;
@@ -803,6 +942,17 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
     ++launches;
   };
   auto stat_cols = [&](const float* colsum, const float* rowsum, float* out) {
+    if (aligned8 && a.E == 1) {
+      // two rounds of two blocks per SM; at least 64 rows each, so that a column is not added to by too many
+      const long long strips = a.C / 256, want = std::max<long long>(1, 148 * 4 / std::max<long long>(1, strips * a.E));
+      const int rows = (int)std::max<long long>(64, (a.R + want - 1) / want), chunks = (int)((a.R + rows - 1) / rows);
+      const size_t smem = rowsum ? (size_t)rows * sizeof(float) : 0;
+      if (smem <= 40 * 1024 && chunks <= 65535 && a.E <= 65535) {
+        instinct_stat_cols_s8<<<dim3((unsigned)strips, chunks, (unsigned)a.E), 256, smem, st>>>(a, colsum, Rf, rowsum, Cf, out, rows);
+        ++launches;
+        return;
+      }
+    }
     const int V = vec ? 4 : 1;
     const int threads = 128;
     const int strips = (int)((a.C + (long long)threads * V - 1) / ((long long)threads * V));
@@ -815,6 +965,20 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
     else { raise(instinct_stat_cols<1>, smem); instinct_stat_cols<1><<<grid, threads, smem, st>>>(a, colsum, Rf, rowsum, Cf, out, rows_per_block); }
     ++launches;
   };
+  // rows and columns of bf16 arrays in one pass; false: this weight does not suit it
+  auto rowcol_s8 = [&](const float* colsum_in, float* rows_out, float* cols_out) -> bool {
+    const int nv = (int)((a.C + 2047) / 2048);
+    // rows long enough to keep 512 threads busy, and a few groups of rows for every block
+    if (!vec || !a.g_bf16 || !a.m_bf16 || a.C < 1536 || nv > 3 || ER < 148 * 8) return false;
+    auto go = [&](auto kern, int rows) {
+      const size_t smem = (size_t)RC_GROUPS * rows * 2 * nv * 512 * 8;
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      kern<<<148, 512, smem, st>>>(a, colsum_in, Rf, rows_out, cols_out);
+    };
+    if (nv == 1) go(instinct_rowcol_s8<1, 6>, 6); else if (nv == 2) go(instinct_rowcol_s8<2, 3>, 3); else go(instinct_rowcol_s8<3, 2>, 2);
+    ++launches;
+    return true;
+  };
   auto rowcol = [&](const float* colsum_in, float* rows_out, float* cols_out, const int* skip_if) {
     const size_t smem = (colsum_in ? 3 : 2) * Cb;
     dim3 grid(blocks_per_expert(smem), E);
@@ -824,7 +988,7 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   };
   auto apply = [&](const float* rs, const float* rs2, const float* c1, const float* c2, bool fuse, const float* rabs) {
     const size_t smem = ((c1 || c2) ? Cb : 0) + (fuse ? Cb : 0);
-    if (s8 && !fuse && smem + 4 * 384 * 6 * 16 <= S8_SMEM) {
+    if (s8_chunks && !fuse && smem + 4 * 384 * 6 * 16 <= S8_SMEM) {
       const int slots = (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2) + ((a.w == nullptr && a.p_bf16) ? 1 : 2);
       s8_launch(instinct_apply_s8<12>, instinct_apply_s8<8>, instinct_apply_s8<6>, instinct_apply_s8<4>, 384, slots, smem, a, rs,
                 Cf, rs2, c1, c2, Rf, rabs, rel2, rel_out);
@@ -852,14 +1016,16 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
         launches += 2;
         break;
       }
-      if (phase != 2) {
+      if (phase != 2 && !rowcol_s8(nullptr, rowA, colA)) {
         stat_rows(nullptr, rowA, nullptr);
         stat_cols(nullptr, rowA, colA);
       }
       if (phase == 1) break;
-      if (stage2) {
+      if (stage2 && !s8_chunks) {
         apply(rowA, nullptr, colA, nullptr, true, nullptr);        // the last row norm on the row staged in shared memory
       } else {
+        // a third look at g and m (from L2 for the usual sizes) and the streamed update: (3072, 1024), (8192,
+        // 1024) and (1024, 4096) together 36 + 47 us against 103 for the update with the row staged
         stat_rows(colA, rowB, nullptr);            // sum_c (mf cs)^2; times rs1^2 inside apply = row sums of u2
         apply(rowA, rowB, colA, nullptr, false, nullptr);
       }
@@ -867,6 +1033,10 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
     }
     case 5:   // hs3: over R (per column), over C (per row), over R again
       stat_cols(nullptr, nullptr, colA);
+      if (!cs && rowcol_s8(colA, rowA, colB)) {
+        apply(rowA, nullptr, colA, colB, false, nullptr);
+        break;
+      }
       stat_rows(colA, rowA, nullptr);
       if (cs) {
         instinct_lag_rows_select<<<(int)std::max<long long>(1, std::min<long long>((ER + 255) / 256, 592)), 256, 0, st>>>(cs, rowA, ER, Cf);

@@ -145,3 +145,30 @@ def test_route_and_slot_fused(N, d, E, k, C):
     assert abs(float(o[4]) - float(aux)) < 1e-5 * max(1.0, float(aux)) and abs(float(o[5]) - float(dropped)) < 1e-6
     ((o[0] * gw.cuda()).sum() + (o[2] * gt.cuda()).sum() + (o[6] * gp.cuda()).sum() + 3 * o[4]).backward()
     assert _rel(xg.grad.cpu(), xc.grad) < 4e-3 and _rel(wg.grad.cpu(), wc.grad) < 1e-4
+
+
+# ------------------------------------------------------------------------------------------------ optimizer
+@pytest.mark.parametrize("shape,bf16", [((1190, 2048), False), ((1200, 1540), True), ((2500, 6144), True), ((1300, 4100), False), ((1024, 4096), False),
+                                        ((3072, 1024), False), ((5, 700, 1540), True), ((3, 640, 2304), True), ((12000, 512), False), ((260, 256), False)])
+def test_instinct_streamed_forms(shape, bf16):
+    """One step on the kernels against the PyTorch statement: whole and cut rows, expert borders inside a block, all width classes."""
+    from memarch_b200.config import OptConfig
+    from memarch_b200.optim import Instinct
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    p0 = torch.randn(*shape, device="cuda", generator=g) * 0.05
+    grad = (torch.randn(*shape, device="cuda", generator=g) * 1e-3).bfloat16()
+    m0 = torch.randn(*shape, device="cuda", generator=g) * 1e-3
+    got = []
+    for own in (True, False):
+        p = torch.nn.Parameter(p0.bfloat16() if bf16 else p0.clone())
+        opt = Instinct([p], OptConfig(lr=1e-2, norm="hs", scale=0.12, m_bf16=True, rel_every=1 << 30))
+        opt.n_step = 1
+        opt.m[0].copy_(m0)
+        kind, wd, vocab = opt.spec(p)
+        opt._sync_lr()
+        with torch.no_grad():
+            (opt._update_cuda if own else opt._update_ref)(0, p, grad, kind, 0.1 if wd else 0.0, opt._lr_t, False)
+        got.append((opt.w[0] if bf16 else p.detach(), opt.m[0]))
+    step = (got[1][0] - (p0.bfloat16().float() if bf16 else p0))
+    assert ((got[0][0] - got[1][0]).norm() / step.norm()).item() < 1e-4          # fp32 sums in another order
+    assert torch.equal(got[0][1], got[1][1])                                      # the momentum does not depend on them
