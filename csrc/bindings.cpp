@@ -68,8 +68,11 @@ std::vector<torch::Tensor> route_bwd(torch::Tensor x, torch::Tensor w, torch::Te
                                      c10::optional<torch::Tensor> d_wt, c10::optional<torch::Tensor> d_wtab,
                                      c10::optional<torch::Tensor> d_aux, c10::optional<torch::Tensor> d_probs);
 int64_t attn_status_read();
-std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor dout, torch::Tensor lse,
-                                       torch::Tensor delta, int64_t window, double scale);
+std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor o, torch::Tensor dout,
+                                       torch::Tensor lse, int64_t window, double scale);
+std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
+torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor qkv,
+                           torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
 int64_t attn_bwd_status_read();
 torch::Tensor embed_sum_fwd(torch::Tensor emb, torch::Tensor x, c10::optional<torch::Tensor> cand, c10::optional<torch::Tensor> sel,
                             c10::optional<torch::Tensor> phr, c10::optional<torch::Tensor> pidx);
@@ -121,6 +124,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_status_read", &mb::attn_status_read);
   m.def("route_fwd", &mb::route_fwd, "router, slotting and auxiliary loss of an expert layer");
   m.def("route_bwd", &mb::route_bwd);
+  m.def("attn_qkv_fwd", &mb::attn_qkv_fwd, "rotation + attention forward on packed projections (head dim 64)");
+  m.def("attn_qkv_bwd", &mb::attn_qkv_bwd);
   m.def("attn_bwd_tc", &mb::attn_bwd_tc, "causal / sliding-window attention backward on tcgen05 (head dim 64)");
   m.def("attn_bwd_status_read", &mb::attn_bwd_status_read);
   m.def("mem_read_fwd", &mb::mem_read_fwd);

@@ -4,10 +4,10 @@ Reference behaviour: `F.scaled_dot_product_attention(rope(q), rope(k), v, is_cau
 window (full.py:156-157); block-masked window attention `kv <= q and q - kv < window` otherwise (FlexAttention with
 an O(T) block list, full2.py:153-181; two-block variants lm.py:448-554).
 
-GPU body: `rope_qk` kernel (rotation of the q and k thirds of the packed qkv activations, `rope_merge_bwd` packs and
-rotates the three gradients back in one pass) followed by the attention core: the library flash kernel by default
-(`MEMARCH_ATTN=lib`), or the own tcgen05 forward kernel `attn_fwd_tc` (`MEMARCH_ATTN=own`, head dim 64: block list from
-window arithmetic, no mask tensor, exact LSE; its backward recomputes through the library).
+GPU body, head dim 64: the own tcgen05 kernels on the packed projections (`_QkvAttn`, `csrc/attn_fwd.cu`,
+`csrc/attn_bwd.cu`: q and k rotated, v read in place, gradients written rotated back into the packed layout).  Other head
+dims, or `MEMARCH_ATTN=lib`: `rope_qk` (rotation of the q and k thirds of the packed qkv activations, `rope_merge_bwd`
+packs and rotates the three gradients back in one pass) around the library flash kernel.
 """
 from __future__ import annotations
 
@@ -18,8 +18,9 @@ import torch.nn.functional as F
 
 from . import _ext, ref
 
-ATTN_CORE = os.environ.get("MEMARCH_ATTN", "lib")
+ATTN_CORE = os.environ.get("MEMARCH_ATTN", "own")
 OWN_WINDOW_EVAL = os.environ.get("MEMARCH_ATTN_EVAL", "own") == "own"
+OWN_CAUSAL_T = 512                                            # plain causal texts up to this length: see `attention`
 OWN_BWD = os.environ.get("MEMARCH_ATTN_BWD", "own") == "own"
 WINDOW_BODY = os.environ.get("MEMARCH_WINDOW", "flash")        # library body of windowed attention with backward: flash | block
 
@@ -75,9 +76,8 @@ class _RopeSplit(torch.autograd.Function):
 
 
 class _OwnAttn(torch.autograd.Function):
-    """Attention core on the own tcgen05 kernels (`csrc/attn_tc.cu`, `csrc/attn_bwd_tc.cu`): S = QKt, O = PV and the five
-    backward products on the tensor cores with TMEM accumulators, softmax by one thread per row, block lists from
-    window arithmetic, exact LSE.  `MEMARCH_ATTN_BWD=lib` makes backward recompute through the library instead."""
+    """Attention core on the own tcgen05 kernels (`csrc/attn_fwd.cu`, `csrc/attn_bwd.cu`): S = QKt, O = PV and the five
+    backward products on the tensor cores with TMEM accumulators, block lists from window arithmetic, exact LSE.  `MEMARCH_ATTN_BWD=lib` makes backward recompute through the library instead."""
 
     @staticmethod
     def forward(ctx, q, k, v, window):
@@ -93,11 +93,9 @@ class _OwnAttn(torch.autograd.Function):
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
         if OWN_BWD:
-            do = do.contiguous()
-            delta = (do.float() * o.float()).sum(-1)
-            dq, dk, dv = _ext.C().attn_bwd_tc(q, k, v, do, lse, delta, ctx.window, float(q.shape[-1]) ** -0.5)
-            _ext.count()
-            return dq.to(q.dtype), dk, dv, None
+            dq, dk, dv = _ext.C().attn_bwd_tc(q, k, v, o, do.contiguous(), lse, ctx.window, float(q.shape[-1]) ** -0.5)
+            _ext.count(3)
+            return dq, dk, dv, None
         q, k, v = (t.detach().requires_grad_() for t in (q, k, v))
         with torch.enable_grad():
             o2 = F.scaled_dot_product_attention(q, k, v, is_causal=True) if ctx.window == 0 else _lib_window(q, k, v, ctx.window)
@@ -108,6 +106,32 @@ class _OwnAttn(torch.autograd.Function):
 def own_attention(q, k, v, window=0):
     """q, k, v (B,H,T,64) bf16 with RoPE applied -> o (B,H,T,64); `window` 0 = plain causal."""
     return _OwnAttn.apply(q, k, v, int(window or 0))
+
+
+class _QkvAttn(torch.autograd.Function):
+    """RoPE + causal / sliding-window attention on packed projections qkv (B,T,3,H,64) -> (B,T,H*64), window 0 = plain
+    causal.  Forward rotates q and k into a buffer of their own and reads v where the projection left it; backward
+    writes dq, dk (rotated back) and dv straight into one packed gradient."""
+
+    @staticmethod
+    def forward(ctx, qkv, window, half):
+        B, T, _, H, hd = qkv.shape
+        cos, sin = rope_tables(T, hd, qkv.device)
+        o, lse, qk = _ext.C().attn_qkv_fwd(qkv, cos, sin, bool(half), int(window))
+        _ext.count(2)
+        ctx.save_for_backward(qkv, o, lse, qk)
+        ctx.window, ctx.half = int(window), bool(half)
+        return o.view(B, T, H * hd)
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, o, lse, qk = ctx.saved_tensors
+        cos, sin = rope_tables(qkv.shape[1], qkv.shape[4], qkv.device)
+        _ext.count(3)
+        do = do.contiguous()
+        if do.data_ptr() % 16:
+            do = do.clone()
+        return _ext.C().attn_qkv_bwd(do, o, lse, qk, qkv, cos, sin, ctx.half, ctx.window), None, None
 
 
 def _lib_window(q, k, v, window):
@@ -160,12 +184,18 @@ def attention(qkv, window=None, rope_half=False, qk_norm=False):
     B, T, _, H, hd = qkv.shape
     win = None if (window is None or window >= T) else int(window)
     if _ext.use_cuda(qkv) and qkv.dtype == torch.bfloat16 and not qk_norm and hd % 8 == 0:
-        q, k, v = _RopeSplit.apply(qkv, rope_half)
-        # own tcgen05 kernel: everywhere when asked for; by default where it is the faster one, i.e. sliding-window
-        # attention without a backward pass (evaluation / generation at long context: only the blocks under the window
-        # are visited, 3.4x faster than the dense-mask library form at T = 16k, window 256)
         no_grad = not (torch.is_grad_enabled() and qkv.requires_grad)
-        if hd == 64 and (ATTN_CORE == "own" or (ATTN_CORE == "lib" and win is not None and no_grad and OWN_WINDOW_EVAL)):
+        # The own kernels serve windows (forward + backward, 2 x 16 384 words, 16 heads, window 256: 700 us against 1221 for the
+        # library flash kernel; 4 x 4096, window 1024: 635 against 1242) and short causal texts (8 x 512, 8 heads: 90
+        # against 157; 16 x 256, 12 heads: 102 against 144).  On longer causal texts the library core is still ahead
+        # (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16 heads: 1222 against 943).
+        own = (ATTN_CORE == "own" and (win is not None or T <= OWN_CAUSAL_T)) or (win is not None and no_grad and OWN_WINDOW_EVAL)
+        if hd == 64 and own and (no_grad or OWN_BWD):
+            qkv = qkv.contiguous()
+            if qkv.data_ptr() % 16 == 0:
+                return _QkvAttn.apply(qkv, win or 0, rope_half)
+        q, k, v = _RopeSplit.apply(qkv, rope_half)
+        if hd == 64 and own:
             return own_attention(q, k, v, win or 0).transpose(1, 2).reshape(B, T, H * hd)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True) if win is None else _flash_window(q, k, v, win)
         return o.transpose(1, 2).reshape(B, T, H * hd)

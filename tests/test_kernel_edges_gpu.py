@@ -172,3 +172,28 @@ def test_instinct_streamed_forms(shape, bf16):
     step = (got[1][0] - (p0.bfloat16().float() if bf16 else p0))
     assert ((got[0][0] - got[1][0]).norm() / step.norm()).item() < 1e-4          # fp32 sums in another order
     assert torch.equal(got[0][1], got[1][1])                                      # the momentum does not depend on them
+
+
+# ------------------------------------------------------------------------------------------------ attention
+@pytest.mark.parametrize("B,T,H,window,half", [(1, 1, 1, 0, False), (2, 63, 3, 0, True), (1, 64, 2, 0, False), (2, 65, 1, 0, False), (1, 127, 3, 5, True), (2, 128, 2, 0, True),
+                                               (2, 129, 2, 0, False), (1, 300, 2, 1, False), (1, 511, 2, 64, False), (1, 700, 2, 100, True), (2, 900, 3, 129, False),
+                                               (8, 260, 20, 0, False), (6, 520, 24, 0, True), (10, 400, 20, 130, False)])
+def test_attention_on_packed_projections(B, T, H, window, half):
+    """Rotation, attention and the gradient of the packed projections; the last three have more tiles than CTAs, in pairs
+    (causal, odd and even numbers of tiles) and singly (window)."""
+    from memarch_b200.ops import _ext, ref
+    from memarch_b200.ops.attention import _QkvAttn
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(B, T, 3, H, 64, device="cuda", generator=g).bfloat16().requires_grad_()
+    go = torch.randn(B, T, H * 64, device="cuda", generator=g).bfloat16()
+    o = _QkvAttn.apply(qkv, window, half)
+    o.backward(go)
+    torch.cuda.synchronize()
+    assert _ext.C().attn_status_read() == 0 and _ext.C().attn_bwd_status_read() == 0
+    x = qkv.detach().float().requires_grad_()
+    r = ref.window_attention(x[:, :, 0], x[:, :, 1], x[:, :, 2], window or None, half).reshape(B, T, H * 64)
+    r.backward(go.float())
+    assert _rel(o, r.detach()) < 1e-2                                             # bf16 q, k, P and output
+    for i in range(3):
+        a, b = qkv.grad[:, :, i], x.grad[:, :, i]
+        assert (a.double() - b.double()).norm() < 2e-2 * max(b.double().norm(), 1e-2 * x.grad.double().norm()), i
