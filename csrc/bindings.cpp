@@ -73,6 +73,17 @@ std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::
 std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
 torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor qkv,
                            torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
+std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, c10::optional<torch::Tensor> pending, torch::Tensor nw, double eps, torch::Tensor wqkv,
+                                         torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
+std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, c10::optional<torch::Tensor> dh, torch::Tensor h, torch::Tensor n, torch::Tensor rstd,
+                                         torch::Tensor qkv, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor nw,
+                                         torch::Tensor wqkv, torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window,
+                                         bool want_lo, bool grad_f32);
+std::vector<torch::Tensor> ffn_half_fwd(torch::Tensor h, torch::Tensor a, torch::Tensor nw, double eps, torch::Tensor wup, torch::Tensor wdown,
+                                        bool swiglu, bool add_out);
+std::vector<torch::Tensor> ffn_half_bwd(torch::Tensor dy, c10::optional<torch::Tensor> dx2, torch::Tensor x2, torch::Tensor n, torch::Tensor rstd,
+                                        torch::Tensor pre, torch::Tensor hid, torch::Tensor nw, torch::Tensor wup, torch::Tensor wdown,
+                                        bool swiglu, bool grad_f32);
 int64_t attn_bwd_status_read();
 torch::Tensor embed_sum_fwd(torch::Tensor emb, torch::Tensor x, c10::optional<torch::Tensor> cand, c10::optional<torch::Tensor> sel,
                             c10::optional<torch::Tensor> phr, c10::optional<torch::Tensor> pidx);
@@ -124,6 +135,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_status_read", &mb::attn_status_read);
   m.def("route_fwd", &mb::route_fwd, "router, slotting and auxiliary loss of an expert layer");
   m.def("route_bwd", &mb::route_bwd);
+  m.def("attn_half_fwd", &mb::attn_half_fwd, "attention half of a light layer");
+  m.def("attn_half_bwd", &mb::attn_half_bwd);
+  m.def("ffn_half_fwd", &mb::ffn_half_fwd, "feed-forward half of a light layer");
+  m.def("ffn_half_bwd", &mb::ffn_half_bwd);
   m.def("attn_qkv_fwd", &mb::attn_qkv_fwd, "rotation + attention forward on packed projections (head dim 64)");
   m.def("attn_qkv_bwd", &mb::attn_qkv_bwd);
   m.def("attn_bwd_tc", &mb::attn_bwd_tc, "causal / sliding-window attention backward on tcgen05 (head dim 64)");

@@ -11,11 +11,17 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import ops
+from ..ops import layer
 
 
 def _cdt(x):
     """Compute dtype of matmul operands: bf16 on the GPU (tcgen05), the tensor's own dtype on CPU."""
     return torch.bfloat16 if x.is_cuda else x.dtype
+
+
+def _eps(norm):
+    """The norm's epsilon; torch's default is the machine epsilon of the input, fp32 on this path."""
+    return torch.finfo(torch.float32).eps if norm.eps is None else norm.eps
 
 
 class FineMoE(nn.Module):
@@ -111,6 +117,12 @@ class LightBlock(nn.Module):
             if pending is not None:
                 x, pending = ops.resid_add(x, pending), None
             x = x + self.x0_l * self.cur_x0
+        plain = not hasattr(self, "moe") and self.cur_sel is None
+        win = 0 if window is None or window >= T else int(window)
+        if (plain and tether is None and self.cur_ve is None and self.attn_gain == 1.0 and "qk" not in self.blk
+                and layer.attn_half_ok(x, pending, self.n1.weight, self.qkv.weight, self.o.weight, self.heads, window)):
+            x, a = layer.attn_half(x, pending, self.n1.weight, self.qkv.weight, self.o.weight, _eps(self.n1), win, self.rope_half)
+            return self._feed_forward(x, a, defer)
         if pending is not None:
             x, n1 = ops.add_rmsnorm(x, pending, self.n1.weight, self.n1.eps)
         else:
@@ -146,7 +158,13 @@ class LightBlock(nn.Module):
             xs = ops.rmsnorm(x, self.n2.weight, self.n2.eps, out_dtype=dt).gather(1, idx[..., None].expand(-1, -1, D))
             y = ops.linear(self._act(ops.linear(xs, self.up.weight)), self.down.weight) * ok[..., None].to(dt)
             return fin(x.scatter_add(1, idx[..., None].expand(-1, -1, D), y.to(x.dtype)))
-        x, n2 = ops.add_rmsnorm(x, ops.linear(a, self.o.weight, direct=True), self.n2.weight, self.n2.eps)
+        return self._feed_forward(x, ops.linear(a, self.o.weight, direct=True), defer)
+
+    def _feed_forward(self, x, a, defer):
+        """x + a, its norm and the FFN: the layer's output, or with `defer` (stream, FFN output not yet added)."""
+        if layer.ffn_half_ok(x, a, self.n2.weight, self.up.weight, self.down.weight, not self.relu2):
+            return layer.ffn_half(x, a, self.n2.weight, self.up.weight, self.down.weight, _eps(self.n2), not self.relu2, not defer)
+        x, n2 = ops.add_rmsnorm(x, a, self.n2.weight, self.n2.eps)
         y = ops.ffn(n2, self.up.weight, self.down.weight, "relu2" if self.relu2 else "swiglu", direct=True)
         if defer:
             return x, y

@@ -203,6 +203,24 @@ class _Linear(torch.autograd.Function):
 WEIGHT_GRAD_SINK = None
 
 
+def shadow_bf16(w):
+    """The bf16 copy of an fp32 weight, made or brought up to date if need be."""
+    sh = getattr(w, "_bf16_shadow", None)
+    if sh is None or sh.shape != w.shape:
+        sh = w.detach().to(torch.bfloat16)
+        w._bf16_shadow, w._shadow_ver = sh, w._version
+    elif getattr(w, "_shadow_ver", None) != w._version:
+        sh.copy_(w.detach())                       # refreshed in place: the buffer may be one that other ranks write into
+        w._shadow_ver = w._version
+    return sh.detach()
+
+
+def offer_grad(w, g):
+    """Hand a weight's gradient to the optimizer; None when it was taken, else the gradient for autograd to accumulate."""
+    sink = WEIGHT_GRAD_SINK
+    return None if sink is not None and sink(w, g) else g
+
+
 class _WeightBf16(torch.autograd.Function):
     """fp32 master weight -> the bf16 operand of the GEMMs.
 
@@ -215,21 +233,11 @@ class _WeightBf16(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w):
         ctx.w = w
-        sh = getattr(w, "_bf16_shadow", None)
-        if sh is None or sh.shape != w.shape:
-            sh = w.detach().to(torch.bfloat16)
-            w._bf16_shadow, w._shadow_ver = sh, w._version
-        elif getattr(w, "_shadow_ver", None) != w._version:
-            sh.copy_(w.detach())                   # refreshed in place: the buffer may be one that other ranks write into
-            w._shadow_ver = w._version
-        return sh.detach()
+        return shadow_bf16(w)
 
     @staticmethod
     def backward(ctx, g):
-        sink = WEIGHT_GRAD_SINK
-        if sink is not None and sink(ctx.w, g):
-            return None
-        return g
+        return offer_grad(ctx.w, g)
 
 
 def weight_bf16(w, direct=False):
