@@ -19,6 +19,7 @@ void peer_gather(std::vector<int64_t> src_ptrs, torch::Tensor dst, int64_t rank,
 void peer_allreduce(std::vector<int64_t> in_ptrs, std::vector<int64_t> out_ptrs, int64_t mc_in, int64_t mc_out, int64_t offset,
                     int64_t numel, bool is_bf16, int64_t rank, double scale);
 void gemm_set_pair(bool on);
+bool gemm_pair_on();
 std::vector<torch::Tensor> rmsnorm_fwd(torch::Tensor x, torch::Tensor w, double eps, bool out_bf16);
 std::vector<torch::Tensor> rmsnorm_bwd(torch::Tensor dy, torch::Tensor x, torch::Tensor w, torch::Tensor rstd,
                                        c10::optional<torch::Tensor> add, bool want_lo);
@@ -99,6 +100,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_status", &mb::gemm_status, "read and clear the GEMM status word (0 = ok)");
   m.def("gemm_set_debug", &mb::gemm_set_debug, "pair kernel: test / measurement bits and row-tile group size of the tile order",
         pybind11::arg("dbg") = 0, pybind11::arg("group_m") = 0);
+  m.def("gemm_pair_on", &mb::gemm_pair_on);
   m.def("gemm_set_pair", &mb::gemm_set_pair, "switch the CTA-pair (cta_group::2) GEMM kernel on or off");
   m.def("gemm_peer", &mb::gemm_peer, "segmented GEMM: A tiles from peer buffers, result rows to the owners' buffers");
   m.def("peer_barrier", &mb::peer_barrier, "bounded device-side barrier over symmetric flags");

@@ -15,7 +15,7 @@ struct GemmParams {
   long long out_gs, out2_gs, aux_gs;   // group strides in elements
   int ldo, ldo2, ldaux;                // row pitches in elements
   int epi, out_f32, accumulate;
-  int m_tiles, n_tiles;
+  int m_tiles, n_tiles, bn;  // bn: columns of a tile (pair kernel: 256 or 128, else 256)
   int ntail;                 // 1: the last N tile issues MMAs only as wide as its valid columns (rounded up to 16)
   int* status;
   // M may be cut into `n_seg` segments of `seg_M` rows, each read through its own A tensor map (a peer GPU's

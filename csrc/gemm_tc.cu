@@ -175,9 +175,9 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, int g, int se
 // Width of the MMA for N tile `nt`: the full tile, or for a ragged last tile its valid columns rounded up to 16
 // (rows of B past N are zero-filled by TMA; accumulator columns past the width are never stored).
 __device__ __forceinline__ int tile_n_eff(const GemmParams& p, int nt) {
-  if (!p.ntail || p.epi == EPI_SWIGLU) return BN;
-  const int rem = p.N - nt * BN;
-  return rem >= BN ? BN : ((rem + 15) & ~15);
+  if (!p.ntail || p.epi == EPI_SWIGLU) return p.bn;
+  const int rem = p.N - nt * p.bn;
+  return rem >= p.bn ? p.bn : ((rem + 15) & ~15);
 }
 
 template <bool A_MN, bool B_MN>
@@ -474,7 +474,7 @@ __device__ __forceinline__ void aux_issue(const GemmParams& p, AuxPipe& a, uint8
     const int mseg0 = (mt - seg * p.tiles_per_seg) * 256 * a.mh;
     const bool skip_tile = seg * p.seg_M + mseg0 >= group_rows(p, g) || group_kblocks(p, g) == 0;
     const int h = a.pf_hc >> 2, c = a.pf_hc & 3;
-    const int col0 = nt * BN + c * 64;
+    const int col0 = nt * p.bn + c * 64;
     if (skip_tile || col0 >= p.N) {                     // next half / tile
       if (skip_tile || h + 1 >= a.mh) { a.pf_t += a.npairs; a.pf_hc = 0; }
       else a.pf_hc = (h + 1) << 2;
@@ -487,7 +487,7 @@ __device__ __forceinline__ void aux_issue(const GemmParams& p, AuxPipe& a, uint8
     tma_load_3d_local(b, a.tm, &a.bars[slot], col0, row0, g);
     if (a.nb == 2) tma_load_3d_local(b + EPI_BUF_BYTES, a.tm, &a.bars[slot], p.N + col0, row0, g);
     ++a.issued;
-    if (c == 3) {
+    if (c == (p.bn >> 6) - 1) {
       if (h + 1 >= a.mh) { a.pf_t += a.npairs; a.pf_hc = 0; }
       else a.pf_hc = (h + 1) << 2;
     } else {
@@ -522,8 +522,8 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
     if (aux != nullptr && aux->on) {
       // the staging tiles belong to the prefetch queue: zeros go out by plain 16-byte stores
       const int wide = p.epi == EPI_DSWIGLU ? 2 : 1;
-      for (int c = 0; c < BN / 64; ++c) {
-        const int col0 = nt * BN + c * 64;
+      for (int c = 0; c < p.bn / 64; ++c) {
+        const int col0 = nt * p.bn + c * 64;
         if (col0 >= p.N) break;
         const int pieces = min(8, (p.N - col0 + 7) >> 3), pc = lane & 7;
         for (int w = 0; w < wide; ++w)
@@ -544,8 +544,8 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
     __syncwarp();
     if (p.epi == EPI_SWIGLU) {
       const int H = p.N >> 1;
-      for (int c = 0; c < 2; ++c) {
-        const int col0 = nt * 128 + c * 64;
+      for (int c = 0; c < p.bn / 128; ++c) {
+        const int col0 = nt * (p.bn / 2) + c * 64;
         if (col0 >= H) break;
         epi_send(p, ring, bi, o, col0, row0, og, rows_valid, H, 2, false, lane);
         if (p.out2) {
@@ -555,8 +555,8 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
       }
     } else {
       const int cw = p.out_f32 ? 32 : 64;
-      for (int c = 0; c < BN / cw; ++c) {
-        const int col0 = nt * BN + c * cw;
+      for (int c = 0; c < p.bn / cw; ++c) {
+        const int col0 = nt * p.bn + c * cw;
         if (col0 >= p.N) break;
         epi_send(p, ring, bi, o, col0, row0, og, rows_valid, p.N, esz, false, lane);
         if (p.epi == EPI_RELU2) epi_send(p, ring, bi, o2, col0, row0, g, rows_valid, p.N, 2, false, lane);
@@ -576,15 +576,15 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
     const int H = p.N >> 1;
     const int nb = p.out2 ? 3 : 1;
 #pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      const int col0 = nt * 128 + c * 64;
+    for (int c = 0; c < p.bn / 128; ++c) {
+      const int col0 = nt * (p.bn / 2) + c * 64;
       if (col0 >= H) break;
       const int bi = ring.take(lane);
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t rg[32], ru[32];
         tmem_ld32(taddr + c * 64 + hf * 32, rg);
-        tmem_ld32(taddr + 128 + c * 64 + hf * 32, ru);
+        tmem_ld32(taddr + p.bn / 2 + c * 64 + hf * 32, ru);
         tmem_ld_wait();
         uint32_t ph[16], pg[16], pu[16];
 #pragma unroll
@@ -621,8 +621,8 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
   if (p.out_f32) {
     // fp32 output (weight gradients): 32 columns per staged tile
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      const int col0 = nt * BN + c * 32;
+    for (int c = 0; c < p.bn / 32; ++c) {
+      const int col0 = nt * p.bn + c * 32;
       if (col0 >= p.N) break;
       uint32_t r[32];
       tmem_ld32(taddr + c * 32, r);
@@ -649,8 +649,8 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
   oh.tm = tmO2;
   oh.base = o.base + static_cast<long long>(p.N) * 2;
 #pragma unroll 1
-  for (int c = 0; c < BN / 64; ++c) {
-    const int col0 = nt * BN + c * 64;
+  for (int c = 0; c < p.bn / 64; ++c) {
+    const int col0 = nt * p.bn + c * 64;
     if (col0 >= p.N) break;
     uint32_t r[64];
     tmem_ld32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
@@ -858,8 +858,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         const int ga = g + p.a_g_off;
         int num_kb = group_kblocks(p, g);
         const int kb0 = split_start(p, t, num_kb);
-        const int nb = (p.epi == EPI_SWIGLU) ? (rank == 0 ? nt * 128 : (p.N >> 1) + nt * 128)
-                                             : nt * BN + (int)rank * (tile_n_eff(p, nt) >> 1);
+        const int nb = (p.epi == EPI_SWIGLU) ? (rank == 0 ? 0 : (p.N >> 1)) + nt * (p.bn >> 1)
+                                             : nt * p.bn + (int)rank * (tile_n_eff(p, nt) >> 1);
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_try_wait(&empty[stage], phase ^ 1) && !mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
             atomicCAS(p.status, 0, ST_WAIT_EMPTY); *abort_flag = 1; ok = false; break;
@@ -867,7 +867,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
           uint8_t* sA = smem + stage * STAGE_B;
           uint8_t* sB = sA + MH * A_BYTES;
           const uint32_t lfull = mapa_shared(smem_u32(&full[stage]), 0);      // the leader's barrier
-          if (leader) mbar_expect_tx(&full[stage], 2 * STAGE_B);               // bytes of both CTAs
+          if (leader) mbar_expect_tx(&full[stage], 2 * (MH * A_BYTES + p.bn * BK));  // bytes of both CTAs: bn / 2 rows of B each
           const int k0 = (kb0 + kb) * BK;
 #pragma unroll
           for (int h = 0; h < MH; ++h) {                                       // this CTA's 128 rows of each 256-row block
@@ -883,7 +883,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
             tma_load_3d_pair(sB, &tmB, lfull, k0, nb, g);
           } else {
             tma_load_3d_pair(sB, &tmB, lfull, nb, k0, g);
-            tma_load_3d_pair(sB + 8192, &tmB, lfull, nb + 64, k0, g);
+            if (p.bn == BN) tma_load_3d_pair(sB + 8192, &tmB, lfull, nb + 64, k0, g);
           }
           if (++stage == STAGES3) { stage = 0; phase ^= 1; }
         }
@@ -1024,7 +1024,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         else acc_phase ^= 1;
       }
     }
-    if (ring.tma && lane == 0) bulk_wait_all<0>();           // staged tiles must be read before the CTA's smem goes away
+    if (ring.tma && lane == 0) bulk_wait_read<0>();          // staged tiles must be read before the CTA's smem goes away
     if (aux.on && lane == 0 && !ok) {
       // gave up with prefetches in flight: let them land (bounded) before the CTA's shared memory goes away
       for (uint32_t i = aux.consumed; i < aux.issued; ++i)
@@ -1143,11 +1143,19 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
   for (int i = n_seg; i < 8; ++i) tmAs.m[i] = tmAs.m[0];
   const bool pair = gemm_pair_on() && seg_M >= 256;
   const bool sw = p.epi == EPI_SWIGLU;
-  const int n_tiles = sw ? ((N / 2) + 127) / 128 : (N + BN - 1) / BN;
+  // Tiles of 128 columns where 256 would leave the CTA pairs short of work: the time of a small product is a pair's rounds of
+  // tiles times the width of one (its MMAs and its epilogue); 15 % in favour of the wide tile, which reads A half as often.
+  // Us, 256 -> 128 columns, (M, N, K): (2048, 256, 256) 8.8 -> 7.3; (2048, 256, 1024) 12.5 -> 11.1; (4096, 512, 512) 10.4 -> 9.3;
+  // (256, 1024, 2048) 11.5 -> 10.1.
+  auto tiles_of = [&](int bn) { return (long long)G * n_seg * ((seg_M + 255) / 256) * ((N + bn - 1) / bn) * std::max(1, p.splits); };
+  auto rounds = [&](int bn) { const long long pairs = std::max(1, max_ctas / 2); return (tiles_of(bn) + pairs - 1) / pairs; };
+  const bool narrow = pair && p.count_mode == 0 && rounds(128) * 128 * 115 < rounds(256) * 256 * 100;
+  p.bn = narrow ? 128 : BN;
+  const int n_tiles = (N + p.bn - 1) / p.bn;                 // SwiGLU: a tile holds bn / 2 columns of each half
   // 512-row tiles (see PairCfg) when the contraction is long enough to pay for the half-exposed epilogue and the
   // coarser tiling does not cost more in the last, partly filled wave of tiles than it saves
   bool tall = false;
-  if (pair && n_seg == 1 && p.count_mode == 0 && seg_M >= 1024 && !(sw && p.out2) && p.epi != EPI_DRELU2 &&
+  if (pair && !narrow && n_seg == 1 && p.count_mode == 0 && seg_M >= 1024 && !(sw && p.out2) && p.epi != EPI_DRELU2 &&
       p.epi != EPI_DSWIGLU) {
     auto wave_eff = [&](int tm) {
       const long long tiles = (long long)G * ((seg_M + tm - 1) / tm) * n_tiles, pairs = std::max(1, max_ctas / 2);
@@ -1161,7 +1169,7 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
   const int tile_m = pair ? (tall ? 512 : 256) : BM;
   p.n_seg = n_seg; p.seg_M = seg_M; p.tiles_per_seg = (seg_M + tile_m - 1) / tile_m;
   CUtensorMap tmB = b_mn ? make_tmap_bf16(B, N, K, G, b_rows_pitch, b_gs, 64, 64)
-                         : make_tmap_bf16(B, K, N, G, b_rows_pitch, b_gs, 64, (sw || pair) ? 128 : BN);
+                         : make_tmap_bf16(B, K, N, G, b_rows_pitch, b_gs, 64, pair ? p.bn / 2 : (sw ? 128 : BN));
   p.m_tiles = n_seg * p.tiles_per_seg;
   p.n_tiles = n_tiles;
   static const bool ntail_on = []() { const char* e = std::getenv("MEMARCH_GEMM_NTAIL"); return !(e && e[0] == '0'); }();

@@ -174,8 +174,9 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, ac
 
 
 def gemm_ok(M, N, K):
-    """Shapes the TMA descriptors accept: 16-byte row pitches (multiples of 8 bf16 elements)."""
-    return K % 8 == 0 and N % 8 == 0 and M % 8 == 0 and K >= 16
+    """Shapes the TMA descriptors accept: 16-byte row pitches (multiples of 8 bf16 elements).  Any number of rows M: it is
+    never an inner dimension (in the weight gradient it is the contraction, whose ragged end is filled with zeros)."""
+    return K % 8 == 0 and N % 8 == 0 and M >= 1 and K >= 16
 
 
 class _Linear(torch.autograd.Function):

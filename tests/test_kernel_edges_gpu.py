@@ -118,6 +118,44 @@ def test_gemm_split_contraction(M, N, K):
             assert _rel(acc, want + 1) < 1e-5
 
 
+# ------------------------------------------------------------------------------------------------ narrow tiles
+@pytest.mark.parametrize("M,N,K", [(2048, 256, 256), (257, 264, 128), (4095, 512, 520), (1001, 136, 64), (256, 1024, 2048), (9472, 256, 64), (513, 8, 16)])
+def test_gemm_narrow_tiles(M, N, K):
+    """128-column tiles and their neighbours under the rule, any number of rows: plain, relu2 and SwiGLU epilogues both ways."""
+    from memarch_b200.ops import gemm, linear
+    from memarch_b200.ops.basic import ffn
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, K, device="cuda", generator=g).bfloat16(), torch.randn(N, K, device="cuda", generator=g) * K ** -0.5
+    wd = torch.randn(K, N // 2, device="cuda", generator=g) * N ** -0.5
+    go = torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    xd, w2 = x.double(), w.bfloat16().double()
+    assert _rel(gemm(x, w.bfloat16()), xd @ w2.t()) < 4e-3
+    assert _rel(gemm(x, w.bfloat16(), out_dtype=torch.float32), xd @ w2.t()) < 1e-5
+    xg, wg = x.clone().requires_grad_(), w.clone().requires_grad_()
+    linear(xg, wg).backward(go)
+    assert _rel(xg.grad, go.double() @ w2) < 4e-3 and _rel(wg.grad, go.double().t() @ xd) < 4e-3
+    for act in ("swiglu", "relu2"):
+        H = N // 2 if act == "swiglu" else N
+        down = wd if act == "swiglu" else torch.cat([wd, wd], 1)
+        gy = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        got, want = [], []
+        for native in (True, False):
+            a, u, v = x.clone(), w.clone(), down.clone()
+            if not native:
+                a, u, v = xd.clone(), w2.clone(), down.bfloat16().double()
+            a.requires_grad_(), u.requires_grad_(), v.requires_grad_()
+            if native:
+                y = ffn(a, u, v, act)
+            else:
+                p = a @ u.t()
+                y = (torch.nn.functional.silu(p[:, :H]) * p[:, H:] if act == "swiglu" else p.relu().square()) @ v.t()
+            y.backward(gy.to(y.dtype))
+            (got if native else want).extend([y, a.grad, u.grad, v.grad])
+        # bf16 hidden activations and pre-activations: two to three roundings of 2^-9 along the chain
+        for q, r in zip(got, want):
+            assert _rel(q, r) < 1e-2
+
+
 # ------------------------------------------------------------------------------------------------ routing
 @pytest.mark.parametrize("N,d,E,k,C", [(1, 8, 1, 1, 1), (31, 64, 3, 2, 7), (33, 256, 8, 2, 64), (100, 264, 48, 4, 3), (700, 2048, 8, 2, 176), (257, 512, 128, 8, 9), (4000, 768, 16, 2, 626)])
 def test_route_and_slot_fused(N, d, E, k, C):
