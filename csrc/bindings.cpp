@@ -35,6 +35,10 @@ void ce_rows(torch::Tensor logits, torch::Tensor y, torch::Tensor loss, c10::opt
              c10::optional<torch::Tensor> hit, c10::optional<torch::Tensor> dg);
 torch::Tensor gather_rows(torch::Tensor src, torch::Tensor table, c10::optional<torch::Tensor> scale);
 torch::Tensor gather_sum_rows(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w, int64_t N);
+torch::Tensor rows_gather(torch::Tensor src, torch::Tensor table);
+torch::Tensor rows_gather_sum(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w);
+std::vector<torch::Tensor> combine_bwd(torch::Tensor go, torch::Tensor table, torch::Tensor w, torch::Tensor ye);
+void err_probe(torch::Tensor g, torch::Tensor buf);
 torch::Tensor row_dot(torch::Tensor go, torch::Tensor table, torch::Tensor ye);
 int64_t instinct_step(torch::Tensor p, torch::Tensor grad, torch::Tensor m, c10::optional<torch::Tensor> w,
                       c10::optional<torch::Tensor> cs, torch::Tensor gvec, int64_t index, torch::Tensor stake,
@@ -123,6 +127,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_rows", &mb::gather_rows);
   m.def("gather_sum_rows", &mb::gather_sum_rows);
   m.def("row_dot", &mb::row_dot);
+  m.def("rows_gather", &mb::rows_gather);
+  m.def("rows_gather_sum", &mb::rows_gather_sum);
+  m.def("combine_bwd", &mb::combine_bwd);
+  m.def("err_probe", &mb::err_probe);
   m.def("instinct_step", &mb::instinct_step, pybind11::arg("p"), pybind11::arg("grad"), pybind11::arg("m"), pybind11::arg("w"),
         pybind11::arg("cs"), pybind11::arg("gvec"), pybind11::arg("index"), pybind11::arg("stake"), pybind11::arg("lr_t"),
         pybind11::arg("rel"), pybind11::arg("beta"), pybind11::arg("wd"), pybind11::arg("kind"), pybind11::arg("sr"),

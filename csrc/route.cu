@@ -9,14 +9,14 @@
 //   aux = E * sum_e (choices of e / all choices) * (mean probability of e over the real tokens).
 // Backward 1 (route_dx_kernel): gradient of the logits from the gradients of the weights, of the place weights and of aux, and
 // dx = dlogits W.  Backward 2 (route_dw_kernel): dW = dlogits^T x.
-// All of it is memory-bound on x (33 MB for 8192 x 2048).  A warp takes 8 tokens at a time, so that W (E x d fp32) is read
-// once per 8 tokens and mostly from L1.  ROUTE_TIME
+// All of it is memory-bound on x (33 MB for 8192 x 2048).  A warp takes 4 or 8 tokens at a time, so that W (E x d fp32) is
+// read once for them and mostly from L1 (the choice stands at route_fwd_launch).  Us for 8192 x 2048, 8 experts, 8 tokens per
+// warp -> 4: route_fwd 59 -> 30, route_dx 55 -> 44; route_dw with 64 tokens per block instead of 256: 48 -> 17.
 #include "common.cuh"
 #include "route_api.h"
 
 namespace mb {
 
-constexpr int RT_WARPS = 4, RT_TOK = ROUTE_TOK / RT_WARPS;      // 8 tokens per warp
 
 __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -29,7 +29,9 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-__global__ void __launch_bounds__(RT_WARPS * 32) route_fwd_kernel(RouteArgs a) {
+template <int TOK>
+__global__ void __launch_bounds__(ROUTE_TOK / TOK * 32) route_fwd_kernel(RouteArgs a) {
+  constexpr int EXP = 32 / TOK;                          // experts at a time: 32 sums per lane
   __shared__ float ps_sh[ROUTE_E];
   __shared__ int cnt_sh[ROUTE_E], real_sh;
   extern __shared__ float lg_sh[];                       // (ROUTE_TOK, E) logits
@@ -37,35 +39,29 @@ __global__ void __launch_bounds__(RT_WARPS * 32) route_fwd_kernel(RouteArgs a) {
   for (int i = threadIdx.x; i < E; i += blockDim.x) { ps_sh[i] = 0.f; cnt_sh[i] = 0; }
   if (threadIdx.x == 0) real_sh = 0;
   __syncthreads();
-  const int n0 = blockIdx.x * ROUTE_TOK + warp * RT_TOK;
-  const int nt = min(RT_TOK, a.N - n0);                  // may be <= 0
+  const int n0 = blockIdx.x * ROUTE_TOK + warp * TOK;
+  const int nt = min(TOK, a.N - n0);                  // may be <= 0
   const bf16* X = reinterpret_cast<const bf16*>(a.x);
-  float* lg = lg_sh + warp * RT_TOK * E;
-  // 8 tokens x 4 experts at a time: every lane sums its columns, then the 32 sums are reduced over the lanes, the lane that
-  // ends up with sum v = token * 4 + expert writes it
-  for (int e0 = 0; e0 < E; e0 += 4) {
+  float* lg = lg_sh + warp * TOK * E;
+  // TOK tokens x EXP experts at a time: every lane sums its columns, then the 32 sums are reduced over the lanes, the lane that
+  // ends up with sum v = token * EXP + expert writes it
+  for (int e0 = 0; e0 < E; e0 += EXP) {
     float acc[32];
 #pragma unroll
     for (int v = 0; v < 32; ++v) acc[v] = 0.f;
     if (nt > 0) {
       for (int c = lane * 8; c < a.d; c += 256) {
-        float w[4][8];
+        float x[TOK][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (e0 + j < E) load8(a.w + (long long)(e0 + j) * a.d + c, w[j]);
-          else {
+        for (int t = 0; t < TOK; ++t) load8(X + (long long)(n0 + min(t, nt - 1)) * a.d + c, x[t]);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) w[j][u] = 0.f;
-          }
-        }
+        for (int j = 0; j < EXP; ++j) {
+          float w[8];
+          load8(a.w + (long long)min(e0 + j, E - 1) * a.d + c, w);       // experts past the last are not written
 #pragma unroll
-        for (int t = 0; t < RT_TOK; ++t) {
-          float x[8];
-          load8(X + (long long)(n0 + min(t, nt - 1)) * a.d + c, x);
+          for (int t = 0; t < TOK; ++t)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int u = 0; u < 8; ++u) acc[t * 4 + j] = fmaf(x[u], w[j][u], acc[t * 4 + j]);
+            for (int u = 0; u < 8; ++u) acc[t * EXP + j] = fmaf(x[t][u], w[u], acc[t * EXP + j]);
         }
       }
     }
@@ -79,7 +75,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) route_fwd_kernel(RouteArgs a) {
         acc[v] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
-    const int t = lane >> 2, e = e0 + (lane & 3);
+    const int t = lane / EXP, e = e0 + lane % EXP;
     if (e < E) lg[t * E + e] = acc[0];
   }
   __syncwarp();
@@ -218,14 +214,15 @@ __global__ void __launch_bounds__(256) route_place_kernel(RouteArgs a) {
   }
 }
 
-__global__ void __launch_bounds__(RT_WARPS * 32) route_dx_kernel(RouteArgs a) {
+template <int TOK>
+__global__ void __launch_bounds__(ROUTE_TOK / TOK * 32) route_dx_kernel(RouteArgs a) {
   extern __shared__ float dl_sh[];                       // (ROUTE_TOK, E)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = a.E;
-  const int n0 = blockIdx.x * ROUTE_TOK + warp * RT_TOK;
-  const int nt = min(RT_TOK, a.N - n0);
-  float* dl = dl_sh + warp * RT_TOK * E;
+  const int n0 = blockIdx.x * ROUTE_TOK + warp * TOK;
+  const int nt = min(TOK, a.N - n0);
+  float* dl = dl_sh + warp * TOK * E;
   const float d_aux = a.d_aux ? *a.d_aux : 0.f;
-  for (int t = 0; t < RT_TOK; ++t) {
+  for (int t = 0; t < TOK; ++t) {
     if (t >= nt) {                                       // absent tokens of the last block
       for (int e = lane; e < E; e += 32) dl[t * E + e] = 0.f;
       continue;
@@ -278,23 +275,23 @@ __global__ void __launch_bounds__(RT_WARPS * 32) route_dx_kernel(RouteArgs a) {
   if (nt <= 0) return;
   bf16* DX = reinterpret_cast<bf16*>(a.dx);
   for (int c = lane * 8; c < a.d; c += 256) {
-    float acc[RT_TOK][8];
+    float acc[TOK][8];
 #pragma unroll
-    for (int t = 0; t < RT_TOK; ++t)
+    for (int t = 0; t < TOK; ++t)
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[t][u] = 0.f;
     for (int e = 0; e < E; ++e) {
       float w[8];
       load8(a.w + (long long)e * a.d + c, w);
 #pragma unroll
-      for (int t = 0; t < RT_TOK; ++t) {
+      for (int t = 0; t < TOK; ++t) {
         const float v = dl[t * E + e];
 #pragma unroll
         for (int u = 0; u < 8; ++u) acc[t][u] = fmaf(v, w[u], acc[t][u]);
       }
     }
 #pragma unroll
-    for (int t = 0; t < RT_TOK; ++t)
+    for (int t = 0; t < TOK; ++t)
       if (t < nt)
         *reinterpret_cast<uint4*>(DX + (long long)(n0 + t) * a.d + c) =
             make_uint4(pack_bf16(acc[t][0], acc[t][1]), pack_bf16(acc[t][2], acc[t][3]), pack_bf16(acc[t][4], acc[t][5]), pack_bf16(acc[t][6], acc[t][7]));
@@ -332,14 +329,21 @@ __global__ void __launch_bounds__(256) route_dw_kernel(RouteArgs a) {
     }
 }
 
+// 4 tokens per warp and 8 experts at a time keep twice the warps in flight; with many experts W no longer fits L1 and 8
+// tokens per warp halve its traffic
 void route_fwd_launch(const RouteArgs& a) {
   const int nb = route_blocks(a.N);
-  route_fwd_kernel<<<nb, RT_WARPS * 32, (size_t)ROUTE_TOK * a.E * 4, a.stream>>>(a);
+  const size_t smem = (size_t)ROUTE_TOK * a.E * 4;
+  if (a.E <= 16) route_fwd_kernel<4><<<nb, ROUTE_TOK / 4 * 32, smem, a.stream>>>(a);
+  else route_fwd_kernel<8><<<nb, ROUTE_TOK / 8 * 32, smem, a.stream>>>(a);
   route_place_kernel<<<nb, 256, 0, a.stream>>>(a);
 }
 void route_bwd_launch(const RouteArgs& a) {
+  const int nb = route_blocks(a.N);
+  const size_t smem = (size_t)ROUTE_TOK * a.E * 4;
   cudaMemsetAsync(a.dw, 0, sizeof(float) * (size_t)a.E * a.d, a.stream);
-  route_dx_kernel<<<route_blocks(a.N), RT_WARPS * 32, (size_t)ROUTE_TOK * a.E * 4, a.stream>>>(a);
+  if (a.E <= 16) route_dx_kernel<4><<<nb, ROUTE_TOK / 4 * 32, smem, a.stream>>>(a);
+  else route_dx_kernel<8><<<nb, ROUTE_TOK / 8 * 32, smem, a.stream>>>(a);
   route_dw_kernel<<<dim3((a.d + 511) / 512, (a.N + DW_RUN - 1) / DW_RUN, (a.E + 7) / 8), 256, 0, a.stream>>>(a);
 }
 

@@ -4,8 +4,8 @@ Reference behaviour: capacity slotting by cumulative rank, slot table gather `xp
 SwiGLU or relu², weighted `index_add` combine (full2.py:532-602, 1102-1110), and the gather-only inverse pair
 `_SlotGather` / `_CombineW` (full2.py:283-328) whose backward needs no scatter-add.
 
-GPU bodies: `gather_rows` (slot <- token, optional per-row scale), `gather_sum_rows` (token <- its k slots, weighted,
-fp32 accumulate), `row_dot` (slot-weight grads) and the grouped tcgen05 GEMMs with the activation in the epilogue.
+GPU bodies: `rows_gather` (slot <- token), `rows_gather_sum` (token <- its k slots, weighted, fp32 accumulate), `combine_bwd`
+(gradients of the slots and of their weights; `gather_rows`, `gather_sum_rows`, `row_dot` for other row types) and the grouped tcgen05 GEMMs with the activation in the epilogue.
 """
 from __future__ import annotations
 
@@ -18,6 +18,11 @@ from .basic import gemm, gemm_ok, relu2, swiglu
 
 
 # ------------------------------------------------------------------------------------------------ dispatch
+def _wide(*ts):
+    """Rows the 16-byte kernels of `csrc/gather.cu` take; the others stay on the element-wise ones."""
+    return all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape[-1] % 8 == 0 and t.data_ptr() % 16 == 0 for t in ts)
+
+
 class _SlotGather(torch.autograd.Function):
     """xe[s] = x[table[s]] (empty slot -> 0).  Backward: dx[n] = Σ_j dxe[flat_idx[n, j]] in fp32."""
 
@@ -27,7 +32,8 @@ class _SlotGather(torch.autograd.Function):
         ctx.N = x.shape[0]
         if _ext.use_cuda(x):
             _ext.count()
-            return _ext.C().gather_rows(x.contiguous(), table, None)
+            x = x.contiguous()
+            return _ext.C().rows_gather(x, table) if _wide(x) else _ext.C().gather_rows(x, table, None)
         N = x.shape[0]
         m = (table < N)[:, None]
         return torch.where(m, x[table.clamp(max=N - 1)], x.new_zeros(()))
@@ -37,7 +43,8 @@ class _SlotGather(torch.autograd.Function):
         table, fi = ctx.saved_tensors
         if _ext.use_cuda(g):
             _ext.count()
-            return _ext.C().gather_sum_rows(g.contiguous(), fi, None, ctx.N), None, None
+            g = g.contiguous()
+            return (_ext.C().rows_gather_sum(g, fi, None) if _wide(g) else _ext.C().gather_sum_rows(g, fi, None, ctx.N)), None, None
         EC = g.shape[0]
         mk = (fi < EC)[..., None]
         dx = torch.where(mk, g[fi.clamp(max=EC - 1)], g.new_zeros(())).float().sum(1).to(g.dtype)
@@ -54,7 +61,8 @@ class _CombineW(torch.autograd.Function):
         ctx.N = N
         if _ext.use_cuda(ye):
             _ext.count()
-            return _ext.C().gather_sum_rows(ye.contiguous(), fi, wtab.float().contiguous(), N)
+            ye, wf = ye.contiguous(), wtab.float().contiguous()
+            return _ext.C().rows_gather_sum(ye, fi, wf) if _wide(ye) else _ext.C().gather_sum_rows(ye, fi, wf, N)
         EC = ye.shape[0]
         c = fi.clamp(max=EC - 1)
         mk = fi < EC
@@ -67,7 +75,11 @@ class _CombineW(torch.autograd.Function):
         N = ctx.N
         if _ext.use_cuda(go):
             C = _ext.C()
-            go = go.contiguous()
+            go, ye = go.contiguous(), ye.contiguous()
+            if _wide(go, ye):
+                dye, dw = C.combine_bwd(go, table, wtab.float().contiguous(), ye)
+                _ext.count()
+                return dye, dw.to(wtab.dtype), None, None, None
             dye = C.gather_rows(go, table, wtab.float().contiguous())
             dw = C.row_dot(go, table, ye.contiguous())
             _ext.count(2)

@@ -185,6 +185,49 @@ def test_route_and_slot_fused(N, d, E, k, C):
     assert _rel(xg.grad.cpu(), xc.grad) < 4e-3 and _rel(wg.grad.cpu(), wc.grad) < 1e-4
 
 
+# ------------------------------------------------------------------------------------------------ expert rows
+@pytest.mark.parametrize("N,d,E,C,k", [(1, 8, 1, 1, 1), (37, 264, 3, 7, 2), (300, 1032, 8, 64, 2), (65, 2048, 4, 33, 4), (50, 100, 2, 9, 2), (500, 768, 2, 100, 8)])
+def test_expert_row_moves(N, d, E, C, k):
+    """Gather, weighted combine and their gradients with empty places, dropped and unwanted choices; widths that are no multiple
+    of 8 take the element-wise kernels."""
+    from memarch_b200.ops import moe as ops_moe
+    g = torch.Generator().manual_seed(N * d)
+    S = E * C
+    place = torch.randperm(max(S, N * k) + 3, generator=g)[:N * k].view(N, k)
+    flat = torch.where(place < S, place, torch.full_like(place, S))
+    table = torch.full((S + 1,), N)
+    table[flat.reshape(-1)] = torch.arange(N)[:, None].expand(N, k).reshape(-1)
+    table = table[:-1].contiguous()
+    x, ye, w = torch.randn(N, d, generator=g).bfloat16(), torch.randn(S, d, generator=g).bfloat16(), torch.rand(S, generator=g)
+    gx, go = torch.randn(S, d, generator=g).bfloat16(), torch.randn(N, d, generator=g).bfloat16()
+    res = []
+    for dev in ("cuda", "cpu"):
+        a, b, c = (t.to(dev).clone().requires_grad_() for t in (x, ye, w))
+        f, t = flat.to(dev), table.to(dev)
+        xe = ops_moe.slot_gather(a, t, f)
+        y = ops_moe.combine(b, c, f, t, N)
+        xe.backward(gx.to(dev)), y.backward(go.to(dev))
+        res.append([xe, y, a.grad, b.grad, c.grad])
+    for i, (a, b) in enumerate(zip(*res)):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        if i == 0:
+            assert torch.equal(a.cpu(), b)
+        else:
+            assert _rel(a.cpu(), b) < 4e-3
+
+
+@pytest.mark.parametrize("E,C,d", [(1, 1, 8), (3, 7, 264), (8, 1025, 768), (5, 63, 2048), (2, 9, 100)])
+def test_expert_error_probe(E, C, d):
+    from memarch_b200.models.moe import _ErrProbe
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x = torch.randn(E, C, d, device="cuda", generator=g).bfloat16().requires_grad_()
+    grad = torch.randn(E, C, d, device="cuda", generator=g).bfloat16()
+    buf = torch.rand(E, device="cuda", generator=g)
+    want = 0.9 * buf.double() + 0.1 * grad.double().norm(dim=-1).mean(1)
+    _ErrProbe.apply(x, buf).backward(grad)
+    assert torch.equal(x.grad, grad) and (buf.double() - want).abs().max() < 1e-5 * want.max()
+
+
 # ------------------------------------------------------------------------------------------------ optimizer
 @pytest.mark.parametrize("shape,bf16", [((1190, 2048), False), ((1200, 1540), True), ((2500, 6144), True), ((1300, 4100), False), ((1024, 4096), False),
                                         ((3072, 1024), False), ((5, 700, 1540), True), ((3, 640, 2304), True), ((12000, 512), False), ((260, 256), False)])
