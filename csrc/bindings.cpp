@@ -35,6 +35,10 @@ void ce_rows(torch::Tensor logits, torch::Tensor y, torch::Tensor loss, c10::opt
              c10::optional<torch::Tensor> hit, c10::optional<torch::Tensor> dg);
 torch::Tensor gather_rows(torch::Tensor src, torch::Tensor table, c10::optional<torch::Tensor> scale);
 torch::Tensor gather_sum_rows(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w, int64_t N);
+torch::Tensor dequant_i8(torch::Tensor q, torch::Tensor scale);
+std::vector<torch::Tensor> quant_rows_wide(torch::Tensor x);
+torch::Tensor groups_take(torch::Tensor src, torch::Tensor idx);
+torch::Tensor groups_put(torch::Tensor a, torch::Tensor ia, torch::Tensor b, torch::Tensor ib);
 torch::Tensor rows_gather(torch::Tensor src, torch::Tensor table);
 torch::Tensor rows_gather_sum(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w);
 std::vector<torch::Tensor> combine_bwd(torch::Tensor go, torch::Tensor table, torch::Tensor w, torch::Tensor ye);
@@ -127,6 +131,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_rows", &mb::gather_rows);
   m.def("gather_sum_rows", &mb::gather_sum_rows);
   m.def("row_dot", &mb::row_dot);
+  m.def("dequant_i8", &mb::dequant_i8);
+  m.def("quant_rows_wide", &mb::quant_rows_wide);
+  m.def("groups_take", &mb::groups_take);
+  m.def("groups_put", &mb::groups_put);
   m.def("rows_gather", &mb::rows_gather);
   m.def("rows_gather_sum", &mb::rows_gather_sum);
   m.def("combine_bwd", &mb::combine_bwd);

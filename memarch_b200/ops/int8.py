@@ -28,12 +28,20 @@ def i8_ok(M, N, K):
     return K % 16 == 0 and K >= 32 and M >= 1 and N >= 1
 
 
+def quant_rows(x):
+    """(int8 rows, fp32 scales) of contiguous bf16 / fp32 rows on the GPU."""
+    C = _ext.C()
+    if x.shape[-1] % 8 == 0 and x.shape[-1] > 0 and x.data_ptr() % 16 == 0 and x.dtype in (torch.bfloat16, torch.float32) and x.dim() >= 2:
+        return C.quant_rows_wide(x)
+    return C.quant_rows_i8(x)
+
+
 def quant_mm(x, w, out_dtype=torch.bfloat16):
     """Q_row(x) · Q_row(w)ᵀ with the scales applied: x (M,K) or (G,M,K), w (N,K) or (G,N,K), floating point in,
     int8 tensor cores on the GPU."""
     C = _ext.C()
-    qx, sx = C.quant_rows_i8(x.contiguous())
-    qw, sw = C.quant_rows_i8(w.contiguous())
+    qx, sx = quant_rows(x.contiguous())
+    qw, sw = quant_rows(w.contiguous())
     _ext.count(3)
     return C.gemm_i8(qx, qw, sx, sw, out_dtype == torch.float32)
 
@@ -42,7 +50,7 @@ def quant_mm_stored(x, w_q, w_s, out_dtype=torch.bfloat16):
     """Q_row(x) · w_qᵀ with the scales applied, for weights already stored as int8: x (G,M,K) floating point,
     w_q (G,N,K) int8, w_s (G,N) fp32 scale of every output column."""
     C = _ext.C()
-    qx, sx = C.quant_rows_i8(x.contiguous())
+    qx, sx = quant_rows(x.contiguous())
     _ext.count(2)
     return C.gemm_i8(qx, w_q, sx, w_s, out_dtype == torch.float32)
 

@@ -13,7 +13,7 @@ import os
 
 import torch
 
-from . import _ext, ref
+from . import _ext, basic, ref
 from .basic import gemm, gemm_ok, relu2, swiglu
 
 
@@ -142,6 +142,8 @@ class _ExpertFFN(torch.autograd.Function):
         kw = dict(groups=E, counts=counts, count_mode=cm)
         if ctx.act == "relu2":
             da = gemm(dy, down, epi=2, aux=a, **kw)                            # dh · 2relu(a)
+        elif basic.FUSE_DSWIGLU and dy.shape[1] >= 256 and h.shape[2] % 8 == 0 and _ext.C().gemm_pair_on():
+            da = gemm(dy, down, epi=5, aux=a, **kw)                            # SwiGLU backward in the epilogue
         else:
             dh = gemm(dy, down, **kw)
             da = _ext.C().swiglu_bwd(dh, a)

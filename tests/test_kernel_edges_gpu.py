@@ -228,6 +228,71 @@ def test_expert_error_probe(E, C, d):
     assert torch.equal(x.grad, grad) and (buf.double() - want).abs().max() < 1e-5 * want.max()
 
 
+# ------------------------------------------------------------------------------------------------ frozen bank
+@pytest.mark.parametrize("E,C,d", [(3, 7, 264), (8, 1025, 768), (2, 9, 100), (2, 1, 9)])
+def test_bank_group_moves(E, C, d):
+    """Groups to the learning and the frozen experts and back; groups that are no multiple of 16 bytes take the general ops."""
+    from memarch_b200.models.moe import _JoinGroups, _SplitGroups
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x = torch.randn(E, C, d, device="cuda", generator=g).bfloat16().requires_grad_()
+    grad = torch.randn(E, C, d, device="cuda", generator=g).bfloat16()
+    order = torch.randperm(E, device="cuda", generator=g)
+    l, f = order[:E // 2].contiguous(), order[E // 2:].contiguous()
+    xl, xf = _SplitGroups.apply(x, l, f)
+    assert torch.equal(xl, x[l]) and torch.equal(xf, x[f])
+    y = _JoinGroups.apply(xl * 2, xf * 3, l, f)
+    y.backward(grad)
+    scale = torch.full((E, 1, 1), 2.0, device="cuda").index_fill_(0, f, 3.0).bfloat16()
+    assert torch.equal(y, x * scale) and torch.equal(x.grad, grad * scale)
+
+
+@pytest.mark.parametrize("F,I,O", [(1, 1, 8), (3, 33, 264), (4, 768, 1536)])
+def test_bank_dequantise(F, I, O):
+    from memarch_b200.ops import _ext
+    g = torch.Generator(device="cuda").manual_seed(I)
+    q = torch.randint(-127, 128, (F, I, O), device="cuda", generator=g).to(torch.int8)
+    s = torch.rand(F, 1, O, device="cuda", generator=g).bfloat16()
+    assert torch.equal(_ext.C().dequant_i8(q, s), q.to(torch.bfloat16) * s)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("R,K", [(1, 8), (9, 264), (2000, 1536), (5, 100)])
+def test_quantised_rows(R, K, dtype):
+    """Both row kernels and the PyTorch statement give the same bytes (zero rows and the largest element included)."""
+    from memarch_b200.ops import _ext, int8
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = (torch.randn(R, K, device="cuda", generator=g) * 3).to(dtype)
+    x[R // 2] = 0
+    q, s = int8.quant_rows(x)
+    q0, s0 = _ext.C().quant_rows_i8(x)
+    assert torch.equal(q, q0) and torch.equal(s, s0)
+
+
+@pytest.mark.parametrize("act", ["swiglu", "relu2"])
+@pytest.mark.parametrize("E,C,d,H", [(2, 255, 64, 64), (2, 256, 64, 64), (3, 300, 128, 200), (1, 513, 72, 136)])
+def test_expert_ffn_backward_epilogue(E, C, d, H, act):
+    from memarch_b200.ops.moe import expert_ffn
+    g = torch.Generator(device="cuda").manual_seed(C)
+    x = torch.randn(E, C, d, device="cuda", generator=g).bfloat16()
+    up = (torch.randn(E, d, 2 * H if act == "swiglu" else H, device="cuda", generator=g) * d ** -0.5).bfloat16()
+    down = (torch.randn(E, H, d, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    gy = torch.randn(E, C, d, device="cuda", generator=g).bfloat16()
+    res = []
+    for native in (True, False):
+        t = [v.clone() if native else v.double() for v in (x, up, down)]
+        [v.requires_grad_() for v in t]
+        if native:
+            y = expert_ffn(*t, act)
+        else:
+            p = t[0] @ t[1]
+            y = (torch.nn.functional.silu(p[..., :H]) * p[..., H:] if act == "swiglu" else p.relu().square()) @ t[2]
+        y.backward(gy.to(y.dtype))
+        res.append([y] + [v.grad for v in t])
+    # bf16 activations, pre-activations and their gradients: two to three roundings of 2^-9 along the chain
+    for a, b in zip(*res):
+        assert _rel(a, b) < 1e-2
+
+
 # ------------------------------------------------------------------------------------------------ optimizer
 @pytest.mark.parametrize("shape,bf16", [((1190, 2048), False), ((1200, 1540), True), ((2500, 6144), True), ((1300, 4100), False), ((1024, 4096), False),
                                         ((3072, 1024), False), ((5, 700, 1540), True), ((3, 640, 2304), True), ((12000, 512), False), ((260, 256), False)])
