@@ -28,23 +28,49 @@ constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTE
 constexpr int GEMM_THREADS = 192;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int GROUP_M = 8;
+constexpr int MAX_COUNT_G = 128;          // groups whose row tiles are counted in shared memory (more keep the plain order)
 
 struct TmapSet { CUtensorMap m[8]; };
 
-// work item t -> group, row tile, column tile (the items of one output tile's splits are neighbours)
-__device__ __forceinline__ void tile_coords(int t, const GemmParams& p, int& g, int& mt, int& nt) {
-  if (p.splits > 1) t /= p.splits;
-  int per_g = p.m_tiles * p.n_tiles;
-  g = t / per_g;
-  int r = t - g * per_g;
+// tile r of a group of m_tiles row tiles, bands of row tiles first
+__device__ __forceinline__ void band_coords(int r, int m_tiles, const GemmParams& p, int& mt, int& nt) {
   const int gm = p.group_m > 0 ? p.group_m : GROUP_M;
   int band = gm * p.n_tiles;
   int b = r / band;
   int first_m = b * gm;
-  int gsz = min(gm, p.m_tiles - first_m);
+  int gsz = min(gm, m_tiles - first_m);
   int rr = r - b * band;
   mt = first_m + rr % gsz;
   nt = rr / gsz;
+}
+
+// work item t -> group, row tile, column tile (the items of one output tile's splits are neighbours).
+// `cum` (count mode 1): row tiles with rows in the groups before each.  The tiles that are computed come first and those of
+// padding rows, which are only cleared, after them, so that every pair gets its share of both: dealt out by position, tiles
+// of padding fell to some pairs and not to others (with 7 of 8 row tiles filled, to every second one).
+// Us, the four products of 8 experts (2048 wide, hidden 4096) with some 12 000 of 8 x 2561 places filled: 1258 -> 1047.
+__device__ __forceinline__ void tile_coords(int t, const GemmParams& p, int& g, int& mt, int& nt, const int* cum = nullptr) {
+  if (p.splits > 1) t /= p.splits;
+  if (cum != nullptr) {
+    const int full = cum[p.G] * p.n_tiles;
+    const bool pad = t >= full;
+    if (pad) t -= full;
+    auto first = [&](int i) { return pad ? i * p.m_tiles - cum[i] : cum[i]; };     // row tiles of this kind before group i
+    const int row = t / p.n_tiles;
+    int lo = 0, hi = p.G;                                                          // first(lo) <= row < first(hi)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (first(mid) <= row) lo = mid; else hi = mid;
+    }
+    g = lo;
+    const int have = cum[g + 1] - cum[g];
+    band_coords(t - first(g) * p.n_tiles, pad ? p.m_tiles - have : have, p, mt, nt);
+    if (pad) mt += have;
+    return;
+  }
+  int per_g = p.m_tiles * p.n_tiles;
+  g = t / per_g;
+  band_coords(t - g * per_g, p.m_tiles, p, mt, nt);
 }
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -450,6 +476,7 @@ struct AuxPipe {
   uint32_t issued, consumed;
   int pf_t, pf_hc;         // cursor of the next chunk to fetch: tile, half * 4 + chunk
   const CUtensorMap* tm;
+  const int* cum;          // see tile_coords
   int rank, q, npairs, total, mh;
   bool on;
 };
@@ -469,7 +496,7 @@ __device__ __forceinline__ int group_kblocks(const GemmParams& p, int g);
 __device__ __forceinline__ void aux_issue(const GemmParams& p, AuxPipe& a, uint8_t* ring_base) {
   while (a.issued - a.consumed < (uint32_t)a.slots && a.pf_t < a.total) {
     int g, mt, nt;
-    tile_coords(a.pf_t, p, g, mt, nt);
+    tile_coords(a.pf_t, p, g, mt, nt, a.cum);
     const int seg = mt / p.tiles_per_seg;
     const int mseg0 = (mt - seg * p.tiles_per_seg) * 256 * a.mh;
     const bool skip_tile = seg * p.seg_M + mseg0 >= group_rows(p, g) || group_kblocks(p, g) == 0;
@@ -816,6 +843,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int total = p.G * p.m_tiles * p.n_tiles * max(1, p.splits);
+  __shared__ int cum_s[MAX_COUNT_G + 1];
+  const int* cum = p.count_mode == 1 && p.n_seg == 1 && p.G <= MAX_COUNT_G ? cum_s : nullptr;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES3; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -830,6 +859,21 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
       mbar_fence_init();
       tma_prefetch_desc(&tmX);
     }
+  }
+  if (cum != nullptr && warp == 2) {
+    // running sums of the groups' row tiles, 32 groups at a time
+    int run = 0;
+    for (int g0 = 0; g0 < p.G; g0 += 32) {
+      int v = g0 + lane < p.G ? (max(0, group_rows(p, g0 + lane)) + TILE_M - 1) / TILE_M : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (g0 + lane < p.G) cum_s[g0 + lane + 1] = run + v;
+      run += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) cum_s[0] = 0;
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -849,7 +893,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
       bool ok = true;
       for (int t = pair; t < total && ok; t += npairs) {
         int g, mt, nt;
-        tile_coords(t, p, g, mt, nt);
+        tile_coords(t, p, g, mt, nt, cum);
         const int seg = mt / p.tiles_per_seg;
         const int mseg0 = (mt - seg * p.tiles_per_seg) * TILE_M;
         if (seg * p.seg_M + mseg0 >= group_rows(p, g)) continue;            // a tile of padding rows
@@ -914,7 +958,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         nkb = 0; idesc = 0;
         if (t >= total) return;
         int g_, mt_, nt_;
-        tile_coords(t, p, g_, mt_, nt_);
+        tile_coords(t, p, g_, mt_, nt_, cum);
         const int seg = mt_ / p.tiles_per_seg;
         if (seg * p.seg_M + (mt_ - seg * p.tiles_per_seg) * TILE_M >= group_rows(p, g_)) return;
         nkb = group_kblocks(p, g_);
@@ -988,13 +1032,13 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
     aux.nb = ring.nb;
     aux.slots = EPI_NBUF / ring.nb;
     aux.issued = aux.consumed = 0;
-    aux.pf_t = pair; aux.pf_hc = 0;
+    aux.pf_t = pair; aux.pf_hc = 0; aux.cum = cum;
     aux.tm = &tmX;
     aux.rank = (int)rank; aux.q = q; aux.npairs = npairs; aux.total = total; aux.mh = MH;
     if (aux.on && lane == 0) aux_issue(p, aux, ring.base);
     for (int t = pair; t < total && ok; t += npairs) {
       int g, mt, nt;
-      tile_coords(t, p, g, mt, nt);
+      tile_coords(t, p, g, mt, nt, cum);
       const int seg = mt / p.tiles_per_seg;
       const int mseg0 = (mt - seg * p.tiles_per_seg) * TILE_M;
       const bool zero_tile = seg * p.seg_M + mseg0 >= group_rows(p, g) || group_kblocks(p, g) == 0;

@@ -407,3 +407,28 @@ def test_light_layer_halves_leave_other_cases_alone():
     assert not ok(x.clone().requires_grad_())
     with torch.no_grad():
         assert ok(x)
+
+
+# ------------------------------------------------------------------------------------------------ padded groups
+@pytest.mark.parametrize("E,C,counts", [(1, 256, [3]), (3, 2561, [2561, 0, 257]), (8, 600, [0, 600, 256, 255, 1, 0, 512, 300]), (128, 257, "mixed"), (130, 300, "mixed"), (2, 300, [0, 0])])
+@pytest.mark.parametrize("act", ["swiglu", "relu2"])
+def test_expert_ffn_counts_order(E, C, counts, act):
+    """Row tiles of padding are dealt out after the others: same results as without counts, empty groups and more groups than
+    the counted order takes included."""
+    from memarch_b200.ops.moe import expert_ffn
+    g = torch.Generator(device="cuda").manual_seed(E)
+    d, H = 64, 136
+    cnt = (torch.arange(E, device="cuda") * 37 % (C + 1) if counts == "mixed" else torch.tensor(counts, device="cuda")).int()
+    live = (torch.arange(C, device="cuda")[None] < cnt[:, None])[..., None]
+    x = torch.randn(E, C, d, device="cuda", generator=g).bfloat16() * live
+    up = (torch.randn(E, d, 2 * H if act == "swiglu" else H, device="cuda", generator=g) * d ** -0.5).bfloat16()
+    down = (torch.randn(E, H, d, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    gy = torch.randn(E, C, d, device="cuda", generator=g).bfloat16() * live
+    res = []
+    for c in (cnt, None):
+        t = [v.clone().requires_grad_() for v in (x, up, down)]
+        y = expert_ffn(*t, act, counts=c)
+        y.backward(gy)
+        res.append([y] + [v.grad for v in t])
+    for a, b in zip(*res):
+        assert torch.equal(a, b) or _rel(a, b) < 1e-5
