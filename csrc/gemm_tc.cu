@@ -473,8 +473,9 @@ __device__ __forceinline__ void epi_send(const GemmParams& p, const EpiRing& rin
 struct AuxPipe {
   uint64_t* bars;          // this warp's mbarriers, one per slot
   int slots, nb;           // nb staging tiles per chunk (1: relu² backward, 2: SwiGLU backward), slots = tiles / nb
-  uint32_t issued, consumed;
-  int pf_t, pf_hc;         // cursor of the next chunk to fetch: tile, half * 4 + chunk
+  uint32_t issued, consumed, freed;   // chunks asked for, used, and whose slot may be loaded again
+  int pf_t, pf_hc;         // cursor of the next chunk to fetch: tile, half * 4 + chunk (-1: the tile's place is not known yet)
+  int pf_row, pf_col, pf_g;
   const CUtensorMap* tm;
   const int* cum;          // see tile_coords
   int rank, q, npairs, total, mh;
@@ -494,32 +495,31 @@ __device__ __forceinline__ int group_kblocks(const GemmParams& p, int g);
 // Issue loads until `slots` chunks are in flight or the tile list ends.  Walks tiles and chunks exactly as the
 // epilogue does (padding tiles and chunks past the last column are skipped).  Lane 0 only.
 __device__ __forceinline__ void aux_issue(const GemmParams& p, AuxPipe& a, uint8_t* ring_base) {
-  while (a.issued - a.consumed < (uint32_t)a.slots && a.pf_t < a.total) {
-    int g, mt, nt;
-    tile_coords(a.pf_t, p, g, mt, nt, a.cum);
-    const int seg = mt / p.tiles_per_seg;
-    const int mseg0 = (mt - seg * p.tiles_per_seg) * 256 * a.mh;
-    const bool skip_tile = seg * p.seg_M + mseg0 >= group_rows(p, g) || group_kblocks(p, g) == 0;
-    const int h = a.pf_hc >> 2, c = a.pf_hc & 3;
-    const int col0 = nt * p.bn + c * 64;
-    if (skip_tile || col0 >= p.N) {                     // next half / tile
-      if (skip_tile || h + 1 >= a.mh) { a.pf_t += a.npairs; a.pf_hc = 0; }
-      else a.pf_hc = (h + 1) << 2;
-      continue;
+  while (a.issued - a.freed < (uint32_t)a.slots && a.pf_t < a.total) {
+    if (a.pf_hc < 0) {
+      int g, mt, nt;
+      tile_coords(a.pf_t, p, g, mt, nt, a.cum);
+      const int seg = mt / p.tiles_per_seg;
+      const int mseg0 = (mt - seg * p.tiles_per_seg) * 256 * a.mh;
+      if (seg * p.seg_M + mseg0 >= group_rows(p, g) || group_kblocks(p, g) == 0) { a.pf_t += a.npairs; continue; }
+      a.pf_row = seg * p.seg_M + mseg0 + a.rank * BM + a.q * 32;
+      a.pf_col = nt * p.bn;
+      a.pf_g = g;
+      a.pf_hc = 0;
     }
-    const int row0 = seg * p.seg_M + mseg0 + h * 256 + a.rank * BM + a.q * 32;
+    const int h = a.pf_hc >> 2, c = a.pf_hc & 3;
+    const int col0 = a.pf_col + c * 64;
+    const bool last = c == (p.bn >> 6) - 1 || col0 + 64 >= p.N;     // of this half
+    const int row0 = a.pf_row + h * 256;
     const int slot = a.issued % a.slots;
     uint8_t* b = ring_base + slot * a.nb * EPI_BUF_BYTES;
     mbar_expect_tx(&a.bars[slot], a.nb * EPI_BUF_BYTES);
-    tma_load_3d_local(b, a.tm, &a.bars[slot], col0, row0, g);
-    if (a.nb == 2) tma_load_3d_local(b + EPI_BUF_BYTES, a.tm, &a.bars[slot], p.N + col0, row0, g);
+    tma_load_3d_local(b, a.tm, &a.bars[slot], col0, row0, a.pf_g);
+    if (a.nb == 2) tma_load_3d_local(b + EPI_BUF_BYTES, a.tm, &a.bars[slot], p.N + col0, row0, a.pf_g);
     ++a.issued;
-    if (c == (p.bn >> 6) - 1) {
-      if (h + 1 >= a.mh) { a.pf_t += a.npairs; a.pf_hc = 0; }
-      else a.pf_hc = (h + 1) << 2;
-    } else {
-      ++a.pf_hc;
-    }
+    if (!last) ++a.pf_hc;
+    else if (h + 1 < a.mh) a.pf_hc = (h + 1) << 2;
+    else { a.pf_t += a.npairs; a.pf_hc = -1; }
   }
 }
 
@@ -723,25 +723,32 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
         coop_load(b1, ab + static_cast<long long>(p.N) * 2, static_cast<long long>(p.ldaux) * 2, rows_valid, pv, lane);
         __syncwarp();
       }
+      // All loads of half a chunk go out before its first store: one epilogue warp per scheduler has nothing else to hide
+      // the round trip to shared memory with, and a store in between holds the next load back.
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        uint4* pg = stage_piece(b0, lane, j);
-        uint4* pu = stage_piece(b1, lane, j);
-        const uint4 ug = *pg, uu = *pu;
-        const uint32_t wg[4] = {ug.x, ug.y, ug.z, ug.w}, wu[4] = {uu.x, uu.y, uu.z, uu.w};
-        uint32_t og[4], ou[4];
+      for (int hf = 0; hf < 2; ++hf) {
+        uint4 ug[4], uu[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 gg = unpack_bf16(wg[q]), uv = unpack_bf16(wu[q]);
-          const float d0 = __uint_as_float(r[8 * j + 2 * q]), d1 = __uint_as_float(r[8 * j + 2 * q + 1]);
-          // sigmoid through the hardware tanh (one special-function instruction, no division): with one epilogue
-          // warp per scheduler the dependent chain of exp + IEEE division per element was what bound this epilogue
-          const float s0 = fmaf(tanh_approx(0.5f * gg.x), 0.5f, 0.5f), s1 = fmaf(tanh_approx(0.5f * gg.y), 0.5f, 0.5f);
-          og[q] = pack_bf16(d0 * uv.x * s0 * (1.f + gg.x * (1.f - s0)), d1 * uv.y * s1 * (1.f + gg.y * (1.f - s1)));
-          ou[q] = pack_bf16(d0 * gg.x * s0, d1 * gg.y * s1);
+        for (int j = 0; j < 4; ++j) { ug[j] = *stage_piece(b0, lane, 4 * hf + j); uu[j] = *stage_piece(b1, lane, 4 * hf + j); }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t wg[4] = {ug[j].x, ug[j].y, ug[j].z, ug[j].w}, wu[4] = {uu[j].x, uu[j].y, uu[j].z, uu[j].w};
+          uint32_t og[4], ou[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 gg = unpack_bf16(wg[q]), uv = unpack_bf16(wu[q]);
+            const float d0 = __uint_as_float(r[32 * hf + 8 * j + 2 * q]), d1 = __uint_as_float(r[32 * hf + 8 * j + 2 * q + 1]);
+            // sigmoid through the hardware tanh (one special-function instruction, no division): with one epilogue
+            // warp per scheduler the dependent chain of exp + IEEE division per element was what bound this epilogue
+            const float s0 = fmaf(tanh_approx(0.5f * gg.x), 0.5f, 0.5f), s1 = fmaf(tanh_approx(0.5f * gg.y), 0.5f, 0.5f);
+            og[q] = pack_bf16(d0 * uv.x * s0 * (1.f + gg.x * (1.f - s0)), d1 * uv.y * s1 * (1.f + gg.y * (1.f - s1)));
+            ou[q] = pack_bf16(d0 * gg.x * s0, d1 * gg.y * s1);
+          }
+          ug[j] = make_uint4(og[0], og[1], og[2], og[3]);
+          uu[j] = make_uint4(ou[0], ou[1], ou[2], ou[3]);
         }
-        *pg = make_uint4(og[0], og[1], og[2], og[3]);
-        *pu = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { *stage_piece(b0, lane, 4 * hf + j) = ug[j]; *stage_piece(b1, lane, 4 * hf + j) = uu[j]; }
       }
     } else if (p.epi == EPI_DRELU2) {
       const char* ab = reinterpret_cast<const char*>(p.aux) + (g * p.aux_gs + static_cast<long long>(row0) * p.ldaux + col0) * 2;
@@ -749,16 +756,22 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
         coop_load(b0, ab, static_cast<long long>(p.ldaux) * 2, rows_valid, min(8, (p.N - col0 + 7) >> 3), lane);
         __syncwarp();
       }
+      uint4 u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] = *stage_piece(b0, lane, j);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        uint4* pp = stage_piece(b0, lane, j);
-        const uint4 u = *pp;
-        const float2 f0 = unpack_bf16(u.x), f1 = unpack_bf16(u.y), f2 = unpack_bf16(u.z), f3 = unpack_bf16(u.w);
-        *pp = make_uint4(pack_bf16(__uint_as_float(r[8 * j + 0]) * 2.f * fmaxf(f0.x, 0.f), __uint_as_float(r[8 * j + 1]) * 2.f * fmaxf(f0.y, 0.f)),
-                         pack_bf16(__uint_as_float(r[8 * j + 2]) * 2.f * fmaxf(f1.x, 0.f), __uint_as_float(r[8 * j + 3]) * 2.f * fmaxf(f1.y, 0.f)),
-                         pack_bf16(__uint_as_float(r[8 * j + 4]) * 2.f * fmaxf(f2.x, 0.f), __uint_as_float(r[8 * j + 5]) * 2.f * fmaxf(f2.y, 0.f)),
-                         pack_bf16(__uint_as_float(r[8 * j + 6]) * 2.f * fmaxf(f3.x, 0.f), __uint_as_float(r[8 * j + 7]) * 2.f * fmaxf(f3.y, 0.f)));
+        const uint32_t w[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+        uint32_t o4[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = unpack_bf16(w[q]);
+          o4[q] = pack_bf16(__uint_as_float(r[8 * j + 2 * q]) * 2.f * fmaxf(f.x, 0.f), __uint_as_float(r[8 * j + 2 * q + 1]) * 2.f * fmaxf(f.y, 0.f));
+        }
+        u[j] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *stage_piece(b0, lane, j) = u[j];
     } else {
       float sc = 1.f;
       if (p.epi == EPI_ROWSCALE) sc = row0_l + lane < p.seg_M ? reinterpret_cast<const float*>(p.aux)[g * p.aux_gs + row] : 0.f;
@@ -779,7 +792,10 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
       ++aux->consumed;
       __syncwarp();                               // direct stores: every lane has read the slot
       if (lane == 0) {
-        bulk_wait_read<0>();                      // TMA stores have read it too: it may take the chunk `slots` ahead
+        // A slot whose TMA stores have read it takes the next chunk.  With three slots or more that is the one before this:
+        // its stores are done by now, those of this chunk would be waited for.
+        if (aux->slots >= 3) { bulk_wait_read<1>(); aux->freed = aux->consumed - 1; }
+        else { bulk_wait_read<0>(); aux->freed = aux->consumed; }
         fence_async_smem();
         aux_issue(p, *aux, ring.base);
       }
@@ -1031,8 +1047,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
     aux.bars = auxbars + q * 4;
     aux.nb = ring.nb;
     aux.slots = EPI_NBUF / ring.nb;
-    aux.issued = aux.consumed = 0;
-    aux.pf_t = pair; aux.pf_hc = 0; aux.cum = cum;
+    aux.issued = aux.consumed = aux.freed = 0;
+    aux.pf_t = pair; aux.pf_hc = -1; aux.cum = cum;
     aux.tm = &tmX;
     aux.rank = (int)rank; aux.q = q; aux.npairs = npairs; aux.total = total; aux.mh = MH;
     if (aux.on && lane == 0) aux_issue(p, aux, ring.base);
