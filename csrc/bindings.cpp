@@ -33,6 +33,7 @@ torch::Tensor resid_add(torch::Tensor x, torch::Tensor y);
 torch::Tensor rope_merge_bwd(torch::Tensor dq, torch::Tensor dk, torch::Tensor dv, torch::Tensor cos, torch::Tensor sin, bool half);
 void ce_rows(torch::Tensor logits, torch::Tensor y, torch::Tensor loss, c10::optional<torch::Tensor> gate,
              c10::optional<torch::Tensor> hit, c10::optional<torch::Tensor> dg);
+torch::Tensor scale_by(torch::Tensor x, torch::Tensor scale, bool out_bf16);
 torch::Tensor gather_rows(torch::Tensor src, torch::Tensor table, c10::optional<torch::Tensor> scale);
 torch::Tensor gather_sum_rows(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w, int64_t N);
 torch::Tensor dequant_i8(torch::Tensor q, torch::Tensor scale);
@@ -128,6 +129,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("resid_add", &mb::resid_add);
   m.def("rope_merge_bwd", &mb::rope_merge_bwd);
   m.def("ce_rows", &mb::ce_rows);
+  m.def("scale_by", &mb::scale_by);
   m.def("gather_rows", &mb::gather_rows);
   m.def("gather_sum_rows", &mb::gather_sum_rows);
   m.def("row_dot", &mb::row_dot);

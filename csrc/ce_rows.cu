@@ -102,4 +102,44 @@ void ce_rows_launch(void* logits, const long long* y, float* loss, const float* 
   ce_rows_kernel<<<n, CE_THREADS, 0, stream>>>(reinterpret_cast<bf16*>(logits), y, loss, gate, hit, dg, stride, V);
 }
 
+// out = x * *scale: the gradients of the forward pass times the one that arrives at the loss.  A plain copy in its traffic;
+// four pieces of four elements per thread in flight.  (50 304 x 2064) fp32: 153 us
+// (127 at the copy rate); the broadcast multiplication of PyTorch took 318.
+template <bool XB, bool OB>
+__global__ void __launch_bounds__(256) scale_kernel(const void* __restrict__ x, const float* __restrict__ scale, void* __restrict__ out, long long n4) {
+  const float f = *scale;
+  const long long step = (long long)gridDim.x * 256;
+  for (long long i0 = blockIdx.x * 256ll + threadIdx.x; i0 < n4; i0 += 4 * step) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long i = i0 + k * step;
+      if (i >= n4) continue;
+      if (XB) {
+        const uint2 u = reinterpret_cast<const uint2*>(x)[i];
+        const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
+        v[k] = make_float4(a.x, a.y, b.x, b.y);
+      } else {
+        v[k] = reinterpret_cast<const float4*>(x)[i];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long i = i0 + k * step;
+      if (i >= n4) continue;
+      if (OB) reinterpret_cast<uint2*>(out)[i] = make_uint2(pack_bf16(v[k].x * f, v[k].y * f), pack_bf16(v[k].z * f, v[k].w * f));
+      else reinterpret_cast<float4*>(out)[i] = make_float4(v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f);
+    }
+  }
+}
+void scale_launch(const void* x, int x_bf16, const float* scale, void* out, int out_bf16, long long n, cudaStream_t stream) {
+  const long long n4 = n / 4, want = (n4 + 1023) / 1024;
+  const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
+  if (!grid) return;
+  if (x_bf16 && out_bf16) scale_kernel<true, true><<<grid, 256, 0, stream>>>(x, scale, out, n4);
+  else if (x_bf16) scale_kernel<true, false><<<grid, 256, 0, stream>>>(x, scale, out, n4);
+  else if (out_bf16) scale_kernel<false, true><<<grid, 256, 0, stream>>>(x, scale, out, n4);
+  else scale_kernel<false, false><<<grid, 256, 0, stream>>>(x, scale, out, n4);
+}
+
 }  // namespace mb

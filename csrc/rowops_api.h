@@ -29,5 +29,7 @@ void rmsnorm_bwd_launch(const NormArgs& a);
 // logits (n, V) bf16 with row pitch `stride`: overwritten with d(loss)/d(logits); see ce_rows.cu
 void ce_rows_launch(void* logits, const long long* y, float* loss, const float* gate, const float* hit, float* dg, long long stride,
                     int n, int V, cudaStream_t stream);
+// out = x * *scale over n elements (n % 4 == 0, 16-byte aligned arrays), fp32 arithmetic
+void scale_launch(const void* x, int x_bf16, const float* scale, void* out, int out_bf16, long long n, cudaStream_t stream);
 
 }  // namespace mb

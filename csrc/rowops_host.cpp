@@ -92,4 +92,15 @@ void ce_rows(torch::Tensor logits, torch::Tensor y, torch::Tensor loss, c10::opt
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
+// x * scale (one fp32 element on the device) in bf16 or fp32
+torch::Tensor scale_by(torch::Tensor x, torch::Tensor scale, bool out_bf16) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.is_contiguous() && float_or_bf16(x) && x.numel() % 4 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
+              scale.scalar_type() == torch::kFloat32 && scale.numel() == 1 && scale.device() == x.device(), "scale_by: bf16 or fp32 by one fp32 element");
+  auto out = torch::empty(x.sizes(), x.options().dtype(out_bf16 ? torch::kBFloat16 : torch::kFloat32));
+  scale_launch(x.data_ptr(), is_bf16(x), scale.data_ptr<float>(), out.data_ptr(), out_bf16, x.numel(), at::cuda::getCurrentCUDAStream());
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  return out;
+}
+
 }  // namespace mb

@@ -24,7 +24,7 @@ def _ce_forward_cuda(h, w, y, gate, hit, cand, cval, chunk):
     hd = h.to(torch.bfloat16).contiguous()
     wd = w.to(torch.bfloat16).contiguous()
     gh = torch.empty_like(hd)
-    gw = torch.zeros(V, d, device=h.device, dtype=torch.float32)
+    gw = torch.empty(V, d, device=h.device, dtype=torch.float32)
     loss = torch.empty(N, device=h.device, dtype=torch.float32)
     dg = torch.empty(N, device=h.device, dtype=torch.float32) if gate is not None else None
     dcv = torch.empty(cval.shape, device=h.device, dtype=torch.float32) if cval is not None else None
@@ -46,8 +46,18 @@ def _ce_forward_cuda(h, w, y, gate, hit, cand, cval, chunk):
         if dcv is not None:
             dcv[i:i + n] = lg.gather(-1, cand[i:i + n]).float()
         gemm(lg, wd, b_mn=True, out=gh[i:i + n])                            # dh = G · W
-        gemm(lg, hc, a_mn=True, b_mn=True, out=gw, out_dtype=torch.float32, accumulate=True)   # dW += Gᵀ · h
+        gemm(lg, hc, a_mn=True, b_mn=True, out=gw, out_dtype=torch.float32, accumulate=i > 0)   # dW += Gᵀ · h
     return loss.sum(), gh, gw, dg, dcv
+
+
+def _scaled(x, go, dtype):
+    """(x * go) in `dtype`; a gradient that is differentiated or batched itself stays on the PyTorch ops."""
+    if (_ext.use_cuda(x) and not (torch.is_grad_enabled() and go.requires_grad) and not torch._C._functorch.is_batchedtensor(go)
+            and go.is_cuda and go.dtype == torch.float32 and x.dtype in (torch.bfloat16, torch.float32)
+            and dtype in (torch.bfloat16, torch.float32) and x.numel() % 4 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0):
+        _ext.count()
+        return _ext.C().scale_by(x, go, dtype == torch.bfloat16)
+    return (x * go).to(dtype)
 
 
 class _LinearCE(torch.autograd.Function):
@@ -67,7 +77,7 @@ class _LinearCE(torch.autograd.Function):
     def backward(ctx, go):
         gh, gw, dg, dcv = ctx.saved_tensors
         hdt, wdt, has_g, gdt, has_c, cdt = ctx.meta
-        return ((gh * go).to(hdt), (gw * go).to(wdt), None,
+        return (_scaled(gh, go, hdt), _scaled(gw, go, wdt), None,
                 (dg * go).to(gdt) if has_g else None, None, None,
                 (dcv * go).to(cdt) if has_c else None, None, None)
 

@@ -432,3 +432,26 @@ def test_expert_ffn_counts_order(E, C, counts, act):
         res.append([y] + [v.grad for v in t])
     for a, b in zip(*res):
         assert torch.equal(a, b) or _rel(a, b) < 1e-5
+
+
+# ------------------------------------------------------------------------------------------------ head
+@pytest.mark.parametrize("N,V,d,chunk", [(1, 16, 16, 4096), (300, 1000, 24, 128), (513, 264, 136, 512), (40, 104, 64, 7)])
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+def test_linear_ce_chunks(N, V, d, chunk, wdt):
+    """Chunks of any length, the first one writes the weight gradient; scaled, repeated and differentiable upstream gradients."""
+    from memarch_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N)
+    h = torch.randn(N, d, device="cuda", generator=g).bfloat16().requires_grad_()
+    w = (torch.randn(V, d, device="cuda", generator=g) * d ** -0.5).to(wdt).requires_grad_()
+    y = torch.randint(0, V, (N,), device="cuda", generator=g)
+    loss = ops.linear_ce(h, w, y, chunk=chunk) * 0.37
+    hd, wd = h.detach().double().requires_grad_(), w.detach().bfloat16().double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(hd @ wd.t(), y, reduction="sum") * 0.37
+    gh, gw = torch.autograd.grad(want, (hd, wd))
+    assert abs(loss.item() - want.item()) < 2e-3 * max(1.0, abs(want.item()))
+    for _ in range(2):
+        a, b = torch.autograd.grad(loss, (h, w), retain_graph=True)
+        # bf16 logits (2^-9 of values up to 4) and bf16 gradients of them
+        assert a.dtype == h.dtype and b.dtype == wdt and _rel(a, gh) < 2e-2 and _rel(b, gw) < 2e-2
+    a2, = torch.autograd.grad(loss, (h,), create_graph=True)
+    assert torch.allclose(a2, a, rtol=1e-2, atol=1e-6)
