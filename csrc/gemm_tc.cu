@@ -803,6 +803,94 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
   }
 }
 
+enum { ACT_NONE = 0, ACT_SWIGLU = 1, ACT_RELU2 = 2 };
+// The activation-backward epilogues with two warps per 32 TMEM lanes, each taking 32 of a chunk's 64 columns: one warp per
+// scheduler could not hide its own chain of shared-memory and special-function latencies.  Both wait for the chunk's
+// pre-activations and write their results over them; the second reports on `done` (a barrier per slot), the first sends
+// the tile and refills the slot before.  All waits are bounded and none is for a warp that may have given up unseen.
+// Us, (M, N, K), one warp -> two, SwiGLU / relu2: (32 768, 4096, 1024) 358 -> 314 / 264 -> 237, plain product 211; (8192, 3072, 768)
+// 85 -> 65 / 60 -> 47, plain 40; (4096, 2048, 512) 31 -> 25 / 23 -> 19, plain 19.  (32 768, 8192, 2048) is bound by power: 1050 / 900.
+template <int ACT>
+__device__ __forceinline__ void epilogue_act(const GemmParams& p, const CUtensorMap* tmO, const CUtensorMap* tmO2, int og, int row0, int nt,
+                                             uint32_t taddr, uint8_t* ring_base, int lane, int half, AuxPipe& aux, uint64_t* done,
+                                             volatile int* abort_flag) {
+#pragma unroll 1
+  for (int c = 0; c < p.bn / 64; ++c) {
+    const int col0 = nt * p.bn + c * 64;
+    if (col0 >= p.N) break;
+    uint32_t r[32];
+    tmem_ld32(taddr + c * 64 + half * 32, r);
+    const int slot = aux.consumed % aux.slots;
+    const uint32_t phase = (aux.consumed / aux.slots) & 1;
+    if (!mbar_wait(&aux.bars[slot], phase, abort_flag)) {
+      if (lane == 0) { atomicCAS(p.status, 0, ST_WAIT_FULL); *abort_flag = 1; }
+      tmem_ld_wait();
+      return;
+    }
+    uint8_t* b0 = ring_base + slot * aux.nb * EPI_BUF_BYTES;
+    uint8_t* b1 = b0 + EPI_BUF_BYTES;
+    uint4 ug[4], uu[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      ug[j] = *stage_piece(b0, lane, 4 * half + j);
+      if (ACT == ACT_SWIGLU) uu[j] = *stage_piece(b1, lane, 4 * half + j);
+    }
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t wg[4] = {ug[j].x, ug[j].y, ug[j].z, ug[j].w};
+      uint32_t o0[4], o1[4];
+      if (ACT == ACT_SWIGLU) {
+        // acc = dh; dg = dh * u * s * (1 + g * (1 - s)), du = dh * g * s with s = sigmoid(g) through the hardware tanh
+        const uint32_t wu[4] = {uu[j].x, uu[j].y, uu[j].z, uu[j].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 gg = unpack_bf16(wg[q]), uv = unpack_bf16(wu[q]);
+          const float d0 = __uint_as_float(r[8 * j + 2 * q]), d1 = __uint_as_float(r[8 * j + 2 * q + 1]);
+          const float s0 = fmaf(tanh_approx(0.5f * gg.x), 0.5f, 0.5f), s1 = fmaf(tanh_approx(0.5f * gg.y), 0.5f, 0.5f);
+          o0[q] = pack_bf16(d0 * uv.x * s0 * (1.f + gg.x * (1.f - s0)), d1 * uv.y * s1 * (1.f + gg.y * (1.f - s1)));
+          o1[q] = pack_bf16(d0 * gg.x * s0, d1 * gg.y * s1);
+        }
+        uu[j] = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = unpack_bf16(wg[q]);
+          o0[q] = pack_bf16(__uint_as_float(r[8 * j + 2 * q]) * 2.f * fmaxf(f.x, 0.f), __uint_as_float(r[8 * j + 2 * q + 1]) * 2.f * fmaxf(f.y, 0.f));
+        }
+      }
+      ug[j] = make_uint4(o0[0], o0[1], o0[2], o0[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      *stage_piece(b0, lane, 4 * half + j) = ug[j];
+      if (ACT == ACT_SWIGLU) *stage_piece(b1, lane, 4 * half + j) = uu[j];
+    }
+    fence_async_smem();
+    __syncwarp();
+    ++aux.consumed;
+    if (lane == 0) {
+      if (half) {
+        mbar_arrive(&done[slot]);
+      } else if (!mbar_wait(&done[slot], phase, abort_flag)) {
+        atomicCAS(p.status, 0, ST_WAIT_FULL); *abort_flag = 1;
+      } else {
+        if (!(p.dbg & DBG_NO_STORE)) {
+          tma_store_3d(tmO, b0, col0, row0, og);
+          if (ACT == ACT_SWIGLU) tma_store_3d(tmO2, b1, col0, row0, og);
+        }
+        bulk_commit();
+        // a slot whose stores have read it takes the next chunk: the one before this, whose stores are done by now
+        bulk_wait_read<1>();
+        aux.freed = aux.consumed - 1;
+        fence_async_smem();
+        aux_issue(p, aux, ring_base);
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // extent of group g under count_mode (rows for mode 1, contraction length for mode 2), else the full extent
 __device__ __forceinline__ int group_rows(const GemmParams& p, int g) {
   return p.count_mode == 1 ? min(p.M, __ldg(p.counts + g)) : p.M;
@@ -826,22 +914,23 @@ __device__ __forceinline__ int split_start(const GemmParams& p, int t, int& num_
 // shared-memory traffic, which on a power-capped part is clock) - 4 stages of 48 KB; the two 256-column accumulators
 // fill TMEM, so the epilogue is only half hidden (the MMAs of the next tile's first block start as soon as the
 // first half is drained): worth it when the contraction is long.
-// DEEP (256-row tiles only): one operand stage less and six staging tiles per epilogue warp instead of four, for the
-// SwiGLU-backward epilogue, which moves two tiles in and two out per 64 accumulator columns and needs three chunks of
-// pre-activations in flight per warp to keep HBM busy.
-template <int MH, bool DEEP = false> struct PairCfg {
-  static constexpr int STAGES = (MH == 2 || DEEP) ? 4 : 5;
-  static constexpr int NBUF = MH == 2 ? 2 : (DEEP ? 6 : 4);
+// ACT (256-row tiles only): the epilogues that multiply by the activation's derivative, ACT_SWIGLU and ACT_RELU2, with eight
+// epilogue warps (see epilogue_act).  SwiGLU moves two tiles in and two out per 64 accumulator columns and needs three chunks
+// of pre-activations in flight to keep HBM busy: one operand stage less, six staging tiles instead of four.
+template <int MH, int ACT = ACT_NONE> struct PairCfg {
+  static constexpr int THREADS = ACT ? 320 : GEMM_THREADS;
+  static constexpr int STAGES = (MH == 2 || ACT == ACT_SWIGLU) ? 4 : 5;
+  static constexpr int NBUF = MH == 2 ? 2 : (ACT == ACT_SWIGLU ? 6 : 4);
   static constexpr int STAGE_BYTES = MH * A_BYTES + BH_BYTES;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 4 * NBUF * EPI_BUF_BYTES + 1024 + 256;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 4 * NBUF * EPI_BUF_BYTES + 1024 + 384;
 };
 
-template <bool A_MN, bool B_MN, int MH, bool DEEP = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+template <bool A_MN, bool B_MN, int MH, int ACT = ACT_NONE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<MH, ACT>::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmO2,
                 const __grid_constant__ CUtensorMap tmX, const GemmParams p) {
-  constexpr int STAGES3 = PairCfg<MH, DEEP>::STAGES, EPI_NBUF = PairCfg<MH, DEEP>::NBUF, STAGE_B = PairCfg<MH, DEEP>::STAGE_BYTES;
+  constexpr int STAGES3 = PairCfg<MH, ACT>::STAGES, EPI_NBUF = PairCfg<MH, ACT>::NBUF, STAGE_B = PairCfg<MH, ACT>::STAGE_BYTES;
   constexpr int TILE_M = 256 * MH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -852,7 +941,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* auxbars = full + 16;              // 4 epilogue warps x 4 slots of the aux prefetch queue (bytes 128..255)
+  uint64_t* auxbars = full + 16;              // 4 lane quarters x 4 slots of the aux prefetch queue (bytes 128..255)
+  uint64_t* halfbars = full + 32;             // the same slots: the second warp's half is written (bytes 256..383)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -864,14 +954,14 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES3; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], ACT ? 16 : 8); }
     *abort_flag = 0;
     mbar_fence_init();
     for (int i = 0; i < p.n_seg; ++i) tma_prefetch_desc(&tmAs.m[i]);
     tma_prefetch_desc(&tmB);
     if (p.store_tma) { tma_prefetch_desc(&tmO); if (p.out2 || p.epi == EPI_DSWIGLU) tma_prefetch_desc(&tmO2); }
     if (p.aux_tma) {
-      for (int i = 0; i < 16; ++i) mbar_init(&auxbars[i], 1);
+      for (int i = 0; i < 16; ++i) { mbar_init(&auxbars[i], 1); mbar_init(&halfbars[i], 1); }
       mbar_fence_init();
       tma_prefetch_desc(&tmX);
     }
@@ -1051,7 +1141,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
     aux.pf_t = pair; aux.pf_hc = -1; aux.cum = cum;
     aux.tm = &tmX;
     aux.rank = (int)rank; aux.q = q; aux.npairs = npairs; aux.total = total; aux.mh = MH;
-    if (aux.on && lane == 0) aux_issue(p, aux, ring.base);
+    [[maybe_unused]] const int half = (warp - 2) >> 2;            // ACT: which 32 of 64 columns
+    if (aux.on && lane == 0 && half == 0) aux_issue(p, aux, ring.base);
     for (int t = pair; t < total && ok; t += npairs) {
       int g, mt, nt;
       tile_coords(t, p, g, mt, nt, cum);
@@ -1070,7 +1161,12 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
         const int row0_l = mseg0 + h * 256 + (int)rank * BM + q * 32;
         const int row0 = seg * p.seg_M + row0_l;
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + (MH == 1 ? acc * BN : h * BN);
-        epilogue_tile3(p, &tmO, &tmO2, g, seg, row0, row0_l, nt, taddr, ring, lane, zero_tile, &aux, abort_flag);
+        bool drained = false;
+        if constexpr (ACT != ACT_NONE) {
+          drained = !zero_tile || half != 0;
+          if (!zero_tile) epilogue_act<ACT>(p, &tmO, &tmO2, g + p.out_g_off, row0, nt, taddr, ring.base, lane, half, aux, halfbars + q * 4, abort_flag);
+        }
+        if (!drained) epilogue_tile3(p, &tmO, &tmO2, g, seg, row0, row0_l, nt, taddr, ring, lane, zero_tile, &aux, abort_flag);
         if (*abort_flag) { ok = false; break; }
         if (!zero_tile) {
           tc_fence_before();
@@ -1085,7 +1181,7 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
       }
     }
     if (ring.tma && lane == 0) bulk_wait_read<0>();          // staged tiles must be read before the CTA's smem goes away
-    if (aux.on && lane == 0 && !ok) {
+    if (aux.on && lane == 0 && half == 0 && !ok) {
       // gave up with prefetches in flight: let them land (bounded) before the CTA's shared memory goes away
       for (uint32_t i = aux.consumed; i < aux.issued; ++i)
         for (uint32_t spin = 0; spin < MB_SPIN_LIMIT; ++spin)
@@ -1241,8 +1337,6 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
   if (grid <= 0) return;
   const bool v3 = pair;
   check(v3 || p.count_mode == 0, "gemm: per-group extents need the pair kernel (>= 256 rows)");
-  const bool deep = v3 && !tall && p.epi == EPI_DSWIGLU && !a_mn;
-  const int smem_bytes = v3 ? (tall ? PairCfg<2>::SMEM : deep ? PairCfg<1, true>::SMEM : PairCfg<1>::SMEM) : SMEM_BYTES;
   CUtensorMap tmO = tmB, tmO2 = tmB;
   if (v3) {
     p.dbg = g_dbg;
@@ -1276,8 +1370,12 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
       p.aux_tma = 1;
     }
   }
+  // eight epilogue warps where the pre-activations come and the results leave by TMA
+  const int act = v3 && !tall && !a_mn && p.aux_tma && p.store_tma ? (p.epi == EPI_DSWIGLU ? ACT_SWIGLU : p.epi == EPI_DRELU2 ? ACT_RELU2 : ACT_NONE) : ACT_NONE;
+  const int smem_bytes = !v3 ? SMEM_BYTES : tall ? PairCfg<2>::SMEM : act == ACT_SWIGLU ? PairCfg<1, ACT_SWIGLU>::SMEM : PairCfg<1>::SMEM;
+  const int threads = act ? PairCfg<1, ACT_SWIGLU>::THREADS : GEMM_THREADS;
   auto launch = [&](auto kern, int id) {
-    static bool attr_set[16][16] = {};
+    static bool attr_set[16][20] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 15][id]) {
@@ -1286,7 +1384,7 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
       attr_set[dev & 15][id] = true;
     }
     if constexpr (std::is_invocable_v<decltype(kern), TmapSet, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams>)
-      kern<<<grid, GEMM_THREADS, smem_bytes, stream>>>(tmAs, tmB, tmO, tmO2, tmX, p);
+      kern<<<grid, threads, smem_bytes, stream>>>(tmAs, tmB, tmO, tmO2, tmX, p);
     else
       kern<<<grid, GEMM_THREADS, smem_bytes, stream>>>(tmAs, tmB, p);
   };
@@ -1296,9 +1394,12 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
     else if (!a_mn && b_mn) launch(gemm_pair_kernel<false, true, 2>, 12 + id);
     else if (a_mn && !b_mn) launch(gemm_pair_kernel<true, false, 2>, 12 + id);
     else launch(gemm_pair_kernel<true, true, 2>, 12 + id);
-  } else if (deep) {
-    if (!b_mn) launch(gemm_pair_kernel<false, false, 1, true>, 4);
-    else launch(gemm_pair_kernel<false, true, 1, true>, 5);
+  } else if (act == ACT_SWIGLU) {
+    if (!b_mn) launch(gemm_pair_kernel<false, false, 1, ACT_SWIGLU>, 4);
+    else launch(gemm_pair_kernel<false, true, 1, ACT_SWIGLU>, 5);
+  } else if (act == ACT_RELU2) {
+    if (!b_mn) launch(gemm_pair_kernel<false, false, 1, ACT_RELU2>, 16);
+    else launch(gemm_pair_kernel<false, true, 1, ACT_RELU2>, 17);
   } else if (v3) {
     if (!a_mn && !b_mn) launch(gemm_pair_kernel<false, false, 1>, 8 + id);
     else if (!a_mn && b_mn) launch(gemm_pair_kernel<false, true, 1>, 8 + id);

@@ -281,9 +281,8 @@ class _LinearAct(torch.autograd.Function):
 
 
 # SwiGLU backward inside the input-gradient GEMM's epilogue (2H pre-activations in, 2H gradients out per H accumulator
-# columns): 0.97 ms at (32768, 8192, 2048) against 0.74 + 0.43 ms for the plain GEMM plus the elementwise kernel.  (With
-# exp + IEEE division for the sigmoid it took 1.6 ms - one epilogue warp per scheduler cannot hide that dependent
-# chain; the hardware tanh made it pay.)  relu² backward: 0.80 ms fused against 0.74 + 0.25 ms.
+# columns), (M, H, K) = (32 768, 4096, 1024): 0.31 ms against 0.21 for the plain product and 0.21 for the element-wise
+# kernel; (32 768, 8192, 2048): 1.05 ms against 0.77 + 0.43.
 FUSE_DSWIGLU = True
 
 

@@ -434,6 +434,26 @@ def test_expert_ffn_counts_order(E, C, counts, act):
         assert torch.equal(a, b) or _rel(a, b) < 1e-5
 
 
+# ------------------------------------------------------------------------------------------------ activation backward
+@pytest.mark.parametrize("M,H,K", [(256, 8, 64), (300, 72, 64), (513, 200, 136), (1000, 264, 2048), (4000, 1032, 72), (9473, 512, 64)])
+@pytest.mark.parametrize("b_mn", [True, False])
+def test_gemm_activation_backward(M, H, K, b_mn):
+    """Two warps per 32 accumulator rows: ragged rows and columns, narrow and wide tiles, more tiles than CTA pairs."""
+    from memarch_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(M)
+    dy, w = torch.randn(M, K, device="cuda", generator=g).bfloat16(), (torch.randn(H, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    pre = torch.randn(M, 2 * H, device="cuda", generator=g).bfloat16()
+    dh = dy.double() @ w.double().t()
+    wm = w.t().contiguous() if b_mn else w
+    gate, up = pre.double().chunk(2, 1)
+    s = gate.sigmoid()
+    want = torch.cat([dh * up * s * (1 + gate * (1 - s)), dh * gate * s], 1)
+    # one rounding to bf16 (2^-9) and the hardware tanh (2^-11 of the sigmoid)
+    assert _rel(gemm(dy, wm, b_mn=b_mn, epi=5, aux=pre), want) < 4e-3
+    p2 = pre[:, :H].contiguous()
+    assert _rel(gemm(dy, wm, b_mn=b_mn, epi=2, aux=p2), dh * 2 * p2.double().relu()) < 4e-3
+
+
 # ------------------------------------------------------------------------------------------------ head
 @pytest.mark.parametrize("N,V,d,chunk", [(1, 16, 16, 4096), (300, 1000, 24, 128), (513, 264, 136, 512), (40, 104, 64, 7)])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
