@@ -34,7 +34,11 @@ static torch::Tensor dgrad(const torch::Tensor& dy, const torch::Tensor& w) {   
 static torch::Tensor wgrad(const torch::Tensor& dy, const torch::Tensor& x, bool f32) {       // dy^T x
   return gemm(dy, x, c10::nullopt, c10::nullopt, c10::nullopt, true, true, false, EPI_NONE, f32, 1, c10::nullopt, 0);
 }
-static torch::Tensor rows(const torch::Tensor& t) { return t.reshape({-1, t.size(-1)}).contiguous(); }
+// (rows, width), contiguous and on a 16-byte boundary
+static torch::Tensor rows(const torch::Tensor& t) {
+  torch::Tensor r = t.reshape({-1, t.size(-1)}).contiguous();
+  return (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) == 0 ? r : r.clone();
+}
 
 // x (B,T,d) fp32; pending (B,T,d) bf16 or none.  -> h (M,d), a (M,d) | n, rstd, qkv, o, lse, qk
 std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, Opt pending, torch::Tensor nw, double eps, torch::Tensor wqkv, torch::Tensor wo,

@@ -173,6 +173,12 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, ac
                   out_dtype == torch.float32, int(groups), counts, int(count_mode) if counts is not None else 0)
 
 
+def dense(t):
+    """`t` contiguous and on a 16-byte boundary, as the tensor maps want it: copied only if it is not."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def gemm_ok(M, N, K):
     """Shapes the TMA descriptors accept: 16-byte row pitches (multiples of 8 bf16 elements).  Any number of rows M: it is
     never an inner dimension (in the weight gradient it is the contraction, whose ragged end is filled with zeros)."""
@@ -190,7 +196,7 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
-        dy = dy.contiguous()
+        dy = dense(dy)
         dx = dw = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy, w, b_mn=True)
@@ -274,7 +280,7 @@ class _LinearAct(torch.autograd.Function):
         x, w, pre = ctx.saved_tensors
         C = _ext.C()
         _ext.count()
-        dpre = C.swiglu_bwd(dh.contiguous(), pre) if ctx.swi else C.relu2_bwd(dh.contiguous(), pre)
+        dpre = C.swiglu_bwd(dense(dh), pre) if ctx.swi else C.relu2_bwd(dense(dh), pre)
         dx = gemm(dpre, w, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = gemm(dpre, x, a_mn=True, b_mn=True) if ctx.needs_input_grad[1] else None
         return dx, dw, None
@@ -305,7 +311,7 @@ class _FFN(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w_up, w_down, pre, h = ctx.saved_tensors
-        dy = dy.contiguous()
+        dy = dense(dy)
         if ctx.swi and not FUSE_DSWIGLU:
             dpre = _ext.C().swiglu_bwd(gemm(dy, w_down, b_mn=True), pre)
         else:
@@ -326,7 +332,7 @@ def ffn(x, w_up, w_down, act, direct=False):
         H = N // 2 if act == "swiglu" else N
         if (gemm_ok(M, N, K) and gemm_ok(M, D, H) and M >= 256 and N % 16 == 0 and H % 8 == 0
                 and w_down.shape[1] == H):
-            y = _FFN.apply(x2.contiguous(), weight_bf16(w_up, direct).contiguous(), weight_bf16(w_down, direct).contiguous(),
+            y = _FFN.apply(dense(x2), dense(weight_bf16(w_up, direct)), dense(weight_bf16(w_down, direct)),
                            act == "swiglu")
             return y.view(*x.shape[:-1], D)
     return linear(linear_act(x, w_up, act, direct=direct), w_down, direct=direct)
@@ -341,7 +347,7 @@ def linear_act(x, w, act, direct=False):
         M, K = x2.shape
         N = wd.shape[0]
         if gemm_ok(M, N, K) and M >= 128 and N % 16 == 0:
-            h = _LinearAct.apply(x2.contiguous(), wd.contiguous(), act == "swiglu")
+            h = _LinearAct.apply(dense(x2), dense(wd), act == "swiglu")
             return h.view(*x.shape[:-1], h.shape[-1])
     y = linear(x, w, direct=direct)
     return relu2(y) if act == "relu2" else swiglu(y)
@@ -359,7 +365,7 @@ def linear(x, w, dtype=None, direct=False):
         M, K = x2.shape
         N = wd.shape[0]
         if PLAIN_GEMM == "tc" and dt == torch.bfloat16 and gemm_ok(M, N, K) and M >= 128:
-            y = _Linear.apply(x2.contiguous(), wd.contiguous())
+            y = _Linear.apply(dense(x2), dense(wd))
         else:
             y = F.linear(x2, wd)
         return y.view(*x.shape[:-1], N)

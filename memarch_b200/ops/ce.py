@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from . import _ext, ref
-from .basic import gemm, gemm_ok
+from .basic import dense, gemm, gemm_ok
 
 CE_ROWS_CHUNK = 4096
 
@@ -21,8 +21,8 @@ def _ce_forward_cuda(h, w, y, gate, hit, cand, cval, chunk):
     C = _ext.C()
     N, d = h.shape
     V = w.shape[0]
-    hd = h.to(torch.bfloat16).contiguous()
-    wd = w.to(torch.bfloat16).contiguous()
+    hd = dense(h.to(torch.bfloat16))
+    wd = dense(w.to(torch.bfloat16))
     gh = torch.empty_like(hd)
     gw = torch.empty(V, d, device=h.device, dtype=torch.float32)
     loss = torch.empty(N, device=h.device, dtype=torch.float32)

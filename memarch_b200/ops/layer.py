@@ -18,7 +18,7 @@ def _trained(w):
 
 
 def _operand(w):
-    return basic.shadow_bf16(w) if torch.is_grad_enabled() else basic.weight_bf16(w).contiguous()
+    return basic.shadow_bf16(w) if torch.is_grad_enabled() else basic.dense(basic.weight_bf16(w))
 
 
 def _common(x, nw, ws):

@@ -475,3 +475,32 @@ def test_linear_ce_chunks(N, V, d, chunk, wdt):
         assert a.dtype == h.dtype and b.dtype == wdt and _rel(a, gh) < 2e-2 and _rel(b, gw) < 2e-2
     a2, = torch.autograd.grad(loss, (h,), create_graph=True)
     assert torch.allclose(a2, a, rtol=1e-2, atol=1e-6)
+
+
+# ------------------------------------------------------------------------------------------------ operands off the 16-byte boundary
+@pytest.mark.parametrize("M", [301, 304])
+def test_operands_off_the_boundary(M):
+    """Inputs and gradients that start between two 16-byte pieces are copied, not refused."""
+    from memarch_b200 import ops
+    from memarch_b200.models.blocks import LightBlock
+    shift = lambda t: torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, gy = (torch.randn(s, 64, device="cuda", generator=g).bfloat16() for s in (M, 64, M))
+    y = torch.randint(0, 64, (M,), device="cuda", generator=g)
+    torch.manual_seed(M)
+    with torch.device("cuda"):
+        b = LightBlock(64, 1)
+    res = []
+    for move in (shift, lambda t: t.clone()):
+        a, u, f = (move(t).requires_grad_() for t in (x, w, x.float()[None]))
+        o = ops.linear(a, u)
+        o.backward(move(gy))
+        q = ops.ffn(a, u, u, "relu2")
+        q.backward(move(gy))
+        loss = ops.linear_ce(a, u, y)
+        loss.backward()
+        h, p = b(f, 16, None, True)
+        torch.autograd.backward([h, p], [f.detach() * 0.5, move(gy[None])])
+        res.append([o, q, loss, a.grad, u.grad, h, p, f.grad])
+    for s, t in zip(*res):
+        assert torch.equal(s, t) or _rel(s, t) < 1e-5
