@@ -30,8 +30,8 @@ struct GemmParams {
   int store_tma, count_mode, dbg, group_m;
   int aux_tma;             // the aux operand of an epilogue (pre-activations) is prefetched by TMA into the staging tiles
   const int* counts;
-  // Pair kernel, plain epilogue: the contraction is cut into `splits` runs of `kb_split` k-blocks, each a work item of its
-  // own whose fp32 partial result is added to the output by the TMA store (0 or 1: not cut).
+  // Pair kernel, plain epilogue, one group: the contraction is cut into `splits` runs of `kb_split` k-blocks, each a work item
+  // of its own whose fp32 partial result goes to its own slab out + run * out_gs (0 or 1: not cut).
   int splits, kb_split;
 };
 
@@ -41,7 +41,8 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
 void launch_gemm(const void* A, long long a_rows_pitch, long long a_gs, bool a_mn, const void* B, long long b_rows_pitch,
                  long long b_gs, bool b_mn, GemmParams p, cudaStream_t stream, int max_ctas);
 int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split);
-void round_rows_launch(const float* src, void* dst, long long rows, int n, int ldo, cudaStream_t stream);
+// dst (rows, n) of pitch ldo (+)= the sum of `splits` fp32 slabs (rows, n), always in the same order; n % 4 == 0, 16-byte rows
+void sum_parts_launch(const float* parts, int splits, void* dst, int f32, int accumulate, long long rows, int n, int ldo, cudaStream_t stream);
 int gemm_sm_count();
 int* gemm_status_word(int device);
 bool gemm_pair_on();

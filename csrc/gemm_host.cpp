@@ -73,28 +73,23 @@ torch::Tensor gemm(torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor
   TORCH_CHECK(epi != EPI_SWIGLU || (!out_f32 && N % 16 == 0),
               "gemm: the SwiGLU epilogue writes bf16 and needs column halves of a multiple of 8 (16-byte TMA coordinates)");
   p.status = gemm_status_word(a.get_device());
-  // few output tiles and a long contraction: split it (the parts are added in fp32, rounded once at the end)
-  torch::Tensor sums;
+  // few output tiles and a long contraction: split it.  Every part is kept in fp32 and they are added in a fixed order: the
+  // same bits on every call.
+  torch::Tensor parts;
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   if (p.epi == EPI_NONE && p.count_mode == 0 && N % 4 == 0) {
     int kb_split = 0;
     const int splits = gemm_splits(M, N, K, G, gemm_sm_count(), kb_split);
     if (splits > 1) {
-      if (!out_f32) {
-        sums = torch::empty({M, N}, a.options().dtype(torch::kFloat32));
-        p.out = sums.data_ptr(); p.ldo = N; p.out_f32 = 1;
-      }
-      if (!accumulate) {
-        C10_CUDA_CHECK(cudaMemset2DAsync(p.out, sizeof(float) * (size_t)p.ldo, 0, sizeof(float) * (size_t)N, M, stream));
-        p.accumulate = 1;
-      }
+      parts = torch::empty({splits, M, N}, a.options().dtype(torch::kFloat32));
+      p.out = parts.data_ptr(); p.ldo = N; p.out_gs = (long long)M * N; p.out_f32 = 1; p.accumulate = 0;
       p.splits = splits; p.kb_split = kb_split;
     }
   }
   launch_gemm(A.data_ptr(), A.stride(1), G > 1 ? A.stride(0) : 0, a_mn, B.data_ptr(), B.stride(1), G > 1 ? B.stride(0) : 0,
               b_mn, p, stream, gemm_sm_count());
-  if (sums.defined()) {
-    round_rows_launch(sums.data_ptr<float>(), O.data_ptr(), M, N, (int)O.stride(1), stream);
+  if (parts.defined()) {
+    sum_parts_launch(parts.data_ptr<float>(), p.splits, O.data_ptr(), out_f32, accumulate, M, N, (int)O.stride(1), stream);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   }
   return out;

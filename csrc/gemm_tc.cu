@@ -1166,7 +1166,8 @@ gemm_pair_kernel(const __grid_constant__ TmapSet tmAs, const __grid_constant__ C
           drained = !zero_tile || half != 0;
           if (!zero_tile) epilogue_act<ACT>(p, &tmO, &tmO2, g + p.out_g_off, row0, nt, taddr, ring.base, lane, half, aux, halfbars + q * 4, abort_flag);
         }
-        if (!drained) epilogue_tile3(p, &tmO, &tmO2, g, seg, row0, row0_l, nt, taddr, ring, lane, zero_tile, &aux, abort_flag);
+        // a part of a cut contraction goes to its own slab
+        if (!drained) epilogue_tile3(p, &tmO, &tmO2, p.splits > 1 ? t % p.splits : g, seg, row0, row0_l, nt, taddr, ring, lane, zero_tile, &aux, abort_flag);
         if (*abort_flag) { ok = false; break; }
         if (!zero_tile) {
           tc_fence_before();
@@ -1330,8 +1331,8 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
   p.n_tiles = n_tiles;
   static const bool ntail_on = []() { const char* e = std::getenv("MEMARCH_GEMM_NTAIL"); return !(e && e[0] == '0'); }();
   p.ntail = ntail_on ? 1 : 0;
-  check(p.splits <= 1 || (pair && !tall && n_seg == 1 && p.count_mode == 0 && p.epi == EPI_NONE && p.out_f32 && p.accumulate),
-        "gemm: split contraction needs the pair kernel, a plain epilogue and an accumulating fp32 output");
+  check(p.splits <= 1 || (pair && !tall && n_seg == 1 && G == 1 && p.count_mode == 0 && p.epi == EPI_NONE && p.out_f32 && !p.accumulate),
+        "gemm: split contraction needs the pair kernel, a plain epilogue and fp32 slabs");
   const int total = G * p.m_tiles * p.n_tiles * std::max(1, p.splits);
   int grid = pair ? 2 * std::min(total, max_ctas / 2) : std::min(total, max_ctas);
   if (grid <= 0) return;
@@ -1347,10 +1348,9 @@ void launch_gemm_seg(const void* const* A_list, int n_seg, int seg_M, int a_grou
     p.store_tma = (n_seg == 1 && !p.out_seg_on && (p.ldo * esz) % 16 == 0 && (G == 1 || (p.out_gs * esz) % 16 == 0) &&
                    (!p.out2 || ((p.ldo2 * 2) % 16 == 0 && (G == 1 || (p.out2_gs * 2) % 16 == 0)))) ? 1 : 0;
     if (!tma_stores_on()) p.store_tma = 0;
-    check(p.splits <= 1 || p.store_tma, "gemm: split contraction adds its parts with TMA stores");
     if (p.store_tma) {
       const int No = sw ? N / 2 : N;
-      tmO = make_tmap(p.out, esz, No, p.M, G, p.ldo, p.out_gs, p.out_f32 ? 32 : 64, 32, false);
+      tmO = make_tmap(p.out, esz, No, p.M, std::max(G, p.splits), p.ldo, p.out_gs, p.out_f32 ? 32 : 64, 32, false);
       if (p.out2) tmO2 = make_tmap(p.out2, 2, N, p.M, G, p.ldo2, p.out2_gs, 64, 32, false);
       // SwiGLU backward writes (d gate | d up) side by side: one map per half, so a ragged last chunk of the first
       // half is clipped at H instead of running into the second
@@ -1421,27 +1421,42 @@ void launch_gemm(const void* A, long long a_rows_pitch, long long a_gs, bool a_m
   launch_gemm_seg(list, 1, p.M, p.G, a_rows_pitch, a_gs, a_mn, B, b_rows_pitch, b_gs, b_mn, p, stream, max_ctas);
 }
 
-// fp32 -> bf16 copy of a (rows, n) matrix, n % 4 == 0
-__global__ void __launch_bounds__(256) round_rows_kernel(const float4* __restrict__ src, bf16* __restrict__ dst, long long n4, int row4, int ldo) {
+// out (+)= parts[0] + parts[1] + ... in this order: the runs of a cut contraction always meet the same way, whichever of
+// them ends first.  The slabs were just written and are read from L2; eight loads in flight per thread.
+template <bool F32>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float4* __restrict__ parts, int splits, void* __restrict__ dst, int accumulate,
+                                                        long long n4, int row4, int ldo) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / row4;
-    const float4 v = src[i];
-    *reinterpret_cast<uint2*>(dst + r * ldo + (i - r * row4) * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    const long long r = i / row4, at = r * ldo + (i - r * row4) * 4;
+    float4 s = parts[i];
+#pragma unroll 8
+    for (int k = 1; k < splits; ++k) {
+      const float4 v = parts[k * n4 + i];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    if (F32) {
+      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(dst) + at);
+      if (accumulate) { const float4 v = *o; s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+      *o = s;
+    } else {
+      *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(dst) + at) = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+    }
   }
 }
-void round_rows_launch(const float* src, void* dst, long long rows, int n, int ldo, cudaStream_t stream) {
+void sum_parts_launch(const float* parts, int splits, void* dst, int f32, int accumulate, long long rows, int n, int ldo, cudaStream_t stream) {
   const long long n4 = rows * (n / 4);
   const int grid = (int)std::min<long long>((n4 + 255) / 256, 148 * 8);
-  round_rows_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<bf16*>(dst), n4, n / 4, ldo);
+  const float4* src = reinterpret_cast<const float4*>(parts);
+  if (f32) sum_parts_kernel<true><<<grid, 256, 0, stream>>>(src, splits, dst, accumulate, n4, n / 4, ldo);
+  else sum_parts_kernel<false><<<grid, 256, 0, stream>>>(src, splits, dst, 0, n4, n / 4, ldo);
 }
 
 // How many runs to cut the contraction of one plain product into (1: none).  A product with fewer output tiles than
-// half of the 74 CTA pairs leaves the rest of the chip idle; every run costs a clear, an fp32 reduce-add and (for bf16) a
-// rounding pass over the output, so a run keeps at least 8 k-blocks (512 of the contraction).  (1000, 256, K = 50304):
-// 333 us whole, 38 + 5 in 18 runs; (256, 1024, K = 2048): 20 us whole, 11.5 + 4 in 4.
+// half of the 74 CTA pairs leaves the rest of the chip idle; every run costs an fp32 slab that a second kernel reads back and
+// adds up in run order, so a run keeps at least 8 k-blocks (512 of the contraction).
 int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
   kb_split = 0;
-  if (G != 1 || M < 256 || !gemm_pair_on() || !tma_stores_on()) return 1;
+  if (G != 1 || M < 256 || !gemm_pair_on()) return 1;
   const int tiles = ((M + 255) / 256) * ((N + BN - 1) / BN), pairs = max_ctas / 2, kb = (K + BK - 1) / BK;
   if (2 * tiles > pairs || kb < 32) return 1;
   const int want = std::min(pairs / tiles, kb / 8);

@@ -118,6 +118,20 @@ def test_gemm_split_contraction(M, N, K):
             assert _rel(acc, want + 1) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(256, 8, 2048), (1000, 256, 50304), (256, 1024, 2048), (512, 1536, 4096), (300, 264, 8200)])
+def test_gemm_split_contraction_repeats(M, N, K):
+    """The parts of a cut contraction are added in a fixed order: the same call gives the same bits."""
+    from memarch_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a, b = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    for kw in (dict(), dict(out_dtype=torch.float32), dict(out_dtype=torch.float32, accumulate=True)):
+        def call():
+            out = torch.full((M, N), 0.5, device="cuda") if "accumulate" in kw else None
+            return gemm(a, b, out=out, **kw)
+        first = call()
+        assert all(torch.equal(call(), first) for _ in range(20))
+
+
 # ------------------------------------------------------------------------------------------------ narrow tiles
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 256), (257, 264, 128), (4095, 512, 520), (1001, 136, 64), (256, 1024, 2048), (9472, 256, 64), (513, 8, 16)])
 def test_gemm_narrow_tiles(M, N, K):
