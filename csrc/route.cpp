@@ -62,6 +62,9 @@ std::vector<torch::Tensor> route_bwd(torch::Tensor x, torch::Tensor w, torch::Te
   a.probs = probs.data_ptr<float>(); a.top_e = i64(top_e); a.flat_idx = i64(flat_idx); a.aux_grad = aux_grad.data_ptr<float>();
   a.d_wt = grad_ptr(d_wt, (int64_t)a.N * a.k); a.d_wtab = grad_ptr(d_wtab, (int64_t)a.E * C); a.d_aux = grad_ptr(d_aux, 1);
   a.d_probs = grad_ptr(d_probs, probs.numel());
+  a.dw_runs = route_dw_runs(a.N, a.d, a.E, a.dw_run);
+  auto part = torch::empty({a.dw_runs, a.E, a.d}, dw.options());
+  a.dw_part = part.data_ptr<float>();
   a.dl = dl.data_ptr<float>(); a.dx = dx.data_ptr(); a.dw = dw.data_ptr<float>();
   route_bwd_launch(a);
   C10_CUDA_KERNEL_LAUNCH_CHECK();

@@ -1,4 +1,4 @@
-// The router of an expert layer in two launches forward and two (and a clear) backward.
+// The router of an expert layer in two launches forward and three backward.
 //
 // Forward 1 (route_fwd_kernel): logits = x W^T in fp32 from the bf16 rows, softmax, top-k by probability (ties: smaller
 // expert first), budget k_tok, renormalised weights, and per block of 32 tokens the number of choices and the sum of
@@ -8,15 +8,16 @@
 // the combine weights of the places, and (first block) filled places, dropped share and the Switch auxiliary loss
 //   aux = E * sum_e (choices of e / all choices) * (mean probability of e over the real tokens).
 // Backward 1 (route_dx_kernel): gradient of the logits from the gradients of the weights, of the place weights and of aux, and
-// dx = dlogits W.  Backward 2 (route_dw_kernel): dW = dlogits^T x.
+// dx = dlogits W.  Backward 2 and 3 (route_dw_kernel, route_dw_fold_kernel): dW = dlogits^T x.
 // All of it is memory-bound on x (33 MB for 8192 x 2048).  A warp takes 4 or 8 tokens at a time, so that W (E x d fp32) is
 // read once for them and mostly from L1 (the choice stands at route_fwd_launch).  Us for 8192 x 2048, 8 experts, 8 tokens per
 // warp -> 4: route_fwd 59 -> 30, route_dx 55 -> 44; route_dw with 64 tokens per block instead of 256: 48 -> 17.
+#include <algorithm>
+
 #include "common.cuh"
 #include "route_api.h"
 
 namespace mb {
-
 
 __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -298,35 +299,65 @@ __global__ void __launch_bounds__(ROUTE_TOK / TOK * 32) route_dx_kernel(RouteArg
   }
 }
 
-// grid (column tiles of 512, token runs, groups of 8 experts): a thread owns two columns of 8 experts
+// grid (column tiles of 512, runs of tokens, groups of 8 experts): a thread owns two columns of 8 experts and walks its run 64
+// tokens at a time.  part[run] (E, d) = the run's share of dW; route_dw_fold_kernel adds the shares in order, so that the
+// gradient has the same bits on every call.
 constexpr int DW_RUN = 64;
 __global__ void __launch_bounds__(256) route_dw_kernel(RouteArgs a) {
   __shared__ __align__(16) float g[DW_RUN][8];
   const int c = (blockIdx.x * 256 + threadIdx.x) * 2, e0 = blockIdx.z * 8;
-  const int n0 = blockIdx.y * DW_RUN, n1 = min(a.N, n0 + DW_RUN);
-  for (int i = threadIdx.x; i < (n1 - n0) * 8; i += 256) {
-    const int e = e0 + (i & 7);
-    g[i >> 3][i & 7] = e < a.E ? a.dl[(long long)(n0 + (i >> 3)) * a.E + e] : 0.f;
-  }
-  __syncthreads();
-  if (c >= a.d) return;
   float acc[8][2] = {};
   const uint32_t* X = reinterpret_cast<const uint32_t*>(a.x);
   const long long pitch = a.d / 2;
+  const int end = min(a.N, (int)(blockIdx.y + 1) * a.dw_run);
+  for (int n0 = blockIdx.y * a.dw_run; n0 < end; n0 += DW_RUN) {
+    const int n1 = min(end, n0 + DW_RUN);
+    __syncthreads();
+    for (int i = threadIdx.x; i < (n1 - n0) * 8; i += 256) {
+      const int e = e0 + (i & 7);
+      g[i >> 3][i & 7] = e < a.E ? a.dl[(long long)(n0 + (i >> 3)) * a.E + e] : 0.f;
+    }
+    __syncthreads();
+    if (c >= a.d) continue;
 #pragma unroll 8
-  for (int n = n0; n < n1; ++n) {
-    const float2 x = unpack_bf16(X[n * pitch + c / 2]);
-    const float4 g0 = *reinterpret_cast<const float4*>(g[n - n0]), g1 = *reinterpret_cast<const float4*>(g[n - n0] + 4);
-    const float ge[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+    for (int n = n0; n < n1; ++n) {
+      const float2 x = unpack_bf16(X[n * pitch + c / 2]);
+      const float4 g0 = *reinterpret_cast<const float4*>(g[n - n0]), g1 = *reinterpret_cast<const float4*>(g[n - n0] + 4);
+      const float ge[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { acc[j][0] = fmaf(ge[j], x.x, acc[j][0]); acc[j][1] = fmaf(ge[j], x.y, acc[j][1]); }
+      for (int j = 0; j < 8; ++j) { acc[j][0] = fmaf(ge[j], x.x, acc[j][0]); acc[j][1] = fmaf(ge[j], x.y, acc[j][1]); }
+    }
   }
+  if (c >= a.d) return;
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    if (e0 + j < a.E) {
-      float* dst = a.dw + (long long)(e0 + j) * a.d + c;
-      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(acc[j][0]), "f"(acc[j][1]) : "memory");
-    }
+    if (e0 + j < a.E)
+      *reinterpret_cast<float2*>(a.dw_part + ((long long)blockIdx.y * a.E + e0 + j) * a.d + c) = make_float2(acc[j][0], acc[j][1]);
+}
+// block = 32 elements of dW x 8 lanes of runs
+__global__ void __launch_bounds__(256) route_dw_fold_kernel(const float* __restrict__ part, float* __restrict__ dw, int runs, int n) {
+  __shared__ float sh[8][33];
+  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5, i = blockIdx.x * 32 + cx;
+  float s = 0.f;
+  if (i < n)
+#pragma unroll 8
+    for (int r = ry; r < runs; r += 8) s += part[(long long)r * n + i];
+  sh[ry][cx] = s;
+  __syncthreads();
+  if (ry == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += sh[k][cx];
+    dw[i] = s;
+  }
+}
+
+// Runs of at least 64 tokens, and at most 32 MB of shares: with 8 experts of 2048 columns that is one run for each 64 of 32 768
+// tokens.
+int route_dw_runs(int N, int d, int E, int& run) {
+  const long long most = std::max<long long>(1, (8ll << 20) / ((long long)E * d));
+  const long long per = ((N + most - 1) / most + DW_RUN - 1) / DW_RUN * DW_RUN;
+  run = (int)per;
+  return (int)((N + per - 1) / per);
 }
 
 // 4 tokens per warp and 8 experts at a time keep twice the warps in flight; with many experts W no longer fits L1 and 8
@@ -341,10 +372,10 @@ void route_fwd_launch(const RouteArgs& a) {
 void route_bwd_launch(const RouteArgs& a) {
   const int nb = route_blocks(a.N);
   const size_t smem = (size_t)ROUTE_TOK * a.E * 4;
-  cudaMemsetAsync(a.dw, 0, sizeof(float) * (size_t)a.E * a.d, a.stream);
   if (a.E <= 16) route_dx_kernel<4><<<nb, ROUTE_TOK / 4 * 32, smem, a.stream>>>(a);
   else route_dx_kernel<8><<<nb, ROUTE_TOK / 8 * 32, smem, a.stream>>>(a);
-  route_dw_kernel<<<dim3((a.d + 511) / 512, (a.N + DW_RUN - 1) / DW_RUN, (a.E + 7) / 8), 256, 0, a.stream>>>(a);
+  route_dw_kernel<<<dim3((a.d + 511) / 512, a.dw_runs, (a.E + 7) / 8), 256, 0, a.stream>>>(a);
+  route_dw_fold_kernel<<<(a.E * a.d + 31) / 32, 256, 0, a.stream>>>(a.dw_part, a.dw, a.dw_runs, a.E * a.d);
 }
 
 }  // namespace mb

@@ -31,10 +31,13 @@ struct RouteArgs {
   float* dl;                   // workspace (N, E): gradient of the logits
   void* dx;                    // (N, d) bf16
   float* dw;                   // (E, d)
+  float* dw_part;              // workspace (dw_runs, E, d)
+  int dw_runs, dw_run;         // runs of tokens and their length: route_dw_runs()
   cudaStream_t stream;
 };
 inline int route_blocks(int N) { return (N + ROUTE_TOK - 1) / ROUTE_TOK; }
 void route_fwd_launch(const RouteArgs& a);
+int route_dw_runs(int N, int d, int E, int& run);
 void route_bwd_launch(const RouteArgs& a);
 
 }  // namespace mb

@@ -208,7 +208,7 @@ def moe_route(xf, router_w, real, k_tok, k_max, E):
 
 class _RouteSlot(torch.autograd.Function):
     """Router product, softmax, top-k, budget, slotting, place weights and the auxiliary loss in two kernels; backward to
-    the rows and the router weight in two (`csrc/route.cu`)."""
+    the rows and the router weight in three (`csrc/route.cu`)."""
 
     @staticmethod
     def forward(ctx, xf, router_w, real, k_tok, k_max, C):
@@ -227,7 +227,7 @@ class _RouteSlot(torch.autograd.Function):
             return None, None, None, None, None, None
         c = lambda t: None if t is None else t.contiguous()
         dx, dW = _ext.C().route_bwd(*ctx.saved_tensors, ctx.C, c(dw), c(dwtab), c(daux), c(dprobs))
-        _ext.count(2)
+        _ext.count(3)
         return dx, dW, None, None, None, None
 
 

@@ -199,6 +199,33 @@ def test_route_and_slot_fused(N, d, E, k, C):
     assert _rel(xg.grad.cpu(), xc.grad) < 4e-3 and _rel(wg.grad.cpu(), wc.grad) < 1e-4
 
 
+@pytest.mark.parametrize("N,d,E", [(8192, 2048, 8), (5000, 264, 16), (40000, 512, 128)])
+def test_router_gradients_repeat(N, d, E):
+    """The router weight's gradient is summed over the tokens in a fixed order: the same call gives the same bits.  The last size
+    has runs of more than 64 tokens."""
+    from memarch_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(N, d, device="cuda", generator=g).bfloat16()
+    w = torch.randn(E, d, device="cuda", generator=g) * d ** -0.5
+    real, k_tok = torch.rand(N, device="cuda", generator=g) > 0.1, torch.full((N,), 2, device="cuda")
+    gw, gp = torch.randn(N, 2, device="cuda", generator=g), torch.randn(N, E, device="cuda", generator=g)
+
+    def grads():
+        xg, wg = x.clone().requires_grad_(), w.clone().requires_grad_()
+        o = ops.route_and_slot(xg, wg, real, k_tok, 2, E, N // E)
+        torch.autograd.backward([o[0], o[6]], [gw, gp])
+        return xg.grad, wg.grad
+    first = grads()
+    for _ in range(10):
+        assert all(torch.equal(a, b) for a, b in zip(grads(), first))
+    # against the sum over the tokens in 64 bits, from the same gradient of the logits
+    p = torch.softmax(x.double() @ w.double().t(), 1).requires_grad_()
+    top, idx = p.topk(2, 1)
+    dp, = torch.autograd.grad([top / top.sum(1, keepdim=True), p], p, [gw.double(), gp.double()])
+    dl = p.detach() * (dp - (dp * p.detach()).sum(1, keepdim=True))
+    assert _rel(first[1], dl.t() @ x.double()) < 1e-4
+
+
 # ------------------------------------------------------------------------------------------------ expert rows
 @pytest.mark.parametrize("N,d,E,C,k", [(1, 8, 1, 1, 1), (37, 264, 3, 7, 2), (300, 1032, 8, 64, 2), (65, 2048, 4, 33, 4), (50, 100, 2, 9, 2), (500, 768, 2, 100, 8)])
 def test_expert_row_moves(N, d, E, C, k):
