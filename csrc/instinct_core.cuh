@@ -579,10 +579,11 @@ __device__ __forceinline__ void st8_bf16(bf16* dst, const float* v) {
 }
 
 // rowsq / rowabs as instinct_stat_rows.  grid (blocks); dynamic shared memory: C floats when colsum is given, then
-// the rings (blockDim * S * 16 * (slots of g + slots of m) bytes).
+// the rings (blockDim * S * 16 * (slots of g + slots of m) bytes).  Dealt out in runs of `unit` chunks: 1, or a row's, which
+// leaves no row cut between warps (the parts of a cut row are added in the order they come).
 template <int S>
 __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, const float* __restrict__ colsum, float col_count,
-                                                             float* __restrict__ rowsq, float* __restrict__ rowabs) {
+                                                             float* __restrict__ rowsq, float* __restrict__ rowabs, long long unit) {
   extern __shared__ __align__(16) float sm[];
   float* cs = colsum ? sm : nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -594,14 +595,14 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
   ring.nslot = gs + ms;
   const long long cpr = a.C >> 8, cpe = a.R * cpr;       // chunks per row, per expert
   const long long NC = a.E * cpe;
-  const long long lo = NC * blockIdx.x / gridDim.x, hi = NC * (blockIdx.x + 1) / gridDim.x;
+  const long long NU = NC / unit, lo = NU * blockIdx.x / gridDim.x * unit, hi = NU * (blockIdx.x + 1) / gridDim.x * unit;
   for (long long seg = lo; seg < hi;) {
     const long long e = seg / cpe, seg_hi = min(hi, (e + 1) * cpe);
     if (cs) {
       __syncthreads();
       load_colscale(cs, colsum, nullptr, e, a.C, col_count);
     }
-    const long long cpw = (seg_hi - seg + nw - 1) / nw;
+    const long long cpw = ((seg_hi - seg) / unit + nw - 1) / nw * unit;
     const long long f0 = min(seg_hi, seg + warp * cpw), total = min(seg_hi, f0 + cpw) - f0;
     // both arrays bf16: 8 consecutive elements per lane are one full 16-byte copy each (faster than two 8-byte ones)
     const bool packed = a.g_bf16 && a.m_bf16;
@@ -916,6 +917,9 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   // dealt out in chunks of 256 elements: two or more for each of 148 x 16 warps (sums), four for each of 148 x 12 (update),
   // else filling and draining the rings costs more than the block-per-row form
   const bool s8_rows = aligned8 && ER * (a.C >> 8) >= 2 * 148 * 16, s8_chunks = aligned8 && ER * (a.C >> 8) >= 4 * 148 * 12;
+  // Kinds without column sums repeat bit for bit: whole rows, one per warp at least, else the block-per-row form.  (The others add
+  // to their columns from many blocks and do not repeat anyway.)
+  const bool by_rows = kind != 4 && kind != 5;
   constexpr size_t S8_SMEM = 216 * 1024;
   // launch `kern<S>` with the deepest ring that fits beside `head` bytes: T threads, `slots` 16-byte slots per stage
   auto s8_launch = [&](auto k12, auto k8, auto k6, auto k4, int T, int slots, size_t head, auto&&... args) {
@@ -931,9 +935,9 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   };
   auto stat_rows = [&](const float* colsum, float* out, float* absout) {
     const size_t smem = colsum ? Cb : 0;
-    if (s8_rows && smem + 4 * 512 * 4 * 16 <= S8_SMEM) {
+    if ((by_rows ? aligned8 && ER >= 148 * 16 : s8_rows) && smem + 4 * 512 * 4 * 16 <= S8_SMEM) {
       s8_launch(instinct_stat_rows_s8<12>, instinct_stat_rows_s8<8>, instinct_stat_rows_s8<6>, instinct_stat_rows_s8<4>, 512,
-                (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2), smem, a, colsum, Rf, out, absout);
+                (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2), smem, a, colsum, Rf, out, absout, by_rows ? a.C >> 8 : 1ll);
       return;
     }
     dim3 grid(blocks_per_expert(smem), E);

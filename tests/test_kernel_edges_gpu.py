@@ -364,6 +364,28 @@ def test_instinct_streamed_forms(shape, bf16):
     assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-7 * grad.float().abs()).all()
 
 
+@pytest.mark.parametrize("norm,shape", [("row", (1024, 4096)), ("row", (3000, 2048)), ("row", (64, 65536)), ("tensor", (1024, 2048)), ("hs", (12000, 512))])
+def test_instinct_row_norms_repeat(norm, shape):
+    """Steps whose norms are taken over rows or the whole weight alone (the last one is a word table) give the same bits on every call."""
+    from memarch_b200.config import OptConfig
+    from memarch_b200.optim import Instinct
+    g = torch.Generator(device="cuda").manual_seed(shape[0])
+    p0, grad = torch.randn(*shape, device="cuda", generator=g) * 0.05, (torch.randn(*shape, device="cuda", generator=g) * 1e-3).bfloat16()
+    m0, res = torch.randn(*shape, device="cuda", generator=g) * 1e-3, []
+    for _ in range(8):
+        p = torch.nn.Parameter(p0.clone())
+        opt = Instinct([p], OptConfig(lr=1e-2, norm=norm, scale=0.12, m_bf16=True, rel_every=1 << 30))
+        opt.n_step = 1
+        opt.m[0].copy_(m0)
+        kind, wd, vocab = opt.spec(p)
+        assert kind in ("row", "tensor", "vocab")
+        opt._sync_lr()
+        with torch.no_grad():
+            opt._update_cuda(0, p, grad, kind, 0.1 if wd else 0.0, opt._lr_t, False)
+        res.append(p.detach().clone())
+    assert all(torch.equal(a, res[0]) for a in res[1:])
+
+
 # ------------------------------------------------------------------------------------------------ attention
 @pytest.mark.parametrize("B,T,H,window,half", [(1, 1, 1, 0, False), (2, 63, 3, 0, True), (1, 64, 2, 0, False), (2, 65, 1, 0, False), (1, 127, 3, 5, True), (2, 128, 2, 0, True),
                                                (2, 129, 2, 0, False), (1, 300, 2, 1, False), (1, 511, 2, 64, False), (1, 700, 2, 100, True), (2, 900, 3, 129, False),
