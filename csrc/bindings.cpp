@@ -53,6 +53,7 @@ int64_t instinct_step(torch::Tensor p, torch::Tensor grad, torch::Tensor m, c10:
 std::vector<torch::Tensor> anchor_select(torch::Tensor s, torch::Tensor tau, int64_t A);
 std::vector<torch::Tensor> moe_slots(torch::Tensor e_flat, int64_t E, int64_t C);
 std::vector<torch::Tensor> lock_find(torch::Tensor x, int64_t vocab, int64_t n_keys, bool longest_only);
+int64_t lock_status(int64_t device);
 std::vector<torch::Tensor> lock_find_bucket(torch::Tensor x, int64_t vocab, int64_t n_keys, c10::optional<torch::Tensor> bucket);
 std::vector<torch::Tensor> moe_route_fwd(torch::Tensor logits, torch::Tensor real, torch::Tensor k_tok, int64_t k_max);
 std::vector<torch::Tensor> mem_read_fwd(torch::Tensor q, torch::Tensor faces, torch::Tensor valid, torch::Tensor dim_pen,
@@ -151,6 +152,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_slots", &mb::moe_slots);
   m.def("lock_find", &mb::lock_find);
   m.def("lock_find_bucket", &mb::lock_find_bucket);
+  m.def("lock_status", &mb::lock_status, "read and clear the status word of the lock search (1: a word id outside the trust table)");
   m.def("attn_fwd_tc", &mb::attn_fwd_tc, "causal / sliding-window attention forward on tcgen05 (head dim 64)");
   m.def("attn_status_read", &mb::attn_status_read);
   m.def("route_fwd", &mb::route_fwd, "router, slotting and auxiliary loss of an expert layer");

@@ -50,4 +50,9 @@ std::vector<torch::Tensor> lock_find_bucket(torch::Tensor x, int64_t vocab, int6
   return find(x, vocab, n_keys, bucket.has_value() && bucket->defined(), bucket, true);
 }
 
+int64_t lock_status(int64_t device) {
+  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  return lock_status_read();
+}
+
 }  // namespace mb

@@ -151,6 +151,17 @@ __global__ void __launch_bounds__(LK_WARPS * 32) lock_search_kernel(const long l
   if (n_pend > 0) look_up(n_pend);
 }
 
+__device__ int lock_status_word = 0;                // a word id that no entry of the trust table belongs to was met
+
+// Trust bucket of word x: ids past the table take its last entry, negative ones count from its end.  Ids below that belong to
+// nobody: the status word says so and no memory outside the table is read.
+__device__ __forceinline__ long long bucket_of(const long long* bucket, long long n, long long x) {
+  long long i = min(x, n - 1);
+  if (i < 0) i += n;
+  if (i < 0) { atomicExch(&lock_status_word, LOCK_BAD_ID); i = 0; }
+  return bucket[i];
+}
+
 // candidates, firing locks (only the longest one when `longest_only`) and trust buckets from the positions
 __global__ void lock_finish_kernel(LockArgs a, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -163,7 +174,7 @@ __global__ void lock_finish_kernel(LockArgs a, long long n) {
       a.on[i * a.n_keys + k] = found && !(a.longest_only && longer);
       longer |= found;
     }
-    if (a.bk) a.bk[i] = a.bucket ? a.bucket[min(a.x[i], a.n_bucket - 1)] : 0;
+    if (a.bk) a.bk[i] = a.bucket ? bucket_of(a.bucket, a.n_bucket, a.x[i]) : 0;
   }
 }
 
@@ -207,8 +218,16 @@ __global__ void lock_scan_kernel(const long long* __restrict__ x, long long* __r
       src[o] = sp;
       on[o] = ok[n];
     }
-    if (bk) bk[(long long)b * T + t] = bucket ? bucket[min(xr[t], n_bucket - 1)] : 0;
+    if (bk) bk[(long long)b * T + t] = bucket ? bucket_of(bucket, n_bucket, xr[t]) : 0;
   }
+}
+
+int lock_status_read() {
+  int v = 0;
+  const int z = 0;
+  cudaMemcpyFromSymbol(&v, lock_status_word, sizeof(int));
+  if (v) cudaMemcpyToSymbol(lock_status_word, &z, sizeof(int));
+  return v;
 }
 
 bool lock_find_launch(const LockArgs& a) {

@@ -8,7 +8,7 @@ struct LockArgs {
   const long long* x;            // (B, T) word ids
   long long *cand, *src;         // (B, T, n_keys)
   bool* on;                      // (B, T, n_keys)
-  const long long* bucket;       // optional table of n_bucket entries: bk[b, t] = bucket[min(x, n_bucket - 1)]
+  const long long* bucket;       // optional table of n_bucket entries: bk[b, t] = bucket[min(x, n_bucket - 1)], x < 0 from the end
   long long* bk;                 // (B, T), zeros without a table; null: not wanted
   long long n_bucket;
   long long vocab;
@@ -17,5 +17,8 @@ struct LockArgs {
 };
 // false: the shared memory could not be had (nothing was launched)
 bool lock_find_launch(const LockArgs& a);
+enum { LOCK_BAD_ID = 1 };
+// status word of the current device, cleared: LOCK_BAD_ID when a word id below -n_bucket was looked up (host sync)
+int lock_status_read();
 
 }  // namespace mb

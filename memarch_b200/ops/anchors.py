@@ -24,6 +24,9 @@ def select_anchors(s, tau, A):
 
 
 def find_locks(x, vocab, n_keys=3, lock_bucket=None):
+    """(candidates, firing locks, trust bucket, source position) per word and key length.  `lock_bucket` is read as
+    `lock_bucket[min(x, len - 1)]`, negative ids from its end; an id below -len is an error: an exception on CPU, on the GPU the
+    bucket of id -len and a status word that the training loop turns into one (`_C.lock_status`)."""
     if _ext.use_cuda(x):
         fused = lock_bucket is None or (lock_bucket.dtype == torch.int64 and lock_bucket.device == x.device
                                         and lock_bucket.is_contiguous() and lock_bucket.dim() == 1)

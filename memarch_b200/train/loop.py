@@ -332,13 +332,16 @@ def _schedules(args, env, tr):
 
 
 def device_status(tr):
-    """Read the status words of the GEMM and peer kernels (host sync); raise if a bounded device wait ran out."""
+    """Read the status words of the GEMM, lock search and peer kernels (host sync); raise if a bounded device wait ran out
+    or a word id lay outside the trust table."""
     from ..ops import _ext
     if tr.device.type != "cuda" or not _ext.available():
         return
     st = _ext.C().gemm_status(tr.device.index or 0)
     if st:
         raise RuntimeError(f"a GEMM kernel gave up a bounded wait (status {st}); results since the last check are not valid")
+    if _ext.C().lock_status(tr.device.index or 0):
+        raise RuntimeError("find_locks: a word id lies below the trust table (ids down to -len(lock_bucket) are served)")
     par = getattr(tr, "parallel", None)
     if par is not None:
         par.check()

@@ -54,6 +54,27 @@ def test_lock_find_tables_and_scan(text, B, T, n_keys):
         assert torch.equal(got[0][..., 0].cpu(), want[0][..., 0]) and torch.equal(got[3][..., 0].cpu(), want[3][..., 0])
 
 
+@pytest.mark.parametrize("B,T", [(2, 700), (1, 1), (1, 30001)])
+def test_lock_buckets_of_ids_outside_the_table(B, T):
+    """Tables and scan: ids past the table take its last entry, negative ones count from its end, ids below that set the status
+    word; memory before the table is never read."""
+    from memarch_b200.ops import _ext, anchors, ref
+    g = torch.Generator().manual_seed(T)
+    x = torch.randint(-40, 90, (B, T), generator=g)
+    x[0, 0] = -40
+    bucket = torch.randint(0, 9, (40,), generator=g)
+    mem = torch.full((120,), -77)                        # entries around the table that must not turn up
+    mem[40:80] = bucket
+    table = mem.cuda()[40:80]
+    got, want = anchors.find_locks(x.cuda(), 50304, 3, table), ref.find_locks(x, 50304, 3, bucket)
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu(), b)
+    assert _ext.C().lock_status(0) == 0
+    x[-1, -1] = -41
+    bk = anchors.find_locks(x.cuda(), 50304, 3, table)[2]
+    assert bk[-1, -1].item() == bucket[0].item() and _ext.C().lock_status(0) == 1 and _ext.C().lock_status(0) == 0
+
+
 # ------------------------------------------------------------------------------------------------ RMSNorm, cross-entropy rows
 @pytest.mark.parametrize("n,d", [(1, 8), (3, 256), (5, 264), (17, 512), (9, 520), (33, 1024), (2, 1032), (700, 2048), (3, 2056), (4, 4096), (5, 4104), (2, 8192), (3, 8200), (5000, 64)])
 def test_rmsnorm_widths(n, d):

@@ -567,6 +567,9 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
         def gemm_status(self, dev):
             return self.st
 
+        def lock_status(self, dev):
+            return 0
+
     class Engine:
         def check(self):
             raise RuntimeError("peer wait timed out (status 5): a rank did not reach the barrier within 4000.0 ms")
@@ -584,6 +587,20 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
         loop.device_status(tr)
     tr_cpu = types.SimpleNamespace(device=torch.device("cpu"), parallel=Engine())
     loop.device_status(tr_cpu)                                    # CPU runs have no status words
+
+
+def test_loop_reports_word_ids_outside_the_trust_table(monkeypatch):
+    """The lock search leaves a status word for an id that no entry of the trust table belongs to; the loop turns it into an
+    exception where it reads the other words."""
+    import types
+    import torch
+    from memarch_b200.ops import _ext
+    from memarch_b200.train import loop
+    fake = types.SimpleNamespace(gemm_status=lambda dev: 0, lock_status=lambda dev: 1)
+    monkeypatch.setattr(_ext, "available", lambda: True)
+    monkeypatch.setattr(_ext, "C", lambda: fake)
+    with pytest.raises(RuntimeError, match="trust table"):
+        loop.device_status(types.SimpleNamespace(device=torch.device("cuda", 0), parallel=None))
 
 
 def test_named_weight_switches_of_the_optimizer():
