@@ -7,8 +7,8 @@
 // n-gram of the share - linear in T for each warp, and the shares of all texts and key lengths run side by side.
 // 32 kept positions are looked up at a time: equal keys inside the batch find each other by match, the first of
 // each group asks the table, the last of each group becomes the table's new latest position.
-// The table is exact: keys are the n-gram itself (21 bits per word), chains resolve equal slots, and a share with more
-// distinct n-grams than nodes (LK_NODES; about T / shares = 256 are expected) answers the overflowing ones by scanning
+// The table is exact: keys are the n-gram itself (21 bits per word; a text with an id outside -2^20 .. 2^20 - 1 is scanned
+// instead), chains resolve equal slots, and a share with more distinct n-grams than nodes (LK_NODES; about T / shares = 256 are expected) answers the overflowing ones by scanning
 // the text back, as all positions were before.
 // What bounds it: staging the text and the walk, T / 128 steps of one warp.  4 texts x 16 384 words, three key lengths: 1183 us by scanning,
 // 38 by the tables.
@@ -31,9 +31,9 @@ struct LockTable {                                   // one per warp
 };
 
 __device__ __forceinline__ unsigned long long ngram_key(const int* tok, int t, int n) {
-  unsigned long long k = (unsigned)tok[t];
-  if (n >= 2) k |= (unsigned long long)(unsigned)tok[t - 1] << 21;
-  if (n >= 3) k |= (unsigned long long)(unsigned)tok[t - 2] << 42;
+  unsigned long long k = (unsigned)tok[t] & 0x1FFFFF;
+  if (n >= 2) k |= (unsigned long long)((unsigned)tok[t - 1] & 0x1FFFFF) << 21;
+  if (n >= 3) k |= (unsigned long long)((unsigned)tok[t - 2] & 0x1FFFFF) << 42;
   return k;
 }
 __device__ __forceinline__ unsigned hash64(unsigned long long k) {
@@ -52,10 +52,23 @@ __global__ void __launch_bounds__(LK_WARPS * 32) lock_search_kernel(const long l
   LockTable& tab = reinterpret_cast<LockTable*>(lk_smem)[warp];
   int* tok = reinterpret_cast<int*>(lk_smem + LK_WARPS * sizeof(LockTable));
   const long long* xr = x + (long long)b * T;
+  int wide = 0;
 #pragma unroll 8
-  for (int t = threadIdx.x; t < T; t += LK_WARPS * 32) tok[t] = (int)xr[t] & 0x1FFFFF;
+  for (int t = threadIdx.x; t < T; t += LK_WARPS * 32) {
+    tok[t] = (int)xr[t];
+    wide |= (unsigned)(tok[t] + (1 << 20)) >> 21;
+  }
   for (int i = lane; i < LK_SLOTS; i += 32) tab.slot[i] = LK_NODES;
-  __syncthreads();
+  if (__syncthreads_or(wide)) {
+    // 21 bits do not tell this text's words apart: scan back from every position, on whole ids
+    for (int t = blockIdx.x * (LK_WARPS * 32) + threadIdx.x; t < T; t += gridDim.x * (LK_WARPS * 32)) {
+      int j = t >= n - 1 ? t - 1 : -1;
+      for (; j >= n - 1; --j)
+        if (tok[j] == tok[t] && (n < 2 || tok[j - 1] == tok[t - 1]) && (n < 3 || tok[j - 2] == tok[t - 2])) break;
+      src[((long long)b * T + t) * n_keys + (n - 1)] = j >= n - 1 ? min(j + 1, T - 1) : 0;
+    }
+    return;
+  }
   // which of this block's warps takes position t: hashed once for all of them (LK_WARPS = none of them, or too early for
   // an n-gram)
   unsigned char* whose = reinterpret_cast<unsigned char*>(tok + T);

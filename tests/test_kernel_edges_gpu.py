@@ -75,6 +75,21 @@ def test_lock_buckets_of_ids_outside_the_table(B, T):
     assert bk[-1, -1].item() == bucket[0].item() and _ext.C().lock_status(0) == 1 and _ext.C().lock_status(0) == 0
 
 
+@pytest.mark.parametrize("T", [40, 2500])
+@pytest.mark.parametrize("low", [-(1 << 20), -(1 << 20) - 1, (1 << 21) - 3, 1 << 30])
+def test_lock_ids_outside_the_vocabulary(T, low):
+    """Words are told apart by their whole id, also where ids differ by a multiple of 2^21."""
+    from memarch_b200.ops import anchors, ref
+    g = torch.Generator().manual_seed(T)
+    x = torch.randint(0, 6, (2, T), generator=g) + torch.where(torch.rand(2, T, generator=g) < 0.5, low, low + (1 << 21) if low < 1 << 30 else 3)
+    x[1] = torch.randint(0, 6, (T,), generator=g)         # the other text is an ordinary one
+    ids, compact = x.unique(return_inverse=True)          # the statement packs n-grams into 64 bits: small ids for it
+    cand, on, bk, src = ref.find_locks(compact, ids.numel(), 3, None)
+    want = torch.where(src > 0, ids[cand], torch.zeros_like(cand)), on, bk, src
+    for a, b in zip(anchors.find_locks(x.cuda(), 50304, 3, None), want):
+        assert torch.equal(a.cpu(), b)
+
+
 # ------------------------------------------------------------------------------------------------ RMSNorm, cross-entropy rows
 @pytest.mark.parametrize("n,d", [(1, 8), (3, 256), (5, 264), (17, 512), (9, 520), (33, 1024), (2, 1032), (700, 2048), (3, 2056), (4, 4096), (5, 4104), (2, 8192), (3, 8200), (5000, 64)])
 def test_rmsnorm_widths(n, d):
