@@ -7,7 +7,11 @@
 
 namespace mb {
 
-static torch::Tensor f32(const torch::Tensor& w) { return w.scalar_type() == torch::kFloat32 ? w : w.to(torch::kFloat32); }
+// the norm weight as the kernels read it: d consecutive fp32 values
+static torch::Tensor norm_weight(const torch::Tensor& w, int64_t d) {
+  TORCH_CHECK(w.numel() == d, "rmsnorm: one weight per column");
+  return w.to(torch::kFloat32).contiguous();
+}
 static bool is_bf16(const torch::Tensor& t) { return t.scalar_type() == torch::kBFloat16; }
 static bool float_or_bf16(const torch::Tensor& t) { return is_bf16(t) || t.scalar_type() == torch::kFloat32; }
 
@@ -17,7 +21,7 @@ std::vector<torch::Tensor> add_rmsnorm_fwd(torch::Tensor x, torch::Tensor y, tor
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && y.is_contiguous() && x.scalar_type() == torch::kFloat32 &&
               is_bf16(y) && x.numel() == y.numel() && x.size(1) % 4 == 0, "add_rmsnorm: fp32 + bf16");
   const int n = x.size(0), d = x.size(1);
-  const torch::Tensor wf = f32(w);
+  const torch::Tensor wf = norm_weight(w, d);
   auto h = torch::empty_like(x);
   auto nn = torch::empty({n, d}, x.options().dtype(torch::kBFloat16));
   auto rstd = torch::empty({n}, x.options());
@@ -34,7 +38,7 @@ std::vector<torch::Tensor> rmsnorm_fwd(torch::Tensor x, torch::Tensor w, double 
   const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(1) % 4 == 0, "rmsnorm: (N,d) contiguous, d % 4 == 0");
   const int n = x.size(0), d = x.size(1);
-  const torch::Tensor wf = f32(w);
+  const torch::Tensor wf = norm_weight(w, d);
   auto y = torch::empty({n, d}, x.options().dtype(out_bf16 ? torch::kBFloat16 : torch::kFloat32));
   auto rstd = torch::empty({n}, x.options().dtype(torch::kFloat32));
   if (n == 0) return {y, rstd};
@@ -60,7 +64,7 @@ std::vector<torch::Tensor> rmsnorm_bwd(torch::Tensor dy, torch::Tensor x, torch:
   const int n = x.size(0), d = x.size(1);
   TORCH_CHECK(d <= 8 * 4 * 256 && d % 4 == 0, "rmsnorm_bwd: d <= 8192");
   TORCH_CHECK(float_or_bf16(x) && float_or_bf16(dy), "rmsnorm_bwd: fp32 or bf16");
-  const torch::Tensor wf = f32(w);
+  const torch::Tensor wf = norm_weight(w, d);
   auto dx = torch::empty_like(x);
   torch::Tensor lo = want_lo ? torch::empty({n, d}, x.options().dtype(torch::kBFloat16)) : torch::Tensor();
   auto f = x.options().dtype(torch::kFloat32);

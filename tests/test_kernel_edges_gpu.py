@@ -508,6 +508,29 @@ def test_light_layer_halves_leave_other_cases_alone():
         assert ok(x)
 
 
+@pytest.mark.parametrize("train", [True, False])
+def test_light_layer_with_strided_norm_weights(train):
+    """Norm weights that are views with a stride give what their contiguous copies give."""
+    from memarch_b200.models.blocks import LightBlock
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        b = LightBlock(128, 2)
+    wide = torch.rand(2, 128, 4, device="cuda") + 0.5
+    x, go = torch.randn(2, 200, 128, device="cuda"), torch.randn(2, 200, 128, device="cuda")
+    res = []
+    for take in (lambda w: w[:, 0], lambda w: w[:, 0].contiguous()):
+        b.n1.weight, b.n2.weight = (torch.nn.Parameter(take(w)) for w in wide)
+        b.zero_grad(set_to_none=True)
+        with torch.set_grad_enabled(train):
+            a = x.clone().requires_grad_()
+            y = b(a, 64)
+        if train:
+            y.backward(go)
+        res.append([y.detach(), a.grad, b.n1.weight.grad, b.n2.weight.grad, b.qkv.weight.grad] if train else [y])
+    for p, q in zip(*res):
+        assert torch.equal(p, q)
+
+
 # ------------------------------------------------------------------------------------------------ padded groups
 @pytest.mark.parametrize("E,C,counts", [(1, 256, [3]), (3, 2561, [2561, 0, 257]), (8, 600, [0, 600, 256, 255, 1, 0, 512, 300]), (128, 257, "mixed"), (130, 300, "mixed"), (2, 300, [0, 0])])
 @pytest.mark.parametrize("act", ["swiglu", "relu2"])
