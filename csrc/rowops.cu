@@ -8,6 +8,7 @@
 
 namespace mb {
 
+static bool on16(const torch::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 static inline cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream(); }
 
 template <typename T> __device__ __forceinline__ float4 ld4(const T* p);
@@ -55,7 +56,7 @@ static inline int ew_grid(long long n, int threads) { return (int)std::min<long 
 
 torch::Tensor relu2_fwd(torch::Tensor a) {
   const c10::cuda::CUDAGuard guard(a.device());
-  TORCH_CHECK(a.is_contiguous() && a.scalar_type() == torch::kBFloat16 && a.numel() % 8 == 0, "relu2: bf16, numel % 8");
+  TORCH_CHECK(a.is_contiguous() && a.scalar_type() == torch::kBFloat16 && a.numel() % 8 == 0 && on16(a), "relu2: bf16, numel % 8, 16-byte aligned");
   auto h = torch::empty_like(a);
   long long n8 = a.numel() / 8;
   if (n8) relu2_fwd_kernel<<<ew_grid(n8, 256), 256, 0, cur_stream()>>>(
@@ -65,7 +66,7 @@ torch::Tensor relu2_fwd(torch::Tensor a) {
 }
 torch::Tensor relu2_bwd(torch::Tensor dh, torch::Tensor a) {
   const c10::cuda::CUDAGuard guard(a.device());
-  TORCH_CHECK(dh.is_contiguous() && a.is_contiguous() && dh.scalar_type() == torch::kBFloat16, "relu2_bwd: bf16");
+  TORCH_CHECK(dh.is_contiguous() && a.is_contiguous() && dh.scalar_type() == torch::kBFloat16 && on16(dh) && on16(a), "relu2_bwd: bf16, 16-byte aligned");
   auto da = torch::empty_like(a);
   long long n8 = a.numel() / 8;
   if (n8) relu2_bwd_kernel<<<ew_grid(n8, 256), 256, 0, cur_stream()>>>(
@@ -117,7 +118,7 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dh, const bf16* __res
 }
 torch::Tensor swiglu_fwd(torch::Tensor gu) {
   const c10::cuda::CUDAGuard guard(gu.device());
-  TORCH_CHECK(gu.is_contiguous() && gu.scalar_type() == torch::kBFloat16 && gu.size(-1) % 16 == 0, "swiglu: bf16, 2H % 16");
+  TORCH_CHECK(gu.is_contiguous() && gu.scalar_type() == torch::kBFloat16 && gu.size(-1) % 16 == 0 && on16(gu), "swiglu: bf16, 2H % 16, 16-byte aligned");
   const int H = gu.size(-1) / 2;
   const long long R = gu.numel() / (2 * H);
   auto shape = gu.sizes().vec();
@@ -130,7 +131,7 @@ torch::Tensor swiglu_fwd(torch::Tensor gu) {
 }
 torch::Tensor swiglu_bwd(torch::Tensor dh, torch::Tensor gu) {
   const c10::cuda::CUDAGuard guard(gu.device());
-  TORCH_CHECK(dh.is_contiguous() && gu.is_contiguous() && dh.scalar_type() == torch::kBFloat16, "swiglu_bwd: bf16");
+  TORCH_CHECK(dh.is_contiguous() && gu.is_contiguous() && dh.scalar_type() == torch::kBFloat16 && on16(dh) && on16(gu), "swiglu_bwd: bf16, 16-byte aligned");
   const int H = gu.size(-1) / 2;
   const long long R = gu.numel() / (2 * H);
   auto dgu = torch::empty_like(gu);
@@ -193,8 +194,8 @@ __global__ void rope_qk_kernel(const bf16* __restrict__ in, bf16* __restrict__ o
 }
 torch::Tensor rope_qk(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, double sign, bool half) {
   const c10::cuda::CUDAGuard guard(qkv.device());
-  TORCH_CHECK(qkv.dim() == 5 && qkv.size(2) == 3 && qkv.is_contiguous() && qkv.scalar_type() == torch::kBFloat16,
-              "rope_qk: (B,T,3,H,hd) bf16 contiguous");
+  TORCH_CHECK(qkv.dim() == 5 && qkv.size(2) == 3 && qkv.is_contiguous() && qkv.scalar_type() == torch::kBFloat16 && on16(qkv),
+              "rope_qk: (B,T,3,H,hd) bf16 contiguous, 16-byte aligned");
   const int B = qkv.size(0), T = qkv.size(1), H = qkv.size(3), hd = qkv.size(4);
   TORCH_CHECK(hd % 16 == 0, "rope_qk: head dim % 16");
   TORCH_CHECK(cos.is_contiguous() && sin.is_contiguous() && cos.scalar_type() == torch::kFloat32 && cos.size(0) >= T &&
@@ -265,8 +266,9 @@ torch::Tensor rope_merge_bwd(torch::Tensor dq, torch::Tensor dk, torch::Tensor d
   const int B = dq.size(0), H = dq.size(1), T = dq.size(2), hd = dq.size(3);
   Src3 src;
   for (int i = 0; i < 3; ++i) {
-    TORCH_CHECK(g[i].dim() == 4 && g[i].scalar_type() == torch::kBFloat16 && g[i].stride(3) == 1 && g[i].size(2) == T,
-                "rope_merge_bwd: (B,H,T,hd) bf16 with contiguous last dim");
+    TORCH_CHECK(g[i].dim() == 4 && g[i].scalar_type() == torch::kBFloat16 && g[i].stride(3) == 1 && g[i].size(2) == T && on16(g[i]) &&
+                g[i].stride(0) % 8 == 0 && g[i].stride(1) % 8 == 0 && g[i].stride(2) % 8 == 0,
+                "rope_merge_bwd: (B,H,T,hd) bf16 with contiguous last dim, 16-byte aligned rows");
     TORCH_CHECK(g[i].stride(0) % 8 == 0 && g[i].stride(1) % 8 == 0 && g[i].stride(2) % 8 == 0 &&
                 (reinterpret_cast<uintptr_t>(g[i].data_ptr()) & 15) == 0, "rope_merge_bwd: 16-byte aligned rows");
     src.p[i] = reinterpret_cast<const bf16*>(g[i].data_ptr());
@@ -291,7 +293,7 @@ __global__ void resid_add_kernel(const float* __restrict__ x, const bf16* __rest
 torch::Tensor resid_add(torch::Tensor x, torch::Tensor y) {
   const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && x.scalar_type() == torch::kFloat32 &&
-              y.scalar_type() == torch::kBFloat16 && x.numel() == y.numel() && x.numel() % 4 == 0, "resid_add: fp32 + bf16");
+              y.scalar_type() == torch::kBFloat16 && x.numel() == y.numel() && x.numel() % 4 == 0 && on16(x) && on16(y), "resid_add: fp32 + bf16, 16-byte aligned");
   auto out = torch::empty_like(x);
   long long n4 = x.numel() / 4;
   if (n4) resid_add_kernel<<<ew_grid(n4, 256), 256, 0, cur_stream()>>>(x.data_ptr<float>(),

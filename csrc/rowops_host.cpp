@@ -7,10 +7,12 @@
 
 namespace mb {
 
-// the norm weight as the kernels read it: d consecutive fp32 values
+static bool on16(const torch::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+// the norm weight as the kernels read it: d consecutive fp32 values from a 16-byte boundary on
 static torch::Tensor norm_weight(const torch::Tensor& w, int64_t d) {
   TORCH_CHECK(w.numel() == d, "rmsnorm: one weight per column");
-  return w.to(torch::kFloat32).contiguous();
+  const torch::Tensor f = w.to(torch::kFloat32).contiguous();
+  return on16(f) ? f : f.clone();
 }
 static bool is_bf16(const torch::Tensor& t) { return t.scalar_type() == torch::kBFloat16; }
 static bool float_or_bf16(const torch::Tensor& t) { return is_bf16(t) || t.scalar_type() == torch::kFloat32; }
@@ -19,7 +21,7 @@ static bool float_or_bf16(const torch::Tensor& t) { return is_bf16(t) || t.scala
 std::vector<torch::Tensor> add_rmsnorm_fwd(torch::Tensor x, torch::Tensor y, torch::Tensor w, double eps) {
   const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && y.is_contiguous() && x.scalar_type() == torch::kFloat32 &&
-              is_bf16(y) && x.numel() == y.numel() && x.size(1) % 4 == 0, "add_rmsnorm: fp32 + bf16");
+              is_bf16(y) && x.numel() == y.numel() && x.size(1) % 4 == 0 && on16(x) && on16(y), "add_rmsnorm: fp32 + bf16, 16-byte aligned");
   const int n = x.size(0), d = x.size(1);
   const torch::Tensor wf = norm_weight(w, d);
   auto h = torch::empty_like(x);
@@ -36,7 +38,7 @@ std::vector<torch::Tensor> add_rmsnorm_fwd(torch::Tensor x, torch::Tensor y, tor
 
 std::vector<torch::Tensor> rmsnorm_fwd(torch::Tensor x, torch::Tensor w, double eps, bool out_bf16) {
   const c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(1) % 4 == 0, "rmsnorm: (N,d) contiguous, d % 4 == 0");
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(1) % 4 == 0 && on16(x), "rmsnorm: (N,d) contiguous and 16-byte aligned, d % 4 == 0");
   const int n = x.size(0), d = x.size(1);
   const torch::Tensor wf = norm_weight(w, d);
   auto y = torch::empty({n, d}, x.options().dtype(out_bf16 ? torch::kBFloat16 : torch::kFloat32));
@@ -58,12 +60,13 @@ std::vector<torch::Tensor> rmsnorm_bwd(torch::Tensor dy, torch::Tensor x, torch:
   const c10::cuda::CUDAGuard guard(x.device());
   NormArgs a{};
   if (add_.has_value() && add_->defined()) {
-    TORCH_CHECK(add_->scalar_type() == torch::kFloat32 && add_->is_contiguous() && add_->numel() == x.numel(), "rmsnorm_bwd: add");
+    TORCH_CHECK(add_->scalar_type() == torch::kFloat32 && add_->is_contiguous() && add_->numel() == x.numel() && on16(*add_), "rmsnorm_bwd: add");
     a.add = add_->data_ptr<float>();
   }
   const int n = x.size(0), d = x.size(1);
   TORCH_CHECK(d <= 8 * 4 * 256 && d % 4 == 0, "rmsnorm_bwd: d <= 8192");
-  TORCH_CHECK(float_or_bf16(x) && float_or_bf16(dy), "rmsnorm_bwd: fp32 or bf16");
+  TORCH_CHECK(float_or_bf16(x) && float_or_bf16(dy) && x.is_contiguous() && dy.is_contiguous() && dy.numel() == x.numel() && on16(x) && on16(dy),
+              "rmsnorm_bwd: fp32 or bf16 rows, contiguous and 16-byte aligned");
   const torch::Tensor wf = norm_weight(w, d);
   auto dx = torch::empty_like(x);
   torch::Tensor lo = want_lo ? torch::empty({n, d}, x.options().dtype(torch::kBFloat16)) : torch::Tensor();

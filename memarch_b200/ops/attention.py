@@ -17,6 +17,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _ext, ref
+from .basic import dense
 
 ATTN_CORE = os.environ.get("MEMARCH_ATTN", "own")
 OWN_WINDOW_EVAL = os.environ.get("MEMARCH_ATTN_EVAL", "own") == "own"
@@ -45,13 +46,13 @@ class _RopeQK(torch.autograd.Function):
         ctx.half = half
         cos, sin = rope_tables(qkv.shape[1], qkv.shape[4], qkv.device)
         _ext.count()
-        return _ext.C().rope_qk(qkv.contiguous(), cos, sin, 1.0, bool(half))
+        return _ext.C().rope_qk(dense(qkv), cos, sin, 1.0, bool(half))
 
     @staticmethod
     def backward(ctx, g):
         cos, sin = rope_tables(g.shape[1], g.shape[4], g.device)
         _ext.count()
-        return _ext.C().rope_qk(g.contiguous(), cos, sin, -1.0, bool(ctx.half)), None
+        return _ext.C().rope_qk(dense(g), cos, sin, -1.0, bool(ctx.half)), None
 
 
 class _RopeSplit(torch.autograd.Function):
@@ -63,14 +64,14 @@ class _RopeSplit(torch.autograd.Function):
         ctx.half = half
         cos, sin = rope_tables(qkv.shape[1], qkv.shape[4], qkv.device)
         _ext.count()
-        r = _ext.C().rope_qk(qkv.contiguous(), cos, sin, 1.0, bool(half))
+        r = _ext.C().rope_qk(dense(qkv), cos, sin, 1.0, bool(half))
         return r[:, :, 0].transpose(1, 2), r[:, :, 1].transpose(1, 2), r[:, :, 2].transpose(1, 2)
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
         cos, sin = rope_tables(dq.shape[2], dq.shape[3], dq.device)
-        fix = lambda t: t if (t.stride(3) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(2) % 8 == 0) \
-            else t.contiguous()
+        fix = lambda t: t if (t.stride(3) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(2) % 8 == 0
+                            and t.data_ptr() % 16 == 0) else dense(t)
         _ext.count()
         return _ext.C().rope_merge_bwd(fix(dq), fix(dk), fix(dv), cos, sin, bool(ctx.half)), None
 
@@ -128,10 +129,7 @@ class _QkvAttn(torch.autograd.Function):
         qkv, o, lse, qk = ctx.saved_tensors
         cos, sin = rope_tables(qkv.shape[1], qkv.shape[4], qkv.device)
         _ext.count(3)
-        do = do.contiguous()
-        if do.data_ptr() % 16:
-            do = do.clone()
-        return _ext.C().attn_qkv_bwd(do, o, lse, qk, qkv, cos, sin, ctx.half, ctx.window), None, None
+        return _ext.C().attn_qkv_bwd(dense(do), o, lse, qk, qkv, cos, sin, ctx.half, ctx.window), None, None
 
 
 def _lib_window(q, k, v, window):
@@ -191,9 +189,7 @@ def attention(qkv, window=None, rope_half=False, qk_norm=False):
         # (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16 heads: 1222 against 943).
         own = (ATTN_CORE == "own" and (win is not None or T <= OWN_CAUSAL_T)) or (win is not None and no_grad and OWN_WINDOW_EVAL)
         if hd == 64 and own and (no_grad or OWN_BWD):
-            qkv = qkv.contiguous()
-            if qkv.data_ptr() % 16 == 0:
-                return _QkvAttn.apply(qkv, win or 0, rope_half)
+            return _QkvAttn.apply(dense(qkv), win or 0, rope_half)
         q, k, v = _RopeSplit.apply(qkv, rope_half)
         if hd == 64 and own:
             return own_attention(q, k, v, win or 0).transpose(1, 2).reshape(B, T, H * hd)

@@ -24,7 +24,7 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, out_bf16):
         C = _ext.C()
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        x2 = dense(x.reshape(-1, x.shape[-1]))
         y, rstd = C.rmsnorm_fwd(x2, w.contiguous(), float(eps), bool(out_bf16))
         _ext.count()
         ctx.save_for_backward(x2, w, rstd)
@@ -35,7 +35,7 @@ class _RMSNorm(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w, rstd = ctx.saved_tensors
         C = _ext.C()
-        dx, dw, _ = C.rmsnorm_bwd(dy.reshape(x2.shape).contiguous(), x2, w.contiguous(), rstd, None, False)
+        dx, dw, _ = C.rmsnorm_bwd(dense(dy.reshape(x2.shape)), x2, w.contiguous(), rstd, None, False)
         _ext.count(2)
         return dx.view(ctx.shape), dw.to(w.dtype), None, None
 
@@ -59,8 +59,8 @@ class _AddRMSNorm(torch.autograd.Function):
     def forward(ctx, x, y, w, eps):
         C = _ext.C()
         shape = x.shape
-        x2 = x.reshape(-1, shape[-1]).contiguous()
-        y2 = y.reshape(-1, shape[-1]).contiguous()
+        x2 = dense(x.reshape(-1, shape[-1]))
+        y2 = dense(y.reshape(-1, shape[-1]))
         h, n, rstd = C.add_rmsnorm_fwd(x2, y2, w.contiguous(), float(eps))
         _ext.count()
         ctx.save_for_backward(h, w, rstd)
@@ -73,8 +73,8 @@ class _AddRMSNorm(torch.autograd.Function):
         C = _ext.C()
         if dn is None:
             return dh, dh.to(torch.bfloat16), None, None
-        add = dh.reshape(h.shape).contiguous().float() if dh is not None else None
-        dx, dw, lo = C.rmsnorm_bwd(dn.reshape(h.shape).contiguous(), h, w.contiguous(), rstd, add, True)
+        add = dense(dh.reshape(h.shape).float()) if dh is not None else None
+        dx, dw, lo = C.rmsnorm_bwd(dense(dn.reshape(h.shape)), h, w.contiguous(), rstd, add, True)
         _ext.count(2)
         return dx.view(ctx.shape), lo.view(ctx.shape), dw.to(w.dtype), None
 
@@ -95,13 +95,13 @@ class _Relu2(torch.autograd.Function):
     def forward(ctx, a):
         ctx.save_for_backward(a)
         _ext.count()
-        return _ext.C().relu2_fwd(a.contiguous())
+        return _ext.C().relu2_fwd(dense(a))
 
     @staticmethod
     def backward(ctx, dh):
         a, = ctx.saved_tensors
         _ext.count()
-        return _ext.C().relu2_bwd(dh.contiguous(), a.contiguous())
+        return _ext.C().relu2_bwd(dense(dh), dense(a))
 
 
 class _SwiGLU(torch.autograd.Function):
@@ -109,13 +109,13 @@ class _SwiGLU(torch.autograd.Function):
     def forward(ctx, gu):
         ctx.save_for_backward(gu)
         _ext.count()
-        return _ext.C().swiglu_fwd(gu.contiguous())
+        return _ext.C().swiglu_fwd(dense(gu))
 
     @staticmethod
     def backward(ctx, dh):
         gu, = ctx.saved_tensors
         _ext.count()
-        return _ext.C().swiglu_bwd(dh.contiguous(), gu.contiguous())
+        return _ext.C().swiglu_bwd(dense(dh), dense(gu))
 
 
 def relu2(a):
@@ -136,7 +136,7 @@ class _ResidAdd(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, y):
         _ext.count()
-        return _ext.C().resid_add(x.contiguous(), y.contiguous())
+        return _ext.C().resid_add(dense(x), dense(y))
 
     @staticmethod
     def backward(ctx, g):

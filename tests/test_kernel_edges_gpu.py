@@ -626,3 +626,45 @@ def test_operands_off_the_boundary(M):
         res.append([o, q, loss, a.grad, u.grad, h, p, f.grad])
     for s, t in zip(*res):
         assert torch.equal(s, t) or _rel(s, t) < 1e-5
+
+
+@pytest.mark.parametrize("B,T", [(1, 40), (2, 130)])
+def test_single_ops_off_the_boundary(B, T):
+    """The row operations one by one and a light layer of few rows: operands, gradients and norm weights that start between two
+    16-byte pieces are copied before any kernel sees them."""
+    from memarch_b200 import ops
+    from memarch_b200.models.blocks import LightBlock
+    from memarch_b200.ops import basic
+    from memarch_b200.ops.attention import attention
+    shift = lambda t: torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, y, w, go, qkv = rnd(B, T, 64), rnd(B, T, 64).bfloat16(), rnd(64) + 2, rnd(B, T, 64), rnd(B, T, 3, 2, 64).bfloat16()
+    torch.manual_seed(T)
+    with torch.device("cuda"):
+        b = LightBlock(64, 1)
+    res = []
+    for move in (shift, lambda t: t.clone()):
+        out = []
+
+        def run(f, *ts, grad):
+            ts = [move(t).requires_grad_() for t in ts]
+            o = f(*ts)
+            for q, r in zip(o if isinstance(o, tuple) else (o,), grad):
+                q.backward(move(r.to(q.dtype)), retain_graph=True)
+                out.append(q.detach())
+            out.extend(t.grad for t in ts)
+        run(lambda a, u: ops.rmsnorm(a, u, 1e-6), x, w, grad=[go])
+        run(lambda a, u: ops.rmsnorm(a, u, 1e-6), y, w, grad=[go])
+        run(lambda a, q, u: ops.add_rmsnorm(a, q, u, 1e-6), x, y, w, grad=[go, go])
+        run(ops.resid_add, x, y, grad=[go])
+        run(basic.relu2, y, grad=[go])
+        run(basic.swiglu, y, grad=[go[..., :32].contiguous()])
+        run(lambda a: attention(a, 33), qkv, grad=[rnd(1).new_ones(B, T, 128)])
+        b.zero_grad(set_to_none=True)
+        b.n1.weight, b.n2.weight = (torch.nn.Parameter(move(w)) for _ in range(2))
+        run(lambda a: b(a, 2048), x, grad=[go])
+        res.append(out + [v.grad for v in b.parameters()])
+    assert len(res[0]) == len(res[1])
+    for p, q in zip(*res):
+        assert _rel(p, q) < 1e-3                                  # the same arithmetic on copied operands
