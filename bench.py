@@ -302,14 +302,15 @@ def run_ours(args):
                "last_loss": host_loss[-1]}
     st = _ext.C().gemm_status(local)
     peer_st = int(_ext.C().peer_status_read()) if parallel is not None and parallel.fused_impl is not None else 0
-    if st or peer_st:
-        raise RuntimeError(f"a bounded device wait ran out during the benchmark (GEMM status {st}, peer status {peer_st})")
+    attn_st = [int(_ext.C().attn_status_read(local)), int(_ext.C().attn_bwd_status_read(local))]
+    if st or peer_st or any(attn_st):
+        raise RuntimeError(f"a bounded device wait ran out during the benchmark (GEMM status {st}, attention {attn_st}, peer status {peer_st})")
     if rank == 0:
         first, last = float(losses[0]), float(losses[-1])
         emit(args, "ours", world, ms, e2e, clocks, int(per_step_launches * args.steps),
              {"parallel_detail": "replicated weights + expert parallel" if world > 1 else "single",
               "mode": args.mode if world > 1 else "single", "selftest": selftest,
-              "loss_first": round(first, 4), "loss_last": round(last, 4), "kernel_status": st, "peer_status": peer_st,
+              "loss_first": round(first, 4), "loss_last": round(last, 4), "kernel_status": st, "attention_status": attn_st, "peer_status": peer_st,
               "losses": [round(float(l), 4) for l in losses[:16]],
               "gemm_tflop_per_step": round(gemm_tflop, 2),
               "gemm_tflops_achieved": round(gemm_tflop / (ms / 1e3), 1),

@@ -22,7 +22,9 @@ static int* attn_word(int device, int which) {
   }
   return w;
 }
-static int64_t read_word(int which) {
+static int64_t read_word(int64_t device, int which) {        // device -1: the current one
+  c10::cuda::OptionalCUDAGuard guard;
+  if (device >= 0) guard.set_index((c10::DeviceIndex)device);
   int dev = 0;
   cudaGetDevice(&dev);
   int v = 0;
@@ -31,8 +33,8 @@ static int64_t read_word(int which) {
   if (v) cudaMemcpy(attn_word(dev, which), &z, sizeof(int), cudaMemcpyHostToDevice);
   return v;
 }
-int64_t attn_status_read() { return read_word(0); }
-int64_t attn_bwd_status_read() { return read_word(1); }
+int64_t attn_status_read(int64_t device) { return read_word(device, 0); }
+int64_t attn_bwd_status_read(int64_t device) { return read_word(device, 1); }
 
 // t (B, H, T, 64) contiguous
 static AttnView view_bhtd(const torch::Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(2), t.stride(1)}; }

@@ -78,7 +78,7 @@ std::vector<torch::Tensor> route_bwd(torch::Tensor x, torch::Tensor w, torch::Te
                                      torch::Tensor top_e, torch::Tensor flat_idx, torch::Tensor aux_grad, int64_t C,
                                      c10::optional<torch::Tensor> d_wt, c10::optional<torch::Tensor> d_wtab,
                                      c10::optional<torch::Tensor> d_aux, c10::optional<torch::Tensor> d_probs);
-int64_t attn_status_read();
+int64_t attn_status_read(int64_t device);
 std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor o, torch::Tensor dout,
                                        torch::Tensor lse, int64_t window, double scale);
 std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
@@ -95,7 +95,7 @@ std::vector<torch::Tensor> ffn_half_fwd(torch::Tensor h, torch::Tensor a, torch:
 std::vector<torch::Tensor> ffn_half_bwd(torch::Tensor dy, c10::optional<torch::Tensor> dx2, torch::Tensor x2, torch::Tensor n, torch::Tensor rstd,
                                         torch::Tensor pre, torch::Tensor hid, torch::Tensor nw, torch::Tensor wup, torch::Tensor wdown,
                                         bool swiglu, bool grad_f32);
-int64_t attn_bwd_status_read();
+int64_t attn_bwd_status_read(int64_t device);
 torch::Tensor embed_sum_fwd(torch::Tensor emb, torch::Tensor x, c10::optional<torch::Tensor> cand, c10::optional<torch::Tensor> sel,
                             c10::optional<torch::Tensor> phr, c10::optional<torch::Tensor> pidx);
 std::vector<torch::Tensor> embed_sum_bwd(torch::Tensor dh, torch::Tensor emb, torch::Tensor x, c10::optional<torch::Tensor> cand,
@@ -154,7 +154,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("lock_find_bucket", &mb::lock_find_bucket);
   m.def("lock_status", &mb::lock_status, "read and clear the status word of the lock search (1: a word id outside the trust table)");
   m.def("attn_fwd_tc", &mb::attn_fwd_tc, "causal / sliding-window attention forward on tcgen05 (head dim 64)");
-  m.def("attn_status_read", &mb::attn_status_read);
+  m.def("attn_status_read", &mb::attn_status_read, "read and clear the status word of the attention forward kernel (0 = ok)", pybind11::arg("device") = -1);
   m.def("route_fwd", &mb::route_fwd, "router, slotting and auxiliary loss of an expert layer");
   m.def("route_bwd", &mb::route_bwd);
   m.def("attn_half_fwd", &mb::attn_half_fwd, "attention half of a light layer");
@@ -164,7 +164,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_qkv_fwd", &mb::attn_qkv_fwd, "rotation + attention forward on packed projections (head dim 64)");
   m.def("attn_qkv_bwd", &mb::attn_qkv_bwd);
   m.def("attn_bwd_tc", &mb::attn_bwd_tc, "causal / sliding-window attention backward on tcgen05 (head dim 64)");
-  m.def("attn_bwd_status_read", &mb::attn_bwd_status_read);
+  m.def("attn_bwd_status_read", &mb::attn_bwd_status_read, "the same for the two backward kernels", pybind11::arg("device") = -1);
   m.def("mem_read_fwd", &mb::mem_read_fwd);
   m.def("mem_read_bwd", &mb::mem_read_bwd);
   m.def("quant_rows_i8", &mb::quant_rows_i8);

@@ -332,15 +332,17 @@ def _schedules(args, env, tr):
 
 
 def device_status(tr):
-    """Read the status words of the GEMM, lock search and peer kernels (host sync); raise if a bounded device wait ran out
-    or a word id lay outside the trust table."""
+    """Read the status words of the GEMM, attention, lock search and peer kernels (host sync); raise if a bounded device wait
+    ran out or a word id lay outside the trust table."""
     from ..ops import _ext
     if tr.device.type != "cuda" or not _ext.available():
         return
-    st = _ext.C().gemm_status(tr.device.index or 0)
-    if st:
-        raise RuntimeError(f"a GEMM kernel gave up a bounded wait (status {st}); results since the last check are not valid")
-    if _ext.C().lock_status(tr.device.index or 0):
+    C, dev = _ext.C(), tr.device.index or 0
+    for what, read in (("a GEMM", C.gemm_status), ("the attention forward", C.attn_status_read), ("an attention backward", C.attn_bwd_status_read)):
+        st = read(dev)
+        if st:
+            raise RuntimeError(f"{what} kernel gave up a bounded wait (status {st}); results since the last check are not valid")
+    if C.lock_status(dev):
         raise RuntimeError("find_locks: a word id lies below the trust table (ids down to -len(lock_bucket) are served)")
     par = getattr(tr, "parallel", None)
     if par is not None:

@@ -570,6 +570,8 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
         def lock_status(self, dev):
             return 0
 
+        attn_status_read = attn_bwd_status_read = lock_status
+
     class Engine:
         def check(self):
             raise RuntimeError("peer wait timed out (status 5): a rank did not reach the barrier within 4000.0 ms")
@@ -589,6 +591,24 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
     loop.device_status(tr_cpu)                                    # CPU runs have no status words
 
 
+@pytest.mark.parametrize("word", ["gemm_status", "attn_status_read", "attn_bwd_status_read"])
+def test_loop_reads_every_kernel_status_word(monkeypatch, word):
+    """Each family of kernels with bounded waits has a status word of its own, asked for on the trainer's device; any of them stops
+    the run."""
+    import types
+    import torch
+    from memarch_b200.ops import _ext
+    from memarch_b200.train import loop
+    asked = []
+    names = ("gemm_status", "attn_status_read", "attn_bwd_status_read", "lock_status")
+    fake = types.SimpleNamespace(**{n: lambda dev, n=n: asked.append((n, dev)) or (7 if n == word else 0) for n in names})
+    monkeypatch.setattr(_ext, "available", lambda: True)
+    monkeypatch.setattr(_ext, "C", lambda: fake)
+    with pytest.raises(RuntimeError, match="bounded wait.*status 7"):
+        loop.device_status(types.SimpleNamespace(device=torch.device("cuda", 2), parallel=None))
+    assert (word, 2) in asked
+
+
 def test_loop_reports_word_ids_outside_the_trust_table(monkeypatch):
     """The lock search leaves a status word for an id that no entry of the trust table belongs to; the loop turns it into an
     exception where it reads the other words."""
@@ -596,7 +616,8 @@ def test_loop_reports_word_ids_outside_the_trust_table(monkeypatch):
     import torch
     from memarch_b200.ops import _ext
     from memarch_b200.train import loop
-    fake = types.SimpleNamespace(gemm_status=lambda dev: 0, lock_status=lambda dev: 1)
+    clean = lambda dev: 0
+    fake = types.SimpleNamespace(gemm_status=clean, attn_status_read=clean, attn_bwd_status_read=clean, lock_status=lambda dev: 1)
     monkeypatch.setattr(_ext, "available", lambda: True)
     monkeypatch.setattr(_ext, "C", lambda: fake)
     with pytest.raises(RuntimeError, match="trust table"):
