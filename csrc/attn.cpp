@@ -111,28 +111,29 @@ static void check_qkv(const torch::Tensor& qkv) {
               (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15) == 0, "attn_qkv: (B, T, 3, H, 64) bf16 contiguous");
 }
 
-// The attention of a light layer on packed projections: qkv (B, T, 3, H, 64) -> o (B, T, H, 64), lse (B, H, T) and the
-// rotated q and k (B, T, 2, H, 64) that the backward pass reads again; v stays in qkv.
-std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window) {
+// The attention of a light layer on packed projections: qkv (B, T, 3, H, 64) -> o (B, T, H, 64), lse (B, H, T) and, with
+// `keep`, the packed array with q and k rotated, all that the backward pass reads of them.  `in_place`: qkv is the caller's own
+// and is rotated where it lies.
+std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window, bool keep, bool in_place) {
   const c10::cuda::CUDAGuard guard(qkv.device());
   check_qkv(qkv);
-  const int64_t B = qkv.size(0), T = qkv.size(1), H = qkv.size(3);
-  auto qk = torch::empty({B, T, 2, H, 64}, qkv.options());
+  const int64_t B = qkv.size(0), T = qkv.size(1), H = qkv.size(3), slots = keep || in_place ? 3 : 2;
+  auto rot = in_place ? qkv : torch::empty({B, T, slots, H, 64}, qkv.options());
   auto o = torch::empty({B, T, H, 64}, qkv.options());
   auto lse = torch::empty({B, H, T}, qkv.options().dtype(torch::kFloat32));
-  if (B * H * T == 0) return {o, lse, qk};
+  if (B * H * T == 0) return {o, lse, rot};
   AttnArgs a = common_args(qkv, B, H, T, window, 0.125, 0);
   set_tables(a, cos, sin, half);
-  rope_qk2_launch(qkv.data_ptr(), qk.data_ptr(), a.cos, a.sin, a.B, a.T, a.H, a.rope_half, a.stream);
-  a.q = view_packed(qk, 0); a.k = view_packed(qk, 1); a.v = view_packed(qkv, 2); a.o = view_bthd(o);
+  rope_qk2_launch(qkv.data_ptr(), rot.data_ptr(), a.cos, a.sin, a.B, a.T, a.H, a.rope_half, (int)slots, a.stream);
+  a.q = view_packed(rot, 0); a.k = view_packed(rot, 1); a.v = slots == 3 ? view_packed(rot, 2) : view_packed(qkv, 2); a.o = view_bthd(o);
   a.lse = lse.data_ptr<float>();
   run_fwd(a);
-  return {o, lse, qk};
+  return {o, lse, rot};
 }
 
-// dout (B, T, H, 64) contiguous -> gradient of the packed projections (B, T, 3, H, 64)
-torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor qkv,
-                           torch::Tensor cos, torch::Tensor sin, bool half, int64_t window) {
+// dout (B, T, H, 64) contiguous -> gradient of the packed projections (B, T, 3, H, 64); qkv with q and k rotated
+torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half,
+                           int64_t window) {
   const c10::cuda::CUDAGuard guard(qkv.device());
   check_qkv(qkv);
   const int64_t B = qkv.size(0), T = qkv.size(1), H = qkv.size(3);
@@ -142,7 +143,7 @@ torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor ls
   if (B * H * T == 0) return dqkv;
   AttnArgs a = common_args(qkv, B, H, T, window, 0.125, 1);
   set_tables(a, cos, sin, half);
-  a.q = view_packed(qk, 0); a.k = view_packed(qk, 1); a.v = view_packed(qkv, 2); a.o = view_bthd(o);
+  a.q = view_packed(qkv, 0); a.k = view_packed(qkv, 1); a.v = view_packed(qkv, 2); a.o = view_bthd(o);
   a.dout = {dout.data_ptr(), T * H * 64, H * 64, 64};
   a.dq = view_packed(dqkv, 0); a.dk = view_packed(dqkv, 1); a.dv = view_packed(dqkv, 2);
   a.lse = lse.data_ptr<float>();

@@ -31,7 +31,7 @@ inline long long attn_stats_floats(int B, int H, int T) { return (long long)B * 
 // nullptr on success, else what went wrong (nothing was launched then)
 const char* attn_fwd_launch(const AttnArgs& a);
 const char* attn_bwd_launch(const AttnArgs& a);
-// q and k slices of qkv (B, T, 3, H, 64) rotated into out (B, T, 2, H, 64)
-void rope_qk2_launch(const void* qkv, void* out, const float* cos, const float* sin, int B, int T, int H, int half, cudaStream_t st);
+// q and k slices of qkv (B, T, 3, H, 64) rotated into out (B, T, slots, H, 64): 2 slots, or 3 with v copied; out may be qkv (3 slots)
+void rope_qk2_launch(const void* qkv, void* out, const float* cos, const float* sin, int B, int T, int H, int half, int slots, cudaStream_t st);
 
 }  // namespace mb

@@ -335,47 +335,51 @@ const char* attn_fwd_launch(const AttnArgs& a) {
 }
 
 // ------------------------------------------------------------------------------------------------ rotation of q and k
-// One thread per 8 head dims (16 bytes).  v is not touched: attention reads it where the projection left it.
-__global__ void rope_qk2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, const float* __restrict__ cs,
-                                const float* __restrict__ sn, long long n, int T, int H, int half) {
-  const int per_tok = 2 * H * 8;                            // 8-element groups of q and k per position
+// q and k of qkv (B, T, 3, H, 64) rotated into slots 0 and 1 of out (B, T, slots, H, 64); with 3 slots v is copied as well unless
+// out is qkv itself.  A thread takes 16 head dims of one head, in two 16-byte pieces that hold whole pairs: it reads them before
+// it writes them, so that out may be qkv.
+__global__ void rope_qk2_kernel(const bf16* in, bf16* out, const float* __restrict__ cs, const float* __restrict__ sn, long long n, int T, int H,
+                                int half, int slots, int moved) {
+  const int per_tok = moved * H * 4;                        // 16-dim groups per position
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const long long tok = i / per_tok;
-    const int rem = (int)(i - tok * per_tok), gi = rem & 7;
+    const int rem = (int)(i - tok * per_tok), gi = rem & 3, head = rem >> 2;            // head: slot * H + h
     const int t = (int)(tok % T);
-    const bf16* src = in + tok * (3 * H * 64) + (long long)rem * 8;
-    uint4 u = *reinterpret_cast<const uint4*>(src);
-    uint32_t* p = reinterpret_cast<uint32_t*>(&u);
-    if (!half) {
-      const float4 c4 = *reinterpret_cast<const float4*>(cs + (long long)t * 32 + gi * 4);
-      const float4 s4 = *reinterpret_cast<const float4*>(sn + (long long)t * 32 + gi * 4);
-      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+    const int lo = half ? gi * 8 : gi * 16, hi = half ? lo + 32 : lo + 8;
+    const bf16* src = in + (tok * 3 * H + head) * 64;
+    bf16* dst = out + (tok * slots * H + head) * 64;
+    uint4 u = *reinterpret_cast<const uint4*>(src + lo), w = *reinterpret_cast<const uint4*>(src + hi);
+    if (head < 2 * H) {
+      uint32_t *p = reinterpret_cast<uint32_t*>(&u), *q = reinterpret_cast<uint32_t*>(&w);
+      const float4 c0 = *reinterpret_cast<const float4*>(cs + (long long)t * 32 + gi * 8), c1 = *reinterpret_cast<const float4*>(cs + (long long)t * 32 + gi * 8 + 4);
+      const float4 s0 = *reinterpret_cast<const float4*>(sn + (long long)t * 32 + gi * 8), s1 = *reinterpret_cast<const float4*>(sn + (long long)t * 32 + gi * 8 + 4);
+      const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      if (!half) {                                          // pairs (2i, 2i + 1)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16(p[j]);
-        p[j] = pack_bf16(f.x * c[j] - f.y * s[j], f.x * s[j] + f.y * c[j]);
-      }
-    } else {
-      const bool first = gi < 4;
-      const uint4 w = *reinterpret_cast<const uint4*>(src + (first ? 32 : -32));
-      const uint32_t* q = reinterpret_cast<const uint32_t*>(&w);
-      const float* cp = cs + (long long)t * 32 + (gi & 3) * 8;
-      const float* sp = sn + (long long)t * 32 + (gi & 3) * 8;
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = unpack_bf16(p[j]), g = unpack_bf16(q[j]);
+          p[j] = pack_bf16(f.x * c[j] - f.y * s[j], f.x * s[j] + f.y * c[j]);
+          q[j] = pack_bf16(g.x * c[j + 4] - g.y * s[j + 4], g.x * s[j + 4] + g.y * c[j + 4]);
+        }
+      } else {                                              // pairs (i, i + 32)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 a = unpack_bf16(p[j]), m = unpack_bf16(q[j]);
-        const float c0 = cp[2 * j], c1 = cp[2 * j + 1], s0 = first ? -sp[2 * j] : sp[2 * j], s1 = first ? -sp[2 * j + 1] : sp[2 * j + 1];
-        p[j] = pack_bf16(a.x * c0 + m.x * s0, a.y * c1 + m.y * s1);
+        for (int j = 0; j < 4; ++j) {
+          const float2 a = unpack_bf16(p[j]), b = unpack_bf16(q[j]);
+          p[j] = pack_bf16(a.x * c[2 * j] - b.x * s[2 * j], a.y * c[2 * j + 1] - b.y * s[2 * j + 1]);
+          q[j] = pack_bf16(b.x * c[2 * j] + a.x * s[2 * j], b.y * c[2 * j + 1] + a.y * s[2 * j + 1]);
+        }
       }
     }
-    *reinterpret_cast<uint4*>(out + i * 8) = u;
+    *reinterpret_cast<uint4*>(dst + lo) = u;
+    *reinterpret_cast<uint4*>(dst + hi) = w;
   }
 }
-void rope_qk2_launch(const void* qkv, void* out, const float* cos, const float* sin, int B, int T, int H, int half, cudaStream_t st) {
-  const long long n = (long long)B * T * 2 * H * 8;
+void rope_qk2_launch(const void* qkv, void* out, const float* cos, const float* sin, int B, int T, int H, int half, int slots, cudaStream_t st) {
+  const int moved = qkv == out ? 2 : slots;
+  const long long n = (long long)B * T * moved * H * 4;
   if (!n) return;
   const int grid = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-  rope_qk2_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const bf16*>(qkv), reinterpret_cast<bf16*>(out), cos, sin, n, T, H, half);
+  rope_qk2_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const bf16*>(qkv), reinterpret_cast<bf16*>(out), cos, sin, n, T, H, half, slots, moved);
 }
 
 }  // namespace mb

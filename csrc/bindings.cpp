@@ -81,13 +81,13 @@ std::vector<torch::Tensor> route_bwd(torch::Tensor x, torch::Tensor w, torch::Te
 int64_t attn_status_read(int64_t device);
 std::vector<torch::Tensor> attn_bwd_tc(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor o, torch::Tensor dout,
                                        torch::Tensor lse, int64_t window, double scale);
-std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
-torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor qkv,
-                           torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
+std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window, bool keep, bool in_place);
+torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half,
+                           int64_t window);
 std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, c10::optional<torch::Tensor> pending, torch::Tensor nw, double eps, torch::Tensor wqkv,
                                          torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
 std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, c10::optional<torch::Tensor> dh, torch::Tensor h, torch::Tensor n, torch::Tensor rstd,
-                                         torch::Tensor qkv, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor nw,
+                                         torch::Tensor qkv, torch::Tensor o, torch::Tensor lse, torch::Tensor nw,
                                          torch::Tensor wqkv, torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window,
                                          bool want_lo, bool grad_f32);
 std::vector<torch::Tensor> ffn_half_fwd(torch::Tensor h, torch::Tensor a, torch::Tensor nw, double eps, torch::Tensor wup, torch::Tensor wdown,

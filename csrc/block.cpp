@@ -17,9 +17,9 @@ std::vector<torch::Tensor> rmsnorm_bwd(torch::Tensor dy, torch::Tensor x, torch:
                                        c10::optional<torch::Tensor> add, bool want_lo);
 std::vector<torch::Tensor> add_rmsnorm_fwd(torch::Tensor x, torch::Tensor y, torch::Tensor w, double eps);
 torch::Tensor resid_add(torch::Tensor x, torch::Tensor y);
-std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
-torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor qkv,
-                           torch::Tensor cos, torch::Tensor sin, bool half, int64_t window);
+std::vector<torch::Tensor> attn_qkv_fwd(torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window, bool keep, bool in_place);
+torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor lse, torch::Tensor qkv, torch::Tensor cos, torch::Tensor sin, bool half,
+                           int64_t window);
 
 typedef c10::optional<torch::Tensor> Opt;
 static bool has(const Opt& t) { return t.has_value() && t->defined(); }
@@ -40,7 +40,7 @@ static torch::Tensor rows(const torch::Tensor& t) {
   return (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) == 0 ? r : r.clone();
 }
 
-// x (B,T,d) fp32; pending (B,T,d) bf16 or none.  -> h (M,d), a (M,d) | n, rstd, qkv, o, lse, qk
+// x (B,T,d) fp32; pending (B,T,d) bf16 or none.  -> h (M,d), a (M,d) | n, rstd, qkv (q and k rotated), o, lse
 std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, Opt pending, torch::Tensor nw, double eps, torch::Tensor wqkv, torch::Tensor wo,
                                          torch::Tensor cos, torch::Tensor sin, bool half, int64_t window) {
   const c10::cuda::CUDAGuard guard(x.device());
@@ -56,14 +56,14 @@ std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, Opt pending, torch::Te
     n = r[0]; rstd = r[1];
   }
   auto qkv = project(n, wqkv).view({B, T, 3, d / 64, 64});
-  auto at = attn_qkv_fwd(qkv, cos, sin, half, window);
+  auto at = attn_qkv_fwd(qkv, cos, sin, half, window, true, true);
   auto a = project(at[0].view({B * T, d}), wo);
-  return {h, a, n, rstd, qkv, at[0], at[1], at[2]};
+  return {h, a, n, rstd, qkv, at[0], at[1]};
 }
 
 // da (B,T,d) bf16; dh (B,T,d) fp32 or none.  -> dx (M,d), dx in bf16 (or undefined), d nw, d wqkv, d wo
 std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, Opt dh, torch::Tensor h, torch::Tensor n, torch::Tensor rstd, torch::Tensor qkv,
-                                         torch::Tensor o, torch::Tensor lse, torch::Tensor qk, torch::Tensor nw, torch::Tensor wqkv,
+                                         torch::Tensor o, torch::Tensor lse, torch::Tensor nw, torch::Tensor wqkv,
                                          torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window, bool want_lo,
                                          bool grad_f32) {
   const c10::cuda::CUDAGuard guard(da.device());
@@ -71,7 +71,7 @@ std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, Opt dh, torch::Tensor
   const torch::Tensor g = rows(da);
   auto dout = dgrad(g, wo);
   auto dwo = wgrad(g, o.view({M, d}), grad_f32);
-  auto dqkv = attn_qkv_bwd(dout, o, lse, qk, qkv, cos, sin, half, window).view({M, 3 * d});
+  auto dqkv = attn_qkv_bwd(dout, o, lse, qkv, cos, sin, half, window).view({M, 3 * d});
   auto dn = dgrad(dqkv, wqkv);
   auto dwqkv = wgrad(dqkv, n, grad_f32);
   auto r = rmsnorm_bwd(dn, h, nw, rstd, has(dh) ? Opt(rows(*dh)) : Opt(), want_lo);

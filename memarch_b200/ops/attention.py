@@ -111,25 +111,27 @@ def own_attention(q, k, v, window=0):
 
 class _QkvAttn(torch.autograd.Function):
     """RoPE + causal / sliding-window attention on packed projections qkv (B,T,3,H,64) -> (B,T,H*64), window 0 = plain
-    causal.  Forward rotates q and k into a buffer of their own and reads v where the projection left it; backward
-    writes dq, dk (rotated back) and dv straight into one packed gradient."""
+    causal.  Forward rotates q and k; for a backward pass one packed array is kept, with v beside them (without one, v is read
+    where the projection left it).  Backward writes dq, dk (rotated back) and dv straight into one packed gradient."""
 
     @staticmethod
     def forward(ctx, qkv, window, half):
         B, T, _, H, hd = qkv.shape
         cos, sin = rope_tables(T, hd, qkv.device)
-        o, lse, qk = _ext.C().attn_qkv_fwd(qkv, cos, sin, bool(half), int(window))
+        keep = ctx.needs_input_grad[0]
+        o, lse, rot = _ext.C().attn_qkv_fwd(qkv, cos, sin, bool(half), int(window), keep, False)
         _ext.count(2)
-        ctx.save_for_backward(qkv, o, lse, qk)
+        if keep:
+            ctx.save_for_backward(o, lse, rot)
         ctx.window, ctx.half = int(window), bool(half)
         return o.view(B, T, H * hd)
 
     @staticmethod
     def backward(ctx, do):
-        qkv, o, lse, qk = ctx.saved_tensors
-        cos, sin = rope_tables(qkv.shape[1], qkv.shape[4], qkv.device)
+        o, lse, rot = ctx.saved_tensors
+        cos, sin = rope_tables(rot.shape[1], rot.shape[4], rot.device)
         _ext.count(3)
-        return _ext.C().attn_qkv_bwd(dense(do), o, lse, qk, qkv, cos, sin, ctx.half, ctx.window), None, None
+        return _ext.C().attn_qkv_bwd(dense(do), o, lse, rot, cos, sin, ctx.half, ctx.window), None, None
 
 
 def _lib_window(q, k, v, window):
@@ -189,7 +191,7 @@ def attention(qkv, window=None, rope_half=False, qk_norm=False):
         # (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16 heads: 1222 against 943).
         own = (ATTN_CORE == "own" and (win is not None or T <= OWN_CAUSAL_T)) or (win is not None and no_grad and OWN_WINDOW_EVAL)
         if hd == 64 and own and (no_grad or OWN_BWD):
-            return _QkvAttn.apply(dense(qkv), win or 0, rope_half)
+            return _QkvAttn.apply(dense(qkv.detach() if no_grad else qkv), win or 0, rope_half)
         q, k, v = _RopeSplit.apply(qkv, rope_half)
         if hd == 64 and own:
             return own_attention(q, k, v, win or 0).transpose(1, 2).reshape(B, T, H * hd)

@@ -62,14 +62,14 @@ class _AttnHalf(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dh, da):
-        h, n, rstd, qkv, o, lse, qk, nw, sq, so = ctx.saved_tensors
+        h, n, rstd, qkv, o, lse, nw, sq, so = ctx.saved_tensors
         if da is None:
             if dh is None:
                 return (None,) * 8
             da = torch.zeros(ctx.shape, device=dh.device, dtype=torch.bfloat16)
         cos, sin = rope_tables(ctx.shape[1], 64, h.device)
         f32 = basic.WEIGHT_GRAD_SINK is None
-        dx, lo, dnw, dwqkv, dwo = _ext.C().attn_half_bwd(da, dh, h, n, rstd, qkv, o, lse, qk, nw, sq, so, cos, sin, ctx.half, ctx.window,
+        dx, lo, dnw, dwqkv, dwo = _ext.C().attn_half_bwd(da, dh, h, n, rstd, qkv, o, lse, nw, sq, so, cos, sin, ctx.half, ctx.window,
                                                          ctx.has_pending, f32)
         _count(dx, 8 * dx.shape[1], 9)
         wqkv, wo = ctx.ws

@@ -447,6 +447,47 @@ def test_attention_on_packed_projections(B, T, H, window, half):
         assert (a.double() - b.double()).norm() < 2e-2 * max(b.double().norm(), 1e-2 * x.grad.double().norm()), i
 
 
+def _held():
+    return torch.cuda.memory_stats()["requested_bytes.all.current"]
+
+
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("half", [False, True])
+def test_attention_keeps_one_packed_array(window, half):
+    """What stays on the device for the backward pass: the output, its log-sums and one packed array with q and k rotated; without a
+    backward pass the result alone.  The projections themselves are not written to."""
+    from memarch_b200.ops.attention import _QkvAttn
+    leaf = torch.randn(2, 500, 3, 8, 64, device="cuda").bfloat16().requires_grad_()
+    _QkvAttn.apply(leaf.detach(), window, half)                       # the rotation's tables
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            qkv = leaf * 1.0
+            before = qkv.detach().clone()
+            m0 = _held()
+            o = _QkvAttn.apply(qkv, window, half)
+            assert torch.equal(qkv, before)
+            kept = _held() - m0
+            size = lambda t: t.numel() * t.element_size()
+            assert kept <= size(o) + grad * (size(qkv) + 2 * 8 * 500 * 4) + 4 * 512
+            del qkv, before, o
+
+
+def test_light_layer_keeps_one_packed_array():
+    """The attention half keeps the norm's output, one packed array, the attention's output and its result."""
+    from memarch_b200.models.blocks import LightBlock
+    from memarch_b200.ops import layer
+    M, d = 2 * 512, 512
+    with torch.device("cuda"):
+        b = LightBlock(d, 8)
+    x = torch.randn(2, 512, d, device="cuda", requires_grad=True)
+    run = lambda: layer.attn_half(x, None, b.n1.weight, b.qkv.weight, b.o.weight, 1e-6, 0, False)
+    run()                                                             # the weights' bf16 copies
+    m0 = _held()
+    out = run()
+    kept = _held() - m0
+    assert len(out) == 2 and kept <= (2 + 6 + 2 + 2) * M * d + (8 + 1) * M * 4 + 8 * 512
+
+
 # ------------------------------------------------------------------------------------------------ light layer halves
 @pytest.mark.parametrize("d,B,T,window,blk,half,defer", [(128, 2, 129, 64, (), False, True), (256, 1, 257, 2048, ("relu2",), False, False), (64, 3, 100, 7, (), True, False),
                                                          (128, 1, 600, 2048, (), False, True), (192, 2, 300, 128, ("relu2",), True, True)])
