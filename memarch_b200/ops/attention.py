@@ -4,9 +4,9 @@ Reference behaviour: `F.scaled_dot_product_attention(rope(q), rope(k), v, is_cau
 window (full.py:156-157); block-masked window attention `kv <= q and q - kv < window` otherwise (FlexAttention with
 an O(T) block list, full2.py:153-181; two-block variants lm.py:448-554).
 
-GPU body, head dim 64: the own tcgen05 kernels on the packed projections (`_QkvAttn`, `csrc/attn_fwd.cu`,
-`csrc/attn_bwd.cu`: q and k rotated, v read in place, gradients written rotated back into the packed layout).  Other head
-dims, or `MEMARCH_ATTN=lib`: `rope_qk` (rotation of the q and k thirds of the packed qkv activations, `rope_merge_bwd`
+GPU body, head dim 64, where `own_core` says so: the own tcgen05 kernels on the packed projections (`_QkvAttn`, `csrc/attn_fwd.cu`,
+`csrc/attn_bwd.cu`: q and k rotated, v read in place, gradients written rotated back into the packed layout).  Otherwise
+`rope_qk` (rotation of the q and k thirds of the packed qkv activations, `rope_merge_bwd`
 packs and rotates the three gradients back in one pass) around the library flash kernel.
 """
 from __future__ import annotations
@@ -19,9 +19,9 @@ import torch.nn.functional as F
 from . import _ext, ref
 from .basic import dense
 
-ATTN_CORE = os.environ.get("MEMARCH_ATTN", "own")
+ATTN_CORE = os.environ.get("MEMARCH_ATTN", "auto")             # auto | own | lib: see `own_core`
 OWN_WINDOW_EVAL = os.environ.get("MEMARCH_ATTN_EVAL", "own") == "own"
-OWN_CAUSAL_T = 512                                            # plain causal texts up to this length: see `attention`
+OWN_CAUSAL_T = 512                                            # plain causal texts up to this length: see `own_core`
 OWN_BWD = os.environ.get("MEMARCH_ATTN_BWD", "own") == "own"
 WINDOW_BODY = os.environ.get("MEMARCH_WINDOW", "flash")        # library body of windowed attention with backward: flash | block
 
@@ -179,17 +179,28 @@ def _flash_window(q, k, v, window):
     return _lib_window(q, k, v, window)
 
 
+def own_core(T, windowed, no_grad):
+    """Whether head-dim-64 attention runs on the own kernels.  `MEMARCH_ATTN=own`: always.  `lib`: only windows without a backward
+    pass, and those only with `MEMARCH_ATTN_EVAL=own` (the default).  `auto`, the default: windows and short causal texts, but windows
+    without a backward pass as `MEMARCH_ATTN_EVAL` says."""
+    # Windows, forward + backward: 2 x 16 384 words, 16 heads, window 256: 700 us against 1221 for the library flash kernel; 4 x
+    # 4096, window 1024: 635 against 1242.  Short causal texts: 8 x 512, 8 heads: 90 against 157; 16 x 256, 12 heads: 102
+    # against 144.  On longer causal texts the library core is still ahead (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16
+    # heads: 1222 against 943).
+    if ATTN_CORE == "own":
+        return True
+    if windowed and no_grad:
+        return OWN_WINDOW_EVAL
+    return ATTN_CORE != "lib" and (windowed or T <= OWN_CAUSAL_T)
+
+
 def attention(qkv, window=None, rope_half=False, qk_norm=False):
     """qkv (B,T,3,H,hd) -> (B,T,H·hd).  `window` None or >= T means plain causal."""
     B, T, _, H, hd = qkv.shape
     win = None if (window is None or window >= T) else int(window)
     if _ext.use_cuda(qkv) and qkv.dtype == torch.bfloat16 and not qk_norm and hd % 8 == 0:
         no_grad = not (torch.is_grad_enabled() and qkv.requires_grad)
-        # The own kernels serve windows (forward + backward, 2 x 16 384 words, 16 heads, window 256: 700 us against 1221 for the
-        # library flash kernel; 4 x 4096, window 1024: 635 against 1242) and short causal texts (8 x 512, 8 heads: 90
-        # against 157; 16 x 256, 12 heads: 102 against 144).  On longer causal texts the library core is still ahead
-        # (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16 heads: 1222 against 943).
-        own = (ATTN_CORE == "own" and (win is not None or T <= OWN_CAUSAL_T)) or (win is not None and no_grad and OWN_WINDOW_EVAL)
+        own = own_core(T, win is not None, no_grad)
         if hd == 64 and own and (no_grad or OWN_BWD):
             return _QkvAttn.apply(dense(qkv.detach() if no_grad else qkv), win or 0, rope_half)
         q, k, v = _RopeSplit.apply(qkv, rope_half)

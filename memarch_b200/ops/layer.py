@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from . import _ext, basic
-from .attention import ATTN_CORE, OWN_BWD, OWN_CAUSAL_T, rope_tables
+from .attention import OWN_BWD, own_core, rope_tables
 
 
 def _trained(w):
@@ -32,10 +32,10 @@ def _common(x, nw, ws):
 
 
 def attn_half_ok(x, pending, nw, wqkv, wo, heads, window):
-    """Head dim 64 and lengths that the own attention kernels serve (see `ops.attention.attention`)."""
+    """Head dim 64 and lengths that the own attention kernels serve (see `ops.attention.own_core`)."""
     B, T, d = x.shape
-    windowed = window is not None and window < T
-    return (d == heads * 64 and ATTN_CORE == "own" and (windowed or T <= OWN_CAUSAL_T) and (OWN_BWD or not torch.is_grad_enabled())
+    no_grad = not torch.is_grad_enabled()
+    return (d == heads * 64 and own_core(T, window is not None and window < T, no_grad) and (OWN_BWD or no_grad)
             and wqkv.shape == (3 * d, d) and wo.shape == (d, d) and _common(x, nw, (wqkv, wo))
             and (pending is None or (pending.dtype == torch.bfloat16 and pending.shape == x.shape)))
 

@@ -591,6 +591,26 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
     loop.device_status(tr_cpu)                                    # CPU runs have no status words
 
 
+def test_attention_core_switches(monkeypatch):
+    """MEMARCH_ATTN=own puts every attention of head dim 64 on the own kernels, lib none but evaluation windows, and
+    MEMARCH_ATTN_EVAL decides about those in the default and the lib setting."""
+    import importlib
+    attn = importlib.import_module("memarch_b200.ops.attention")
+    every = [(T, w, g) for T in (64, 512, 513, 4096) for w in (False, True) for g in (False, True)]
+    for core in ("auto", "own", "lib"):
+        for ev in (True, False):
+            monkeypatch.setattr(attn, "ATTN_CORE", core)
+            monkeypatch.setattr(attn, "OWN_WINDOW_EVAL", ev)
+            for T, windowed, no_grad in every:
+                if core == "own":
+                    want = True
+                elif windowed and no_grad:
+                    want = ev
+                else:
+                    want = core == "auto" and (windowed or T <= attn.OWN_CAUSAL_T)
+                assert attn.own_core(T, windowed, no_grad) is want, (core, ev, T, windowed, no_grad)
+
+
 @pytest.mark.parametrize("word", ["gemm_status", "attn_status_read", "attn_bwd_status_read"])
 def test_loop_reads_every_kernel_status_word(monkeypatch, word):
     """Each family of kernels with bounded waits has a status word of its own, asked for on the trainer's device; any of them stops
