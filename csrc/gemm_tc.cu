@@ -83,6 +83,9 @@ __device__ __forceinline__ float silu_f(float x) {
   const float h = 0.5f * x;
   return fmaf(h, tanh_approx(h), h);
 }
+// sigmoid to a few units of fp32's last place wherever it is: the derivative multiplies by it alone, and for a strongly negative
+// gate (tanh(x / 2) + 1) / 2 leaves nothing but the rounding of the tanh
+__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // Drain one accumulator tile (this warp's 32 TMEM lanes x 256 columns) through the fused epilogue to global memory.
 // `row_l` = this thread's row inside M-segment `seg`; `taddr` = TMEM address of the warp's lanes, column 0 of the tile.
@@ -738,9 +741,7 @@ __device__ __forceinline__ void epilogue_tile3(const GemmParams& p, const CUtens
           for (int q = 0; q < 4; ++q) {
             const float2 gg = unpack_bf16(wg[q]), uv = unpack_bf16(wu[q]);
             const float d0 = __uint_as_float(r[32 * hf + 8 * j + 2 * q]), d1 = __uint_as_float(r[32 * hf + 8 * j + 2 * q + 1]);
-            // sigmoid through the hardware tanh (one special-function instruction, no division): with one epilogue
-            // warp per scheduler the dependent chain of exp + IEEE division per element was what bound this epilogue
-            const float s0 = fmaf(tanh_approx(0.5f * gg.x), 0.5f, 0.5f), s1 = fmaf(tanh_approx(0.5f * gg.y), 0.5f, 0.5f);
+            const float s0 = sigmoid_f(gg.x), s1 = sigmoid_f(gg.y);
             og[q] = pack_bf16(d0 * uv.x * s0 * (1.f + gg.x * (1.f - s0)), d1 * uv.y * s1 * (1.f + gg.y * (1.f - s1)));
             ou[q] = pack_bf16(d0 * gg.x * s0, d1 * gg.y * s1);
           }
@@ -841,13 +842,13 @@ __device__ __forceinline__ void epilogue_act(const GemmParams& p, const CUtensor
       const uint32_t wg[4] = {ug[j].x, ug[j].y, ug[j].z, ug[j].w};
       uint32_t o0[4], o1[4];
       if (ACT == ACT_SWIGLU) {
-        // acc = dh; dg = dh * u * s * (1 + g * (1 - s)), du = dh * g * s with s = sigmoid(g) through the hardware tanh
+        // acc = dh; dg = dh * u * s * (1 + g * (1 - s)), du = dh * g * s with s = sigmoid(g)
         const uint32_t wu[4] = {uu[j].x, uu[j].y, uu[j].z, uu[j].w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float2 gg = unpack_bf16(wg[q]), uv = unpack_bf16(wu[q]);
           const float d0 = __uint_as_float(r[8 * j + 2 * q]), d1 = __uint_as_float(r[8 * j + 2 * q + 1]);
-          const float s0 = fmaf(tanh_approx(0.5f * gg.x), 0.5f, 0.5f), s1 = fmaf(tanh_approx(0.5f * gg.y), 0.5f, 0.5f);
+          const float s0 = sigmoid_f(gg.x), s1 = sigmoid_f(gg.y);
           o0[q] = pack_bf16(d0 * uv.x * s0 * (1.f + gg.x * (1.f - s0)), d1 * uv.y * s1 * (1.f + gg.y * (1.f - s1)));
           o1[q] = pack_bf16(d0 * gg.x * s0, d1 * gg.y * s1);
         }

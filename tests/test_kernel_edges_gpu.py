@@ -617,6 +617,33 @@ def test_gemm_activation_backward(M, H, K, b_mn):
     assert _rel(gemm(dy, wm, b_mn=b_mn, epi=2, aux=p2), dh * 2 * p2.double().relu()) < 4e-3
 
 
+@pytest.mark.parametrize("direct", [False, True])
+@pytest.mark.parametrize("gate", [-3.0, -6.0, -9.0, -20.0, -80.0, -200.0, 9.0, 200.0])
+def test_swiglu_backward_of_extreme_gates(gate, direct):
+    """The sigmoid's relative error stays at that of fp32 where it is small: grouped (experts) and plain products, both epilogues."""
+    from memarch_b200.ops import _ext, gemm
+    g = torch.Generator(device="cuda").manual_seed(1)
+    E, M, H, K = 2, 300, 72, 64
+    dy, w = torch.randn(E, M, K, device="cuda", generator=g).bfloat16(), (torch.randn(E, H, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    pre = torch.randn(E, M, 2 * H, device="cuda", generator=g) * 0.2
+    pre[..., :H] += gate
+    pre = pre.bfloat16()
+    dh = dy.double() @ w.double().mT
+    a, u = pre.double().chunk(2, -1)
+    s = a.sigmoid()
+    want = torch.cat([dh * u * s * (1 + a * (1 - s)), dh * a * s], -1)
+    if direct:
+        _ext.C().gemm_set_debug(8, 0)
+    try:
+        got = gemm(dy, w, groups=E, epi=5, aux=pre), gemm(dy[0].contiguous(), w[0].contiguous(), epi=5, aux=pre[0].contiguous())
+    finally:
+        _ext.C().gemm_set_debug(0, 0)
+    for o, r in zip(got, (want, want[0])):
+        for c, t in zip(o.double().chunk(2, -1), r.chunk(2, -1)):
+            # one rounding to bf16 (2^-9) and three of fp32; results below bf16's normal range (2^-126) count as zero
+            assert (c - t).norm() < 3e-3 * t.norm() + 1e-30
+
+
 # ------------------------------------------------------------------------------------------------ head
 @pytest.mark.parametrize("N,V,d,chunk", [(1, 16, 16, 4096), (300, 1000, 24, 128), (513, 264, 136, 512), (40, 104, 64, 7)])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
