@@ -89,12 +89,13 @@ std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, c10::optional<torch::T
 std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, c10::optional<torch::Tensor> dh, torch::Tensor h, torch::Tensor n, torch::Tensor rstd,
                                          torch::Tensor qkv, torch::Tensor o, torch::Tensor lse, torch::Tensor nw,
                                          torch::Tensor wqkv, torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window,
-                                         bool want_lo, bool grad_f32);
+                                         bool want_lo, bool grad_f32, pybind11::object offer);
 std::vector<torch::Tensor> ffn_half_fwd(torch::Tensor h, torch::Tensor a, torch::Tensor nw, double eps, torch::Tensor wup, torch::Tensor wdown,
                                         bool swiglu, bool add_out);
 std::vector<torch::Tensor> ffn_half_bwd(torch::Tensor dy, c10::optional<torch::Tensor> dx2, torch::Tensor x2, torch::Tensor n, torch::Tensor rstd,
                                         torch::Tensor pre, torch::Tensor hid, torch::Tensor nw, torch::Tensor wup, torch::Tensor wdown,
-                                        bool swiglu, bool grad_f32);
+                                        bool swiglu, bool grad_f32,
+                                        pybind11::object offer);
 int64_t attn_bwd_status_read(int64_t device);
 torch::Tensor embed_sum_fwd(torch::Tensor emb, torch::Tensor x, c10::optional<torch::Tensor> cand, c10::optional<torch::Tensor> sel,
                             c10::optional<torch::Tensor> phr, c10::optional<torch::Tensor> pidx);

@@ -3,7 +3,9 @@
 //   attention half:    h = x (+ pending), n = rmsnorm(h), qkv = n Wqkv^T, o = attention(qkv), a = o Wo^T
 //   feed-forward half: x2 = h + a, n2 = rmsnorm(x2), y = act(n2 Wup^T) Wdown^T (, out = x2 + y)
 // Backward sums the gradient that reaches the residual stream past the half inside the norm's own pass.  Weight gradients leave
-// in fp32 (`grad_f32`: what an fp32 weight's .grad wants) or in bf16 (what the optimizer takes inside backward).
+// in fp32 (`grad_f32`: what an fp32 weight's .grad wants) or in bf16 (what the optimizer takes inside backward: `offer(i, gradient)`,
+// i counting the weights in argument order, is called for each as soon as it and the last product that reads the weight are
+// enqueued, so that its exchange or step runs under what follows).
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -23,6 +25,12 @@ torch::Tensor attn_qkv_bwd(torch::Tensor dout, torch::Tensor o, torch::Tensor ls
 
 typedef c10::optional<torch::Tensor> Opt;
 static bool has(const Opt& t) { return t.has_value() && t->defined(); }
+// hands a gradient to `offer`, which takes it, or returns it
+static torch::Tensor handed(const pybind11::object& offer, int i, torch::Tensor g) {
+  if (offer.is_none()) return g;
+  offer(i, g);
+  return torch::Tensor();
+}
 enum { EPI_NONE = 0, EPI_RELU2 = 1, EPI_DRELU2 = 2, EPI_SWIGLU = 3, EPI_DSWIGLU = 5 };
 
 static torch::Tensor project(const torch::Tensor& a, const torch::Tensor& b) {                     // a b^T
@@ -65,15 +73,15 @@ std::vector<torch::Tensor> attn_half_fwd(torch::Tensor x, Opt pending, torch::Te
 std::vector<torch::Tensor> attn_half_bwd(torch::Tensor da, Opt dh, torch::Tensor h, torch::Tensor n, torch::Tensor rstd, torch::Tensor qkv,
                                          torch::Tensor o, torch::Tensor lse, torch::Tensor nw, torch::Tensor wqkv,
                                          torch::Tensor wo, torch::Tensor cos, torch::Tensor sin, bool half, int64_t window, bool want_lo,
-                                         bool grad_f32) {
+                                         bool grad_f32, pybind11::object offer) {
   const c10::cuda::CUDAGuard guard(da.device());
   const int64_t M = h.size(0), d = h.size(1);
   const torch::Tensor g = rows(da);
   auto dout = dgrad(g, wo);
-  auto dwo = wgrad(g, o.view({M, d}), grad_f32);
+  auto dwo = handed(offer, 1, wgrad(g, o.view({M, d}), grad_f32));
   auto dqkv = attn_qkv_bwd(dout, o, lse, qkv, cos, sin, half, window).view({M, 3 * d});
   auto dn = dgrad(dqkv, wqkv);
-  auto dwqkv = wgrad(dqkv, n, grad_f32);
+  auto dwqkv = handed(offer, 0, wgrad(dqkv, n, grad_f32));
   auto r = rmsnorm_bwd(dn, h, nw, rstd, has(dh) ? Opt(rows(*dh)) : Opt(), want_lo);
   return {r[0], r[2], r[1], dwqkv, dwo};
 }
@@ -93,7 +101,8 @@ std::vector<torch::Tensor> ffn_half_fwd(torch::Tensor h, torch::Tensor a, torch:
 
 // dy (B,T,d) bf16 (or, with `add_out`, the fp32 gradient of x2 + y); dx2 (B,T,d) fp32 or none.  -> dh (M,d), da (M,d) bf16, d nw, d wup, d wdown
 std::vector<torch::Tensor> ffn_half_bwd(torch::Tensor dy, Opt dx2, torch::Tensor x2, torch::Tensor n, torch::Tensor rstd, torch::Tensor pre,
-                                        torch::Tensor hid, torch::Tensor nw, torch::Tensor wup, torch::Tensor wdown, bool swiglu, bool grad_f32) {
+                                        torch::Tensor hid, torch::Tensor nw, torch::Tensor wup, torch::Tensor wdown, bool swiglu, bool grad_f32,
+                                        pybind11::object offer) {
   const c10::cuda::CUDAGuard guard(dy.device());
   torch::Tensor g = rows(dy);
   Opt through = has(dx2) ? Opt(rows(*dx2)) : Opt();
@@ -103,9 +112,9 @@ std::vector<torch::Tensor> ffn_half_bwd(torch::Tensor dy, Opt dx2, torch::Tensor
     g = g.to(torch::kBFloat16);
   }
   auto dpre = gemm(g, wdown, c10::nullopt, c10::nullopt, pre, false, true, false, swiglu ? EPI_DSWIGLU : EPI_DRELU2, false, 1, c10::nullopt, 0);
-  auto dwd = wgrad(g, hid, grad_f32);
+  auto dwd = handed(offer, 1, wgrad(g, hid, grad_f32));
   auto dn = dgrad(dpre, wup);
-  auto dwu = wgrad(dpre, n, grad_f32);
+  auto dwu = handed(offer, 0, wgrad(dpre, n, grad_f32));
   auto r = rmsnorm_bwd(dn, x2, nw, rstd, through, true);
   return {r[0], r[2], r[1], dwu, dwd};
 }

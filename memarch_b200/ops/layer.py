@@ -47,6 +47,18 @@ def ffn_half_ok(h, a, nw, wup, wdown, swiglu):
             and (basic.FUSE_DSWIGLU or not swiglu) and _common(h, nw, (wup, wdown)))
 
 
+def _taker(ws):
+    """(what the native call hands each weight's gradient to as soon as it is enqueued, the gradients it did not keep); without a
+    taker of gradients (None, None): the call returns them."""
+    if basic.WEIGHT_GRAD_SINK is None:
+        return None, None
+    left = [None, None]
+
+    def offer(i, g):
+        left[i] = basic.offer_grad(ws[i], g)
+    return offer, left
+
+
 class _AttnHalf(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, pending, nw, wqkv, wo, eps, window, half):
@@ -68,13 +80,12 @@ class _AttnHalf(torch.autograd.Function):
                 return (None,) * 8
             da = torch.zeros(ctx.shape, device=dh.device, dtype=torch.bfloat16)
         cos, sin = rope_tables(ctx.shape[1], 64, h.device)
-        f32 = basic.WEIGHT_GRAD_SINK is None
-        dx, lo, dnw, dwqkv, dwo = _ext.C().attn_half_bwd(da, dh, h, n, rstd, qkv, o, lse, nw, sq, so, cos, sin, ctx.half, ctx.window,
-                                                         ctx.has_pending, f32)
+        offer, left = _taker(ctx.ws)
+        dx, lo, dnw, *dws = _ext.C().attn_half_bwd(da, dh, h, n, rstd, qkv, o, lse, nw, sq, so, cos, sin, ctx.half, ctx.window,
+                                                   ctx.has_pending, offer is None, offer)
         _count(dx, 8 * dx.shape[1], 9)
-        wqkv, wo = ctx.ws
         return (dx.view(ctx.shape), lo.view(ctx.shape) if ctx.has_pending else None, dnw.to(nw.dtype),
-                basic.offer_grad(wqkv, dwqkv), basic.offer_grad(wo, dwo), None, None, None)
+                *(left or dws), None, None, None)
 
 
 class _FFNHalf(torch.autograd.Function):
@@ -96,12 +107,11 @@ class _FFNHalf(torch.autograd.Function):
             if dx2 is None:
                 return (None,) * 8
             dy = torch.zeros(ctx.shape, device=x2.device, dtype=torch.bfloat16)
-        f32 = basic.WEIGHT_GRAD_SINK is None
-        dh, da, dnw, dwu, dwd = _ext.C().ffn_half_bwd(dy, dx2, x2, n, rstd, pre, hid, nw, su, sd, ctx.swiglu, f32)
+        offer, left = _taker(ctx.ws)
+        dh, da, dnw, *dws = _ext.C().ffn_half_bwd(dy, dx2, x2, n, rstd, pre, hid, nw, su, sd, ctx.swiglu, offer is None, offer)
         wup, wdown = ctx.ws
         _count(dh, 2 * (wup.shape[0] + wdown.shape[1]), 6)
-        return (dh.view(ctx.shape), da.view(ctx.shape), dnw.to(nw.dtype), basic.offer_grad(wup, dwu), basic.offer_grad(wdown, dwd),
-                None, None, None)
+        return dh.view(ctx.shape), da.view(ctx.shape), dnw.to(nw.dtype), *(left or dws), None, None, None
 
 
 def _count(x, width, launches):

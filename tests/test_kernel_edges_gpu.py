@@ -534,6 +534,33 @@ def test_light_layer_halves_match_single_ops(monkeypatch, d, B, T, window, blk, 
         assert a.dtype == c.dtype and _rel(a, c) < 6e-3
 
 
+@pytest.mark.parametrize("keeps", [True, False])
+def test_light_layer_hands_gradients_over_early(monkeypatch, keeps):
+    """A weight's gradient reaches the optimizer before the rest of its half is enqueued: between two offers the native call
+    allocates what it goes on with.  A gradient that the optimizer declines goes to `.grad`."""
+    from memarch_b200.models.blocks import LightBlock
+    from memarch_b200.ops import basic
+    with torch.device("cuda"):
+        b = LightBlock(128, 2)
+    names = {id(p): n for n, p in b.named_parameters()}
+    seen = []
+
+    def sink(w, g):
+        seen.append((names[id(w)], torch.cuda.memory_stats()["allocation.all.allocated"]))
+        return keeps
+    x = torch.randn(2, 200, 128, device="cuda", requires_grad=True)
+    monkeypatch.setattr(basic, "WEIGHT_GRAD_SINK", sink)
+    y = b(x, 64)
+    y.backward(torch.ones_like(y))
+    end = torch.cuda.memory_stats()["allocation.all.allocated"]
+    assert [n for n, _ in seen] == ["down.weight", "up.weight", "o.weight", "qkv.weight"]
+    at = [c for _, c in seen] + [end]
+    # after the offer of `down`: the input gradient and that of `up`; of `up`: the norm's; of `o`: the packed gradient, statistics,
+    # input gradient and that of `qkv`; of `qkv`: the norm's
+    assert [q - p >= k for p, q, k in zip(at, at[1:], (2, 2, 4, 2))] == [True] * 4
+    assert all((p.grad is None) == keeps for n, p in b.named_parameters() if n in dict(seen))
+
+
 def test_light_layer_halves_leave_other_cases_alone():
     """Frozen weights, a stream without a gradient, bf16 streams and short batches stay on the single ops."""
     from memarch_b200.models.blocks import LightBlock
