@@ -459,17 +459,17 @@ def test_attention_keeps_one_packed_array(window, half):
     from memarch_b200.ops.attention import _QkvAttn
     leaf = torch.randn(2, 500, 3, 8, 64, device="cuda").bfloat16().requires_grad_()
     _QkvAttn.apply(leaf.detach(), window, half)                       # the rotation's tables
+    size = lambda t: t.numel() * t.element_size()
     for grad in (False, True):
         with torch.set_grad_enabled(grad):
+            m0 = _held()
             qkv = leaf * 1.0
             before = qkv.detach().clone()
-            m0 = _held()
             o = _QkvAttn.apply(qkv, window, half)
             assert torch.equal(qkv, before)
-            kept = _held() - m0
-            size = lambda t: t.numel() * t.element_size()
-            assert kept <= size(o) + grad * (size(qkv) + 2 * 8 * 500 * 4) + 4 * 512
-            del qkv, before, o
+            del qkv, before                                           # the caller is done with the projections
+            assert _held() - m0 <= size(o) + grad * (size(leaf) + 2 * 8 * 500 * 4) + 4 * 512
+            del o
 
 
 def test_light_layer_keeps_one_packed_array():
