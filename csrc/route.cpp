@@ -36,10 +36,11 @@ std::vector<torch::Tensor> route_fwd(torch::Tensor x, torch::Tensor w, torch::Te
   auto counts = torch::empty({E}, i);
   const int64_t nb = route_blocks(a.N);
   TORCH_CHECK(N > 0, "route: no tokens");
-  auto work_i = torch::empty({nb * (E + 1)}, i), psum = torch::empty({nb * E}, f);
+  auto work_i = torch::empty({(nb + 1) * (E + 1)}, i), psum = torch::empty({(nb + 1) * E}, f);
   a.wt = wt.data_ptr<float>(); a.wtab = wtab.data_ptr<float>(); a.probs = probs.data_ptr<float>(); a.aux = aux.data_ptr<float>();
   a.dropped = dropped.data_ptr<float>(); a.aux_grad = aux_grad.data_ptr<float>(); a.table = i64(table); a.flat_idx = i64(flat_idx);
   a.top_e = i64(top_e); a.counts = counts.data_ptr<int>(); a.hist = work_i.data_ptr<int>(); a.n_real = a.hist + nb * E; a.psum = psum.data_ptr<float>();
+  if (nb > ROUTE_SCAN) { a.total = a.n_real + nb; a.ps = a.psum + nb * E; }
   route_fwd_launch(a);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   return {wt, wtab, aux, probs, table, flat_idx, dropped, counts, top_e, aux_grad};

@@ -1,10 +1,11 @@
-// The router of an expert layer in two launches forward and three backward.
+// The router of an expert layer in two launches forward (three for more than 32 768 tokens) and three backward.
 //
 // Forward 1 (route_fwd_kernel): logits = x W^T in fp32 from the bf16 rows, softmax, top-k by probability (ties: smaller
 // expert first), budget k_tok, renormalised weights, and per block of 32 tokens the number of choices and the sum of
 // probabilities of every expert.
 // Forward 2 (route_place_kernel): choices in (token, choice) order take the next free place of their expert, places beyond C
-// drop; a block's first free places are the sums of the earlier blocks' numbers.  Fills the slot table, its inverse,
+// drop; a block's first free places are the sums of the earlier blocks' numbers (taken by each block, or from ROUTE_SCAN blocks on
+// by route_scan_kernel once).  Fills the slot table, its inverse,
 // the combine weights of the places, and (first block) filled places, dropped share and the Switch auxiliary loss
 //   aux = E * sum_e (choices of e / all choices) * (mean probability of e over the real tokens).
 // Backward 1 (route_dx_kernel): gradient of the logits from the gradients of the weights, of the place weights and of aux, and
@@ -145,6 +146,38 @@ __global__ void __launch_bounds__(ROUTE_TOK / TOK * 32) route_fwd_kernel(RouteAr
   if (threadIdx.x == 0) a.n_real[blockIdx.x] = real_sh;
 }
 
+// block = one expert: its numbers of choices per block become the places taken before each block; totals beside them
+__global__ void __launch_bounds__(256) route_scan_kernel(RouteArgs a, int nb) {
+  __shared__ int sums[256];
+  __shared__ float psums[256];
+  const int e = blockIdx.x, E = a.E, tid = threadIdx.x, per = (nb + 255) / 256;
+  const int b0 = min(nb, tid * per), b1 = min(nb, b0 + per);
+  int s = 0;
+  float p = 0.f;
+  for (int b = b0; b < b1; ++b) { s += a.hist[(long long)b * E + e]; p += a.psum[(long long)b * E + e]; }
+  sums[tid] = s;
+  psums[tid] = p;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {
+    const int v = tid >= o ? sums[tid - o] : 0;
+    __syncthreads();
+    sums[tid] += v;
+    __syncthreads();
+  }
+  int run = sums[tid] - s;
+  for (int b = b0; b < b1; ++b) {
+    const int h = a.hist[(long long)b * E + e];
+    a.hist[(long long)b * E + e] = run;
+    run += h;
+  }
+  if (tid == 0) {
+    float t = 0.f;
+    for (int i = 0; i < 256; ++i) t += psums[i];
+    a.ps[e] = t;
+    a.total[e] = sums[255];
+  }
+}
+
 __global__ void __launch_bounds__(256) route_place_kernel(RouteArgs a) {
   __shared__ int base[ROUTE_E], total[ROUTE_E];
   __shared__ float ps[ROUTE_E];
@@ -157,7 +190,9 @@ __global__ void __launch_bounds__(256) route_place_kernel(RouteArgs a) {
   __syncthreads();
   // sums over the blocks: a thread takes one expert and every (256 / E)-th block
   const int lanes = blockDim.x / E;
-  if (tid < lanes * E) {
+  if (a.total) {
+    for (int e = tid; e < E; e += blockDim.x) { base[e] = a.hist[(long long)blockIdx.x * E + e]; total[e] = a.total[e]; ps[e] = a.ps[e]; }
+  } else if (tid < lanes * E) {
     const int e = tid % E;
     int before = 0, all = 0;
     float p = 0.f;
@@ -367,6 +402,7 @@ void route_fwd_launch(const RouteArgs& a) {
   const size_t smem = (size_t)ROUTE_TOK * a.E * 4;
   if (a.E <= 16) route_fwd_kernel<4><<<nb, ROUTE_TOK / 4 * 32, smem, a.stream>>>(a);
   else route_fwd_kernel<8><<<nb, ROUTE_TOK / 8 * 32, smem, a.stream>>>(a);
+  if (a.total) route_scan_kernel<<<a.E, 256, 0, a.stream>>>(a, nb);
   route_place_kernel<<<nb, 256, 0, a.stream>>>(a);
 }
 void route_bwd_launch(const RouteArgs& a) {

@@ -26,6 +26,8 @@ struct RouteArgs {
   int* hist;                   // workspace (blocks, E)
   float* psum;                 // workspace (blocks, E)
   int* n_real;                 // workspace (blocks)
+  int* total;                  // workspace (E), or null: every block of route_place_kernel adds up the blocks' numbers itself
+  float* ps;                   // workspace (E) beside it
   // backward (null: no gradient arrives there)
   const float *d_wt, *d_wtab, *d_aux, *d_probs;
   float* dl;                   // workspace (N, E): gradient of the logits
@@ -35,6 +37,9 @@ struct RouteArgs {
   int dw_runs, dw_run;         // runs of tokens and their length: route_dw_runs()
   cudaStream_t stream;
 };
+// Blocks from which on their numbers are added up once, in a kernel of their own, instead of by every block: the latter is quadratic
+// in the tokens.
+constexpr int ROUTE_SCAN = 1024;
 inline int route_blocks(int N) { return (N + ROUTE_TOK - 1) / ROUTE_TOK; }
 void route_fwd_launch(const RouteArgs& a);
 int route_dw_runs(int N, int d, int E, int& run);

@@ -235,6 +235,28 @@ def test_route_and_slot_fused(N, d, E, k, C):
     assert _rel(xg.grad.cpu(), xc.grad) < 4e-3 and _rel(wg.grad.cpu(), wc.grad) < 1e-4
 
 
+@pytest.mark.parametrize("N,E,k,C", [(32768, 8, 2, 9000), (32769, 8, 2, 8000), (70001, 64, 4, 4000), (40000, 128, 8, 2500), (33000, 1, 1, 30000)])
+def test_route_places_of_many_tokens(N, E, k, C):
+    """Both sides of the line from which on the blocks' numbers are added up once: places, filled counts, dropped share and the auxiliary
+    loss from the kernel's own choices."""
+    from memarch_b200 import ops
+    from memarch_b200.ops import ref
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(N, 16, device="cuda", generator=g).bfloat16()
+    w = torch.randn(E, 16, device="cuda", generator=g) * 0.5
+    real, k_tok = torch.rand(N, device="cuda", generator=g) > 0.2, torch.randint(0, k + 1, (N,), device="cuda", generator=g)
+    wt, table, wtab, flat, aux, dropped, probs, counts = ops.route_and_slot(x, w, real, k_tok, k, E, C, want_counts=True)
+    top = probs.topk(k, 1).indices
+    keep = torch.arange(k, device="cuda")[None] < k_tok[:, None]
+    e_flat = torch.where(keep, top, torch.full_like(top, E))
+    t2, _, f2, d2 = ref.moe_slots(e_flat.cpu(), wt.detach().cpu(), E, C)
+    assert torch.equal(table.cpu(), t2) and torch.equal(flat.cpu(), f2) and abs(float(dropped) - float(d2)) < 1e-6
+    cnt = torch.bincount(e_flat[keep], minlength=E)
+    assert torch.equal(counts.long(), cnt.clamp(max=C))
+    want = E * (cnt.double() / cnt.sum() * (probs.double() * real[:, None]).sum(0) / real.sum()).sum()
+    assert abs(float(aux) - float(want)) < 1e-4 * float(want)
+
+
 @pytest.mark.parametrize("N,d,E", [(8192, 2048, 8), (5000, 264, 16), (40000, 512, 128)])
 def test_router_gradients_repeat(N, d, E):
     """The router weight's gradient is summed over the tokens in a fixed order: the same call gives the same bits.  The last size
