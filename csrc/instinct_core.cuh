@@ -872,6 +872,16 @@ static __global__ void instinct_lag_rows_select(float* __restrict__ cs, float* _
   }
 }
 
+// out[r] = sum of the `cuts` parts of row r, in a fixed order; a warp per row
+static __global__ void __launch_bounds__(256) instinct_fold_cuts(const float* __restrict__ part, float* __restrict__ out, long long rows, int cuts) {
+  const long long r = (blockIdx.x * 256ll + threadIdx.x) >> 5;
+  if (r >= rows) return;
+  float s = 0.f;
+  for (int i = threadIdx.x & 31; i < cuts; i += 32) s += part[r * cuts + i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) out[r] = s;
+}
+
 // Launch sequence; returns the number of kernels launched, or -1 when this weight cannot take the requested form
 // (nothing is launched then).  `cs` / `cs_ok`: lagged homeostasis state (previous step's second-axis mean squares and
 // the "all positive" flag), or null for the exact form.
@@ -917,9 +927,14 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   // dealt out in chunks of 256 elements: two or more for each of 148 x 16 warps (sums), four for each of 148 x 12 (update),
   // else filling and draining the rings costs more than the block-per-row form
   const bool s8_rows = aligned8 && ER * (a.C >> 8) >= 2 * 148 * 16, s8_chunks = aligned8 && ER * (a.C >> 8) >= 4 * 148 * 12;
-  // Kinds without column sums repeat bit for bit: whole rows, one per warp at least, else the block-per-row form.  (The others add
-  // to their columns from many blocks and do not repeat anyway.)
+  // Kinds without column sums repeat bit for bit: whole rows, one per warp at least; fewer rows are cut into `cuts` equal runs of
+  // chunks each, as many as the idle column sums' place holds, whose sums are added in a fixed order; else the block-per-row form.
+  // (The others add to their columns from many blocks and do not repeat anyway.)  2 M elements under one norm: 656 us with the
+  // block-per-row form.
   const bool by_rows = kind != 4 && kind != 5;
+  long long cuts = 1;
+  if (by_rows && s8_rows && ER < 148 * 16)
+    while ((a.C >> 8) % (2 * cuts) == 0 && ER * cuts < 148 * 16 && ER * 2 * cuts <= EC) cuts *= 2;
   constexpr size_t S8_SMEM = 216 * 1024;
   // launch `kern<S>` with the deepest ring that fits beside `head` bytes: T threads, `slots` 16-byte slots per stage
   auto s8_launch = [&](auto k12, auto k8, auto k6, auto k4, int T, int slots, size_t head, auto&&... args) {
@@ -935,6 +950,17 @@ inline int64_t instinct_launch(const InstinctArgs& a, int kind, float* scratch, 
   };
   auto stat_rows = [&](const float* colsum, float* out, float* absout) {
     const size_t smem = colsum ? Cb : 0;
+    if (cuts > 1 && ER * cuts >= 148 * 8) {              // by rows: no column scales
+      InstinctArgs c = a;
+      c.E = 1; c.R = ER * cuts; c.C = a.C / cuts;
+      s8_launch(instinct_stat_rows_s8<12>, instinct_stat_rows_s8<8>, instinct_stat_rows_s8<6>, instinct_stat_rows_s8<4>, 512,
+                (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2), 0, c, (const float*)nullptr, Rf, colA, absout ? colB : nullptr, c.C >> 8);
+      const int grid = (int)((ER + 7) / 8);
+      instinct_fold_cuts<<<grid, 256, 0, st>>>(colA, out, ER, (int)cuts);
+      if (absout) instinct_fold_cuts<<<grid, 256, 0, st>>>(colB, absout, ER, (int)cuts);
+      launches += absout ? 2 : 1;
+      return;
+    }
     if ((by_rows ? aligned8 && ER >= 148 * 16 : s8_rows) && smem + 4 * 512 * 4 * 16 <= S8_SMEM) {
       s8_launch(instinct_stat_rows_s8<12>, instinct_stat_rows_s8<8>, instinct_stat_rows_s8<6>, instinct_stat_rows_s8<4>, 512,
                 (a.g_bf16 ? 1 : 2) + (a.m_bf16 ? 1 : 2), smem, a, colsum, Rf, out, absout, by_rows ? a.C >> 8 : 1ll);
