@@ -274,10 +274,10 @@ def run_ours(args):
     def step_dev(s):
         losses.append(tr.step(store.batch(args.batch, args.seq), s))
 
-    n0, f0 = _ext.launch_count, _ext.gemm_flops
+    n0, f0 = _ext.launches(), _ext.gemm_flops
     sampler = ClockSampler(local) if rank == 0 else None
     ms, clocks = timed_loop(step_dev, args.steps, args.warmup, world, sampler)
-    per_step_launches = (_ext.launch_count - n0) / (args.steps + args.warmup)
+    per_step_launches = (_ext.launches() - n0) / (args.steps + args.warmup)
     # tensor-core work of this package's own GEMMs per step and GPU (nominal 2MNK; attention and the optimizer's
     # element-wise work are not in it), against the measured sustained cuBLAS rate when the driver wrote one
     gemm_tflop = (_ext.gemm_flops - f0) / (args.steps + args.warmup) / 1e12

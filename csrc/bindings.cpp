@@ -7,6 +7,7 @@ torch::Tensor gemm(torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor
                    int64_t groups, c10::optional<torch::Tensor> counts, int64_t count_mode);
 void gemm_set_debug(int64_t dbg, int64_t group_m);
 int gemm_status(int device);
+int64_t gemm_sum_launches();
 torch::Tensor gemm_peer(std::vector<int64_t> a_ptrs, int64_t seg_M, int64_t K, int64_t a_groups, int64_t a_pitch,
                         int64_t a_gs, int64_t a_g_off, torch::Tensor b, bool b_mn, c10::optional<torch::Tensor> out_local,
                         std::vector<int64_t> out_ptrs, int64_t out_ld, int64_t out_gs, int64_t out_g_off,
@@ -109,6 +110,7 @@ torch::Tensor moe_route_bwd(torch::Tensor probs, torch::Tensor top_e, torch::Ten
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &mb::gemm, "tcgen05 GEMM C = A * B^T (bf16, fp32 accumulate in TMEM)");
   m.def("gemm_status", &mb::gemm_status, "read and clear the GEMM status word (0 = ok)");
+  m.def("gemm_sum_launches", &mb::gemm_sum_launches, "kernels launched so far that add the parts of a cut contraction");
   m.def("gemm_set_debug", &mb::gemm_set_debug, "pair kernel: test / measurement bits and row-tile group size of the tile order",
         pybind11::arg("dbg") = 0, pybind11::arg("group_m") = 0);
   m.def("gemm_pair_on", &mb::gemm_pair_on);

@@ -3,9 +3,15 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <atomic>
+
 #include "gemm_api.h"
 
 namespace mb {
+
+// kernels that added the parts of cut contractions, since the library was loaded
+static std::atomic<int64_t> sum_launches{0};
+int64_t gemm_sum_launches() { return sum_launches.load(); }
 
 // torch binding.  a: (G?, M, K) or MN-major (G?, K, M); b: (G?, N, K) or MN-major (G?, K, N).
 torch::Tensor gemm(torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor> out_,
@@ -91,6 +97,7 @@ torch::Tensor gemm(torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor
   if (parts.defined()) {
     sum_parts_launch(parts.data_ptr<float>(), p.splits, O.data_ptr(), out_f32, accumulate, M, N, (int)O.stride(1), stream);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
+    ++sum_launches;
   }
   return out;
 }

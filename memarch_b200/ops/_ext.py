@@ -16,7 +16,7 @@ import torch
 _lock = threading.Lock()
 _mod = None
 _err = None
-launch_count = 0          # kernels of this package launched since process start (bench.py reports the delta)
+launch_count = 0          # kernels of this package launched since process start, as the ops count them: see `launches`
 gemm_flops = 0            # nominal 2·M·N·K of the tensor-core GEMMs issued through `ops.gemm` (padding places included)
 
 
@@ -74,6 +74,12 @@ def use_cuda(*tensors) -> bool:
 def count(n: int = 1):
     global launch_count
     launch_count += n
+
+
+def launches() -> int:
+    """Kernels of this package launched since process start: what the ops counted, and the second kernel of products whose
+    contraction was cut, which only the native side knows of."""
+    return launch_count + (_mod.gemm_sum_launches() if _mod is not None else 0)
 
 
 def count_flops(n: int):

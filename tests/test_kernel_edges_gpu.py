@@ -168,6 +168,15 @@ def test_gemm_split_contraction_repeats(M, N, K):
         assert all(torch.equal(call(), first) for _ in range(20))
 
 
+@pytest.mark.parametrize("K,kernels", [(1024, 1), (4096, 2)])
+def test_launches_of_split_products_are_counted(K, kernels):
+    from memarch_b200.ops import _ext, gemm
+    a, b = (torch.zeros(512, K, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    n = _ext.launches()
+    gemm(a, b)
+    assert _ext.launches() - n == kernels
+
+
 # ------------------------------------------------------------------------------------------------ narrow tiles
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 256), (257, 264, 128), (4095, 512, 520), (1001, 136, 64), (256, 1024, 2048), (9472, 256, 64), (513, 8, 16)])
 def test_gemm_narrow_tiles(M, N, K):
