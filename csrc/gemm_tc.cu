@@ -1473,9 +1473,12 @@ void sum_parts_launch(const float* parts, int splits, void* dst, int f32, int ac
   if (splits >= 8) go(std::integral_constant<int, 8>()); else go(std::integral_constant<int, 1>());
 }
 
-// How many runs to cut the contraction of one plain product into (1: none).  A product with fewer output tiles than
-// half of the 74 CTA pairs leaves the rest of the chip idle; every run costs an fp32 slab that a second kernel reads back and
-// adds up in run order, so a run keeps at least 8 k-blocks (512 of the contraction).
+// How many runs to cut the contraction of one plain product into (1: none).  A product with fewer output tiles than half of the
+// 74 CTA pairs leaves the rest of the chip idle.  A cut saves each pair kb - kb_split k-blocks of 64 (0.3 us each) and costs a second
+// launch and an fp32 slab per run and tile that is written and read back, 8 k-blocks and 0.45 per slab.  The line is measured
+// against the whole product as launch_gemm_seg runs it, with 128-column tiles where it takes them.  Us, (M, N, K), cut / whole:
+// (256, 256, 2048) 17.4 / 20.5; (1024, 512, 2048) 21.5 / 22.5; (1024, 1024, 3072) 27.6 / 26.6 and 4096 29.7 / 31.7; (4096, 512,
+// 2048) 27.7 / 22.5, 4096 35.8 / 34.8 and 8192 50 / 55; (1000, 256, 50304) 48 / 255.
 int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
   kb_split = 0;
   if (G != 1 || M < 256 || !gemm_pair_on()) return 1;
@@ -1483,8 +1486,10 @@ int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
   if (2 * tiles > pairs || kb < 32) return 1;
   const int want = std::min(pairs / tiles, kb / 8);
   if (want < 2) return 1;
-  kb_split = (kb + want - 1) / want;
-  return (kb + kb_split - 1) / kb_split;
+  const int run = (kb + want - 1) / want, runs = (kb + run - 1) / run;
+  if (20 * (kb - run) <= 160 + 9 * tiles * runs) return 1;
+  kb_split = run;
+  return runs;
 }
 
 int gemm_sm_count() {

@@ -177,6 +177,21 @@ def test_launches_of_split_products_are_counted(K, kernels):
     assert _ext.launches() - n == kernels
 
 
+@pytest.mark.parametrize("M,N,K,kernels", [(256, 256, 1984, 1), (256, 256, 1985, 2), (1024, 1024, 3072, 1), (1024, 1024, 4096, 2), (4096, 512, 2048, 1), (4096, 512, 4096, 1),
+                                           (4096, 512, 8192, 2), (255, 256, 8192, 1), (9472, 256, 16384, 2), (9473, 256, 16384, 1)])
+def test_products_are_cut_where_it_pays(M, N, K, kernels):
+    """The line between whole and cut products (a cut one is two kernels), and the result on both sides of it."""
+    from memarch_b200.ops import _ext, gemm
+    K8 = (K + 7) // 8 * 8
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = torch.randn(M, K8, device="cuda", generator=g).bfloat16(), torch.randn(N, K8, device="cuda", generator=g).bfloat16()
+    n = _ext.launches()
+    out = gemm(a, b)
+    assert _ext.launches() - n == kernels
+    rows = torch.arange(0, M, max(1, M // 64), device="cuda")
+    assert _rel(out[rows], a[rows].double() @ b.double().t()) < 4e-3
+
+
 # ------------------------------------------------------------------------------------------------ narrow tiles
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 256), (257, 264, 128), (4095, 512, 520), (1001, 136, 64), (256, 1024, 2048), (9472, 256, 64), (513, 8, 16)])
 def test_gemm_narrow_tiles(M, N, K):
