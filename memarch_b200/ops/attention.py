@@ -21,7 +21,7 @@ from .basic import dense
 
 ATTN_CORE = os.environ.get("MEMARCH_ATTN", "auto")             # auto | own | lib: see `own_core`
 OWN_WINDOW_EVAL = os.environ.get("MEMARCH_ATTN_EVAL", "own") == "own"
-OWN_CAUSAL_T = 512                                            # plain causal texts up to this length: see `own_core`
+OWN_CAUSAL_T, OWN_CAUSAL_WORK = 512, 100_000                   # plain causal texts: length, words x heads in all; see `own_core`
 OWN_BWD = os.environ.get("MEMARCH_ATTN_BWD", "own") == "own"
 WINDOW_BODY = os.environ.get("MEMARCH_WINDOW", "flash")        # library body of windowed attention with backward: flash | block
 
@@ -179,19 +179,20 @@ def _flash_window(q, k, v, window):
     return _lib_window(q, k, v, window)
 
 
-def own_core(T, windowed, no_grad):
+def own_core(B, T, H, windowed, no_grad):
     """Whether head-dim-64 attention runs on the own kernels.  `MEMARCH_ATTN=own`: always.  `lib`: only windows without a backward
-    pass, and those only with `MEMARCH_ATTN_EVAL=own` (the default).  `auto`, the default: windows and short causal texts, but windows
-    without a backward pass as `MEMARCH_ATTN_EVAL` says."""
-    # Windows, forward + backward: 2 x 16 384 words, 16 heads, window 256: 700 us against 1221 for the library flash kernel; 4 x
-    # 4096, window 1024: 635 against 1242.  Short causal texts: 8 x 512, 8 heads: 90 against 157; 16 x 256, 12 heads: 102
-    # against 144.  On longer causal texts the library core is still ahead (32 x 1024, 32 heads: 1570 against 1361; 16 x 2048, 16
-    # heads: 1222 against 943).
+    pass, and those only with `MEMARCH_ATTN_EVAL=own` (the default).  `auto`, the default: windows and short causal texts (with a backward pass
+    only few of them), but windows without a backward pass as `MEMARCH_ATTN_EVAL` says."""
+    # Us, own against library core, forward + backward.  Windows: 2 x 16 384 words, 16 heads, window 256: 700 / 1221; 4 x 4096, window
+    # 1024: 635 / 1242.  Causal, 4 texts, 8 heads, 256, 512, 768 and 1024 words: 70 / 184, 76 / 162, 101 / 158, 117 / 159 (the library's
+    # time is the host's); 16 texts, 12 heads, 256, 384, 512, 640 and 1024 words: 101 / 175, 157 / 163, 177 / 182, 212 / 206,
+    # 372 / 288; 32 texts, 32 heads, 256, 384, 512 and 1024 words: 303 / 289, 536 / 473, 632 / 582, 1594 / 1364: full, the chip does the
+    # library's one backward kernel faster.  Forward alone, 32 texts, 32 heads, 256, 384 and 512 words: 73 / 87, 143 / 169, 181 / 175.
     if ATTN_CORE == "own":
         return True
     if windowed and no_grad:
         return OWN_WINDOW_EVAL
-    return ATTN_CORE != "lib" and (windowed or T <= OWN_CAUSAL_T)
+    return ATTN_CORE != "lib" and (windowed or (T <= OWN_CAUSAL_T and (no_grad or B * T * H <= OWN_CAUSAL_WORK)))
 
 
 def attention(qkv, window=None, rope_half=False, qk_norm=False):
@@ -200,7 +201,7 @@ def attention(qkv, window=None, rope_half=False, qk_norm=False):
     win = None if (window is None or window >= T) else int(window)
     if _ext.use_cuda(qkv) and qkv.dtype == torch.bfloat16 and not qk_norm and hd % 8 == 0:
         no_grad = not (torch.is_grad_enabled() and qkv.requires_grad)
-        own = own_core(T, win is not None, no_grad)
+        own = own_core(B, T, H, win is not None, no_grad)
         if hd == 64 and own and (no_grad or OWN_BWD):
             return _QkvAttn.apply(dense(qkv.detach() if no_grad else qkv), win or 0, rope_half)
         q, k, v = _RopeSplit.apply(qkv, rope_half)

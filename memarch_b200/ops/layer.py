@@ -35,7 +35,7 @@ def attn_half_ok(x, pending, nw, wqkv, wo, heads, window):
     """Head dim 64 and lengths that the own attention kernels serve (see `ops.attention.own_core`)."""
     B, T, d = x.shape
     no_grad = not torch.is_grad_enabled()
-    return (d == heads * 64 and own_core(T, window is not None and window < T, no_grad) and (OWN_BWD or no_grad)
+    return (d == heads * 64 and own_core(B, T, heads, window is not None and window < T, no_grad) and (OWN_BWD or no_grad)
             and wqkv.shape == (3 * d, d) and wo.shape == (d, d) and _common(x, nw, (wqkv, wo))
             and (pending is None or (pending.dtype == torch.bfloat16 and pending.shape == x.shape)))
 

@@ -596,19 +596,20 @@ def test_attention_core_switches(monkeypatch):
     MEMARCH_ATTN_EVAL decides about those in the default and the lib setting."""
     import importlib
     attn = importlib.import_module("memarch_b200.ops.attention")
-    every = [(T, w, g) for T in (64, 512, 513, 4096) for w in (False, True) for g in (False, True)]
+    every = [(B, T, w, g) for B in (1, 64) for T in (64, 512, 513, 4096) for w in (False, True) for g in (False, True)]
     for core in ("auto", "own", "lib"):
         for ev in (True, False):
             monkeypatch.setattr(attn, "ATTN_CORE", core)
             monkeypatch.setattr(attn, "OWN_WINDOW_EVAL", ev)
-            for T, windowed, no_grad in every:
+            for B, T, windowed, no_grad in every:
                 if core == "own":
                     want = True
                 elif windowed and no_grad:
                     want = ev
                 else:
-                    want = core == "auto" and (windowed or T <= attn.OWN_CAUSAL_T)
-                assert attn.own_core(T, windowed, no_grad) is want, (core, ev, T, windowed, no_grad)
+                    few = no_grad or B * T * 8 <= attn.OWN_CAUSAL_WORK
+                    want = core == "auto" and (windowed or (T <= attn.OWN_CAUSAL_T and few))
+                assert attn.own_core(B, T, 8, windowed, no_grad) is want, (core, ev, B, T, windowed, no_grad)
 
 
 @pytest.mark.parametrize("word", ["gemm_status", "attn_status_read", "attn_bwd_status_read"])
