@@ -8,7 +8,7 @@
 namespace mb {
 
 static void check_rows(const torch::Tensor& t, int64_t d, const char* what) {
-  TORCH_CHECK(t.is_contiguous() && t.scalar_type() == torch::kBFloat16 && t.size(-1) == d && d % 8 == 0 &&
+  TORCH_CHECK(t.is_contiguous() && t.scalar_type() == torch::kBFloat16 && t.size(-1) == d && d > 0 && d % 8 == 0 &&
               (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, what, ": contiguous 16-byte aligned bf16 rows, d % 8 == 0");
 }
 static const long long* i64(const torch::Tensor& t) {
@@ -32,8 +32,9 @@ torch::Tensor rows_gather(torch::Tensor src, torch::Tensor table) {
 
 torch::Tensor rows_gather_sum(torch::Tensor src, torch::Tensor idx, c10::optional<torch::Tensor> w) {
   const c10::cuda::CUDAGuard guard(src.device());
-  const int64_t d = src.size(-1), S = src.numel() / d, N = idx.size(0);
+  const int64_t d = src.size(-1), N = idx.size(0);
   check_rows(src, d, "rows_gather_sum");
+  const int64_t S = src.numel() / d;
   auto out = torch::empty({N, d}, src.options());
   if (N) rows_gather_sum_launch(src.data_ptr(), i64(idx), w.has_value() && w->defined() ? f32(*w, S) : nullptr, out.data_ptr(), N, (int)idx.size(1),
                                 (int)d, S, at::cuda::getCurrentCUDAStream());

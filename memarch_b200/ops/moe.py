@@ -20,7 +20,8 @@ from .basic import gemm, gemm_ok, relu2, swiglu
 # ------------------------------------------------------------------------------------------------ dispatch
 def _wide(*ts):
     """Rows the 16-byte kernels of `csrc/gather.cu` take; the others stay on the element-wise ones."""
-    return all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape[-1] % 8 == 0 and t.data_ptr() % 16 == 0 for t in ts)
+    return all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape[-1] > 0 and t.shape[-1] % 8 == 0 and t.data_ptr() % 16 == 0
+               for t in ts)
 
 
 class _SlotGather(torch.autograd.Function):

@@ -591,6 +591,14 @@ def test_training_loop_raises_when_a_device_wait_has_run_out(monkeypatch):
     loop.device_status(tr_cpu)                                    # CPU runs have no status words
 
 
+def test_rows_without_columns_stay_on_the_general_kernels():
+    """The 16-byte row kernels divide by the row's length: rows of no columns are not theirs."""
+    import torch
+    from memarch_b200.ops.moe import _wide
+    assert _wide(torch.zeros(3, 8, dtype=torch.bfloat16)) and _wide(torch.zeros(0, 8, dtype=torch.bfloat16))
+    assert not _wide(torch.zeros(3, 0, dtype=torch.bfloat16)) and not _wide(torch.zeros(3, 8, dtype=torch.bfloat16), torch.zeros(3, 12, dtype=torch.bfloat16))
+
+
 def test_attention_core_switches(monkeypatch):
     """MEMARCH_ATTN=own puts every attention of head dim 64 on the own kernels, lib none but evaluation windows, and
     MEMARCH_ATTN_EVAL decides about those in the default and the lib setting."""
