@@ -15,24 +15,27 @@ import warnings
 
 import torch
 
+# this package's kernels live in namespace mb: by name, the others there are row kernels
+OWN_BUCKETS = (
+    ("own tcgen05 gemm", ("mb::gemm_", "mb::sum_parts")),
+    ("attention", ("mb::attn_", "mb::rope_qk", "mb::rope_merge")),
+    ("optimizer", ("mb::instinct", "mb::noalloc")),
+    ("collectives", ("mb::peer_", "mb::allreduce", "mb::broadcast_from", "mb::reduce_to")),
+)
 BUCKETS = (
-    ("own tcgen05 gemm", ("gemm_tc",)),
     ("library gemm", ("gemm", "cutlass", "cublas", "nvjet", "sm90_xmma", "sm100_xmma", "xmma")),
     ("attention", ("attn", "flash", "fmha", "sdpa", "cudnn")),
-    ("optimizer", ("instinct",)),
-    ("collectives", ("nccl", "peer_", "allreduce", "multimem")),
-    ("own row kernels", ("rmsnorm", "relu2", "swiglu", "rope", "ce_rows", "resid_add", "gather_rows", "gather_sum",
-                         "row_dot", "anchor_select", "moe_slots", "lock_find")),
+    ("collectives", ("nccl", "multimem")),
     ("copies", ("memcpy", "memset", "copy_", "CatArrayBatchedCopy", "direct_copy")),
 )
 
 
 def bucket_of(name):
-    low = name.lower()
-    for b, keys in BUCKETS:
+    low, own = name.lower(), "mb::" in name
+    for b, keys in OWN_BUCKETS if own else BUCKETS:
         if any(k.lower() in low for k in keys):
             return b
-    return "other"
+    return "own row kernels" if own else "other"
 
 
 def _setup(args, device):

@@ -599,6 +599,18 @@ def test_rows_without_columns_stay_on_the_general_kernels():
     assert not _wide(torch.zeros(3, 0, dtype=torch.bfloat16)) and not _wide(torch.zeros(3, 8, dtype=torch.bfloat16), torch.zeros(3, 12, dtype=torch.bfloat16))
 
 
+def test_profile_families():
+    """Own kernels are told from library ones by their namespace, whatever their name holds."""
+    from memarch_b200.utils.profile import bucket_of
+    for name, want in (("void mb::gemm_pair_kernel<false, true, 1, 0>(...)", "own tcgen05 gemm"), ("mb::sum_parts_kernel<true>", "own tcgen05 gemm"),
+                       ("mb::attn_dkv_kernel(CUtensorMap)", "attention"), ("void mb::instinct_rowcol_s8<1, 6>(mb::InstinctArgs)", "optimizer"),
+                       ("mb::route_place_kernel(mb::RouteArgs)", "own row kernels"), ("mb::lock_search_kernel(long long const*)", "own row kernels"),
+                       ("mb::combine_bwd_kernel(uint4 const*)", "own row kernels"), ("mb::peer_gather_kernel", "collectives"),
+                       ("nvjet_sm100_tst_128x256", "library gemm"), ("pytorch_flash::flash_bwd_kernel", "attention"),
+                       ("at::native::vectorized_elementwise_kernel<4>", "other"), ("Memset (Device)", "copies")):
+        assert bucket_of(name) == want, name
+
+
 def test_attention_core_switches(monkeypatch):
     """MEMARCH_ATTN=own puts every attention of head dim 64 on the own kernels, lib none but evaluation windows, and
     MEMARCH_ATTN_EVAL decides about those in the default and the lib setting."""
