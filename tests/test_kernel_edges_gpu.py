@@ -230,6 +230,33 @@ def test_gemm_narrow_tiles(M, N, K):
             assert _rel(q, r) < 1e-2
 
 
+@pytest.mark.parametrize("M", [128, 129, 133, 200, 255])
+@pytest.mark.parametrize("act", [None, "swiglu", "relu2"])
+def test_few_ragged_rows_on_the_single_cta_kernel(M, act):
+    """128 to 255 rows, most of them no multiple of 8: plain and activation epilogues, input and weight gradients."""
+    from memarch_b200.ops import basic
+    g = torch.Generator(device="cuda").manual_seed(M)
+    K, H = 136, 72
+    N = 2 * H if act == "swiglu" else H * 2
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    res = []
+    for own in (True, False):
+        a, u = (t.clone() if own else t.double() for t in (x, w))
+        a.requires_grad_(), u.requires_grad_()
+        if own:
+            y = basic.linear(a, u) if act is None else basic.linear_act(a, u, act)
+        else:
+            p = a @ u.t()
+            y = p if act is None else torch.nn.functional.silu(p[:, :H]) * p[:, H:] if act == "swiglu" else p.relu().square()
+        go = torch.randn(y.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).bfloat16()
+        y.backward(go.to(y.dtype))
+        res.append([y.detach(), a.grad, u.grad])
+    # bf16 pre-activations, activations and their gradients: two to three roundings of 2^-9 along the chain
+    for p, q in zip(*res):
+        assert _rel(p, q) < 1e-2
+
+
 # ------------------------------------------------------------------------------------------------ routing
 @pytest.mark.parametrize("N,d,E,k,C", [(1, 8, 1, 1, 1), (31, 64, 3, 2, 7), (33, 256, 8, 2, 64), (100, 264, 48, 4, 3), (700, 2048, 8, 2, 176), (257, 512, 128, 8, 9), (4000, 768, 16, 2, 626)])
 def test_route_and_slot_fused(N, d, E, k, C):
