@@ -445,7 +445,8 @@ def test_expert_ffn_backward_epilogue(E, C, d, H, act):
 
 # ------------------------------------------------------------------------------------------------ optimizer
 @pytest.mark.parametrize("shape,bf16", [((1190, 2048), False), ((1200, 1540), True), ((2500, 6144), True), ((1300, 4100), False), ((1024, 4096), False),
-                                        ((3072, 1024), False), ((5, 700, 1540), True), ((3, 640, 2304), True), ((12000, 512), False), ((260, 256), False)])
+                                        ((3072, 1024), False), ((5, 700, 1540), True), ((3, 640, 2304), True), ((12000, 512), False), ((260, 256), False),
+                                        ((4, 1024, 256), True), ((4, 592, 256), True), ((3, 789, 256), True), ((2500, 256), False)])
 def test_instinct_streamed_forms(shape, bf16):
     """One step on the kernels against the PyTorch statement: whole and cut rows, expert borders inside a block, all width classes."""
     from memarch_b200.config import OptConfig
