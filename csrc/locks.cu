@@ -31,9 +31,9 @@ struct LockTable {                                   // one per warp
 };
 
 __device__ __forceinline__ unsigned long long ngram_key(const int* tok, int t, int n) {
-  unsigned long long k = (unsigned)tok[t] & 0x1FFFFF;
-  if (n >= 2) k |= (unsigned long long)((unsigned)tok[t - 1] & 0x1FFFFF) << 21;
-  if (n >= 3) k |= (unsigned long long)((unsigned)tok[t - 2] & 0x1FFFFF) << 42;
+  unsigned long long k = (unsigned)tok[t];
+  if (n >= 2) k |= (unsigned long long)(unsigned)tok[t - 1] << 21;
+  if (n >= 3) k |= (unsigned long long)(unsigned)tok[t - 2] << 42;
   return k;
 }
 __device__ __forceinline__ unsigned hash64(unsigned long long k) {
@@ -55,8 +55,9 @@ __global__ void __launch_bounds__(LK_WARPS * 32) lock_search_kernel(const long l
   int wide = 0;
 #pragma unroll 8
   for (int t = threadIdx.x; t < T; t += LK_WARPS * 32) {
-    tok[t] = (int)xr[t];
-    wide |= (unsigned)(tok[t] + (1 << 20)) >> 21;
+    const int id = (int)xr[t];
+    tok[t] = id & 0x1FFFFF;
+    wide |= (unsigned)(id + (1 << 20)) >> 21;
   }
   for (int i = lane; i < LK_SLOTS; i += 32) tab.slot[i] = LK_NODES;
   if (__syncthreads_or(wide)) {
@@ -64,7 +65,7 @@ __global__ void __launch_bounds__(LK_WARPS * 32) lock_search_kernel(const long l
     for (int t = blockIdx.x * (LK_WARPS * 32) + threadIdx.x; t < T; t += gridDim.x * (LK_WARPS * 32)) {
       int j = t >= n - 1 ? t - 1 : -1;
       for (; j >= n - 1; --j)
-        if (tok[j] == tok[t] && (n < 2 || tok[j - 1] == tok[t - 1]) && (n < 3 || tok[j - 2] == tok[t - 2])) break;
+        if ((int)xr[j] == (int)xr[t] && (n < 2 || (int)xr[j - 1] == (int)xr[t - 1]) && (n < 3 || (int)xr[j - 2] == (int)xr[t - 2])) break;
       src[((long long)b * T + t) * n_keys + (n - 1)] = j >= n - 1 ? min(j + 1, T - 1) : 0;
     }
     return;
