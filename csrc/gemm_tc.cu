@@ -1474,11 +1474,12 @@ void sum_parts_launch(const float* parts, int splits, void* dst, int f32, int ac
 }
 
 // How many runs to cut the contraction of one plain product into (1: none).  A product with fewer output tiles than half of the
-// 74 CTA pairs leaves the rest of the chip idle.  A cut saves each pair kb - kb_split k-blocks of 64 (0.3 us each) and costs a second
-// launch and an fp32 slab per run and tile that is written and read back, 8 k-blocks and 0.45 per slab.  The line is measured
-// against the whole product as launch_gemm_seg runs it, with 128-column tiles where it takes them.  Us, (M, N, K), cut / whole:
-// (256, 256, 2048) 17.4 / 20.5; (1024, 512, 2048) 21.5 / 22.5; (1024, 1024, 3072) 27.6 / 26.6 and 4096 29.7 / 31.7; (4096, 512,
-// 2048) 27.7 / 22.5, 4096 35.8 / 34.8 and 8192 50 / 55; (1000, 256, 50304) 48 / 255.
+// 74 CTA pairs leaves the rest of the chip idle.  A cut saves each pair kb - kb_split k-blocks of 64 (0.27 us each) and costs a second
+// launch and an fp32 slab per run and tile that is written and read back, 5 k-blocks and 0.31 per slab.  The line is measured
+// against the whole product as launch_gemm_seg runs it, with 128-column tiles where it takes them, in runs of products back to
+// back.  Us, (M, N, K), cut / whole: (256, 256, 2048) 14.5 / 17; (1024, 512, 2048) 16.5 / 18.6; (1536, 512, 2048) 17.5 / 18.6; (1024,
+// 1024, 2048) 20.6 / 18.6 and 3072 20.8 / 24.3; (4096, 512, 2048) 22.6 / 20, 3072 25 / 25 and 4096 28.8 / 30.3; (1024, 256, 50304)
+// 42 / 240.
 int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
   kb_split = 0;
   if (G != 1 || M < 256 || !gemm_pair_on()) return 1;
@@ -1487,7 +1488,7 @@ int gemm_splits(int M, int N, int K, int G, int max_ctas, int& kb_split) {
   const int want = std::min(pairs / tiles, kb / 8);
   if (want < 2) return 1;
   const int run = (kb + want - 1) / want, runs = (kb + run - 1) / run;
-  if (20 * (kb - run) <= 160 + 9 * tiles * runs) return 1;
+  if (100 * (kb - run) <= 500 + 31 * tiles * runs) return 1;
   kb_split = run;
   return runs;
 }
