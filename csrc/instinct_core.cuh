@@ -595,14 +595,14 @@ __global__ void __launch_bounds__(512) instinct_stat_rows_s8(InstinctArgs a, con
   ring.nslot = gs + ms;
   const long long cpr = a.C >> 8, cpe = a.R * cpr;       // chunks per row, per expert
   const long long NC = a.E * cpe;
-  const long long NU = NC / unit, lo = NU * blockIdx.x / gridDim.x * unit, hi = NU * (blockIdx.x + 1) / gridDim.x * unit;
+  const long long NU = unit == 1 ? NC : NC / unit, lo = NU * blockIdx.x / gridDim.x * unit, hi = NU * (blockIdx.x + 1) / gridDim.x * unit;
   for (long long seg = lo; seg < hi;) {
     const long long e = seg / cpe, seg_hi = min(hi, (e + 1) * cpe);
     if (cs) {
       __syncthreads();
       load_colscale(cs, colsum, nullptr, e, a.C, col_count);
     }
-    const long long cpw = ((seg_hi - seg) / unit + nw - 1) / nw * unit;
+    const long long cpw = ((unit == 1 ? seg_hi - seg : (seg_hi - seg) / unit) + nw - 1) / nw * unit;
     const long long f0 = min(seg_hi, seg + warp * cpw), total = min(seg_hi, f0 + cpw) - f0;
     // both arrays bf16: 8 consecutive elements per lane are one full 16-byte copy each (faster than two 8-byte ones)
     const bool packed = a.g_bf16 && a.m_bf16;
