@@ -267,7 +267,7 @@ torch::Tensor rope_merge_bwd(torch::Tensor dq, torch::Tensor dk, torch::Tensor d
   Src3 src;
   for (int i = 0; i < 3; ++i) {
     TORCH_CHECK(g[i].dim() == 4 && g[i].scalar_type() == torch::kBFloat16 && g[i].stride(3) == 1 && g[i].size(2) == T && on16(g[i]) &&
-                (B == 1 || g[i].stride(0) % 8 == 0) && (H == 1 || g[i].stride(1) % 8 == 0) && (T == 1 || g[i].stride(2) % 8 == 0),
+                g[i].stride(0) % 8 == 0 && g[i].stride(1) % 8 == 0 && g[i].stride(2) % 8 == 0,
                 "rope_merge_bwd: (B,H,T,hd) bf16 with contiguous last dim, 16-byte aligned rows");
     TORCH_CHECK(g[i].stride(0) % 8 == 0 && g[i].stride(1) % 8 == 0 && g[i].stride(2) % 8 == 0 &&
                 (reinterpret_cast<uintptr_t>(g[i].data_ptr()) & 15) == 0, "rope_merge_bwd: 16-byte aligned rows");

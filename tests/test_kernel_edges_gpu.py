@@ -562,17 +562,6 @@ def test_light_layer_keeps_one_packed_array():
     assert len(out) == 2 and kept <= (2 + 6 + 2 + 2) * M * d + (8 + 1) * M * 4 + 8 * 512
 
 
-def test_rotation_backward_ignores_strides_of_single_places():
-    """A dimension of one place has no stride to speak of: gradients of one text, head or word are taken as they are."""
-    from memarch_b200.ops import _ext
-    from memarch_b200.ops.attention import rope_tables
-    cos, sin = rope_tables(1, 64, "cuda")
-    g = torch.randn(3, 64, device="cuda").bfloat16()
-    odd = [torch.as_strided(t, (1, 1, 1, 64), (67, 3, 5, 1)) for t in g]
-    even = [t.clone().view(1, 1, 1, 64) for t in g]
-    assert torch.equal(_ext.C().rope_merge_bwd(*odd, cos, sin, False), _ext.C().rope_merge_bwd(*even, cos, sin, False))
-
-
 # ------------------------------------------------------------------------------------------------ light layer halves
 @pytest.mark.parametrize("d,B,T,window,blk,half,defer", [(128, 2, 129, 64, (), False, True), (256, 1, 257, 2048, ("relu2",), False, False), (64, 3, 100, 7, (), True, False),
                                                          (128, 1, 600, 2048, (), False, True), (192, 2, 300, 128, ("relu2",), True, True)])
