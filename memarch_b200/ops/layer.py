@@ -8,6 +8,7 @@ weight leaves its GEMM in fp32 instead of being rounded to bf16 and cast back.
 from __future__ import annotations
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from . import _ext, basic
 from .attention import OWN_BWD, own_core, rope_tables
@@ -28,7 +29,13 @@ def _common(x, nw, ws):
     if torch.is_grad_enabled():
         # every weight trained and the stream part of the graph, as in a training step
         return x.requires_grad and nw.requires_grad and all(_trained(w) for w in ws)
-    return all(w.dtype in (torch.float32, torch.bfloat16) for w in ws)
+    return all(w.dtype in (torch.float32, torch.bfloat16) for w in ws) and _no_tangent(x, nw, *ws)
+
+
+def _no_tangent(*ts):
+    """Without gradients no autograd node stands around the native call: forward-mode derivatives are left to the single ops,
+    whose nodes refuse them, instead of being lost."""
+    return all(unpack_dual(t).tangent is None for t in ts)
 
 
 def attn_half_ok(x, pending, nw, wqkv, wo, heads, window):
@@ -37,14 +44,14 @@ def attn_half_ok(x, pending, nw, wqkv, wo, heads, window):
     no_grad = not torch.is_grad_enabled()
     return (d == heads * 64 and own_core(B, T, heads, window is not None and window < T, no_grad) and (OWN_BWD or no_grad)
             and wqkv.shape == (3 * d, d) and wo.shape == (d, d) and _common(x, nw, (wqkv, wo))
-            and (pending is None or (pending.dtype == torch.bfloat16 and pending.shape == x.shape)))
+            and (pending is None or (pending.dtype == torch.bfloat16 and pending.shape == x.shape and (not no_grad or _no_tangent(pending)))))
 
 
 def ffn_half_ok(h, a, nw, wup, wdown, swiglu):
     N, d = wup.shape
     H = N // 2 if swiglu else N
     return (a.dtype == torch.bfloat16 and a.shape == h.shape and d == h.shape[2] and wdown.shape == (d, H) and N % 16 == 0 and H % 8 == 0
-            and (basic.FUSE_DSWIGLU or not swiglu) and _common(h, nw, (wup, wdown)))
+            and (basic.FUSE_DSWIGLU or not swiglu) and _common(h, nw, (wup, wdown)) and (torch.is_grad_enabled() or _no_tangent(a)))
 
 
 def _taker(ws):

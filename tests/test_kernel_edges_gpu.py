@@ -651,6 +651,29 @@ def test_light_layer_halves_leave_other_cases_alone():
 
 
 @pytest.mark.parametrize("train", [True, False])
+@pytest.mark.parametrize("what", ["x", "pending", "norm", "up"])
+def test_light_layer_refuses_forward_mode(train, what):
+    """No forward-mode derivative is implemented: one that is asked for is refused, with and without gradients, not dropped."""
+    import torch.autograd.forward_ad as fw
+    from memarch_b200.models.blocks import LightBlock
+    with torch.device("cuda"):
+        b = LightBlock(128, 2)
+    x = torch.randn(2, 200, 128, device="cuda", requires_grad=True)
+    pending = torch.randn_like(x).bfloat16()
+    with torch.set_grad_enabled(train), fw.dual_level():
+        dual = lambda t: fw.make_dual(t.detach(), torch.ones_like(t))
+        if what == "norm":
+            del b.n2.weight
+            b.n2.weight = dual(torch.ones(128, device="cuda"))
+        if what == "up":
+            w = b.up.weight
+            del b.up.weight
+            b.up.weight = dual(w)
+        with pytest.raises((RuntimeError, NotImplementedError), match="jvp|forward.mode|forward AD"):
+            b(dual(x) if what == "x" else x, 64, pending=dual(pending) if what == "pending" else pending)
+
+
+@pytest.mark.parametrize("train", [True, False])
 def test_light_layer_with_strided_norm_weights(train):
     """Norm weights that are views with a stride give what their contiguous copies give."""
     from memarch_b200.models.blocks import LightBlock
