@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(LK_WARPS * 32) lock_search_kernel(const long l
   for (int t = threadIdx.x; t < T; t += LK_WARPS * 32) {
     const int id = (int)xr[t];
     tok[t] = id & 0x1FFFFF;
-    wide |= (unsigned)(id + (1 << 20)) >> 21;
+    wide |= ((unsigned)id + (1u << 20)) >> 21;
   }
   for (int i = lane; i < LK_SLOTS; i += 32) tab.slot[i] = LK_NODES;
   if (__syncthreads_or(wide)) {

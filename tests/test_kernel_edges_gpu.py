@@ -76,7 +76,7 @@ def test_lock_buckets_of_ids_outside_the_table(B, T):
 
 
 @pytest.mark.parametrize("T", [40, 2500])
-@pytest.mark.parametrize("low", [-(1 << 20), -(1 << 20) - 1, (1 << 21) - 3, 1 << 30])
+@pytest.mark.parametrize("low", [-(1 << 20), -(1 << 20) - 1, (1 << 21) - 3, 1 << 30, (1 << 31) - 12])
 def test_lock_ids_outside_the_vocabulary(T, low):
     """Words are told apart by their whole id, also where ids differ by a multiple of 2^21."""
     from memarch_b200.ops import anchors, ref
